@@ -7,18 +7,24 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = [os.path.join(HERE, "csrc", f) for f in ("dpg_host.cu", "dpg_kernel.cu", "dpg_maps.cu")]
+SRC = [os.path.join(HERE, "csrc", f"dpg_{f}.cu") for f in ("host", "kernel", "queue", "adjoint", "energy", "big", "maps")]
 OUT = os.path.join(HERE, "libdpg_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-         "-Xcompiler", "-fPIC", "-shared", "--expt-relaxed-constexpr"]
+         "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 
 
 def build(verbose=False):
-    cmd = [NVCC] + FLAGS + (["-Xptxas", "-v"] if verbose else []) + SRC + ["-o", OUT, "-lcudart"]
-    subprocess.check_call(cmd)
+    flags = FLAGS + (["-Xptxas", "-v"] if verbose else [])
+    with tempfile.TemporaryDirectory() as tmp:  # one nvcc per translation unit, side by side
+        objs = [os.path.join(tmp, os.path.basename(f) + ".o") for f in SRC]
+        jobs = [subprocess.Popen([NVCC] + flags + ["-c", f, "-o", o]) for f, o in zip(SRC, objs)]
+        if any([j.wait() for j in jobs]):
+            raise RuntimeError("nvcc failed")
+        subprocess.check_call([NVCC] + flags + ["-shared"] + objs + ["-o", OUT, "-lcudart"])
     return OUT
 
 

@@ -1,0 +1,38 @@
+// dpg_adjoint.cu — the reverse mode's kernel instances and launch.
+#include "dpg_phases.cuh"
+
+namespace {
+#include "dpg_adjoint.cuh"
+}  // namespace
+
+int dpg_configure_adjoint(const DpgPlanDev* plan, int bytes) {
+  KernelFn k = pick_adjoint_kernel(plan);
+  if (!k) return DPG_OK;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+  return DPG_OK;
+}
+
+int dpg_launch_adjoint(const DpgPlanDev* plan, const DpgLaunch* Lin, cudaStream_t stream) {
+  if (Lin->C <= 0) return DPG_OK;
+  if (!plan->adj_ok) return dpg::fail(DPG_ERR_UNSUPPORTED, "reverse mode is not available for this bucket");
+  KernelFn k = pick_adjoint_kernel(plan);
+  if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no adjoint kernel instance for this bucket size");
+  const int grid = std::min(Lin->C, dpg::num_sms());
+  DpgLaunch L = *Lin;
+  void* scratch = nullptr;
+  const size_t per = plan->scratch_per_cta;
+  cudaError_t ea = dpg::ws_alloc(&scratch, (size_t)grid * per * 2 * sizeof(double), stream);
+  if (ea != cudaSuccess) {
+    cudaGetLastError();
+    return dpg::fail(DPG_ERR_OUT_OF_MEMORY, std::string("scratch allocation: ") + cudaGetErrorString(ea));
+  }
+  L.scratch = (double*)scratch;
+  L.scratch2 = L.scratch + (size_t)grid * per;
+  size_t bytes = (size_t)plan->sm_total * sizeof(double);
+  k<<<grid, NT, bytes, stream>>>(*plan, L);
+  cudaError_t e = cudaGetLastError();
+  cudaFreeAsync(scratch, stream);
+  if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
+  return DPG_OK;
+}

@@ -16,27 +16,30 @@
 
 #define DPG_CHA 4  // quadrature points per pull-back chunk (two 8-row tiles of (point, slot))
 
-// Element (r, c) of a C-fragment tiled N x (M+1) matrix in a scratch slot
-// (tile (I, J) at ((J * NBT + I) * 32 + lane) double2, lane = r * 4 + c / 2).
-__device__ __forceinline__ size_t cfrag_index(int NBT, int r, int c) {
-  return ((size_t)((c >> 3) * NBT + (r >> 3)) * 32 + (r & 7) * 4 + ((c & 7) >> 1)) * 2 + (c & 1);
-}
-
-// Xe = G^-1 [B | F] per column tile: forward W = L^-1 Y, then backward X = L^-T W,
-// in registers; the result replaces Y in the scratch slot.
+// Xe = G^-1 [B | F] per column tile: forward W = Ls^-1 S Y, then backward X = S Ls^-T W (S: the
+// equilibration scales, S G S = Ls Ls^T), in registers; the result replaces Y in the scratch slot.
 template <int NBTM>
 __device__ __forceinline__ void phase_adj_solve(const DpgPlanDev& P, const DpgLaunch& L) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const double* GT = dpg_smem + P.sm_gt;
   const double* LINV = dpg_smem + P.sm_linv;
+  const double* scale = dpg_smem + P.sm_scale;
   const int J = warp;
   if (J < P.MBT) {
     double2* scr = reinterpret_cast<double2*>(L.scratch + (size_t)blockIdx.x * P.scratch_per_cta) +
                    (size_t)J * P.NBT * 32 + lane;
     double2 acc[NBTM];
 #pragma unroll
-    for (int I = 0; I < NBTM; I++) acc[I] = (I < P.NBT) ? scr[I * 32] : make_double2(0.0, 0.0);
+    for (int I = 0; I < NBTM; I++) {
+      acc[I] = make_double2(0.0, 0.0);
+      if (I < P.NBT) {
+        acc[I] = scr[I * 32];
+        const double si = scale[I * 8 + g];
+        acc[I].x *= si;
+        acc[I].y *= si;
+      }
+    }
     // forward: X_k = L_kk^-1 Y_k; Y_i -= L_ik X_k
 #pragma unroll
     for (int k = 0; k < NBTM; k++) {
@@ -52,17 +55,7 @@ __device__ __forceinline__ void phase_adj_solve(const DpgPlanDev& P, const DpgLa
         cfrag_to_bfrag(x, lane, x0, x1);
         x0 = -x0;
         x1 = -x1;
-#pragma unroll
-        for (int i = k + 1; i < NBTM; i += 2) {
-          const double* Lik = GT + (i * (i + 1) / 2 + k) * 64;
-          if (i + 1 < NBTM && i + 1 < P.NBT) {
-            const double* Li1k = GT + ((i + 1) * (i + 2) / 2 + k) * 64;
-            dmma16x8(acc[i], acc[i + 1], Lik[lane], Li1k[lane], Lik[32 + lane], Li1k[32 + lane], x0, x1);
-          } else if (i < P.NBT) {
-            dmma(acc[i], Lik[lane], x0);
-            dmma(acc[i], Lik[32 + lane], x1);
-          }
-        }
+        solve_update<NBTM>(GT, P.NBT, k, lane, acc, x0, x1);
       }
     }
     // backward: X_k = L_kk^-T W_k; W_i -= L_ki^T X_k for i < k.  A-fragments of a
@@ -97,7 +90,10 @@ __device__ __forceinline__ void phase_adj_solve(const DpgPlanDev& P, const DpgLa
     }
 #pragma unroll
     for (int I = 0; I < NBTM; I++)
-      if (I < P.NBT) scr[I * 32] = acc[I];
+      if (I < P.NBT) {
+        const double si = scale[I * 8 + g];
+        scr[I * 32] = make_double2(acc[I].x * si, acc[I].y * si);
+      }
   }
   __syncthreads();
 }
@@ -168,16 +164,18 @@ __device__ __forceinline__ void adj_feature_gemm(const DpgPlanDev& P, const DpgL
       const double* f1 = fs + q1 * fsl + V.foff + k * V.ldA + t;
       const bool ok0 = q0 < nq, ok1 = q1 < nq;
       // 16 test rows per m16n8k16: A rows g = (point q0, slot k), rows g + 8 = (point q1, slot k)
-      // (the vars' rows are padded to multiples of 16); the same accumulation order as four
-      // m8n8k4 steps per point pair
+      // (the staged slots are padded to multiples of 16 rows; X has whole tiles only)
       double c4[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int i = 0; i < V.ntiles * 8; i += 16) {
+      const int nrow = V.ntiles * 8;
+      for (int i = 0; i < nrow; i += 16) {
         double av[8], bv[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           av[2 * j] = ok0 ? f0[i + 4 * j] : 0.0;
           av[2 * j + 1] = ok1 ? f1[i + 4 * j] : 0.0;
-          bv[j] = src[cfrag_index(P.NBT, V.ntile0 * 8 + i + 4 * j + t, J * 8 + g)];
+          // (the zero slots of a missing last tile meet the tile before it)
+          const int ri = i + 4 * j < nrow ? i + 4 * j : i + 4 * j - 8;
+          bv[j] = src[cfrag_index(P.NBT, V.ntile0 * 8 + ri + t, J * 8 + g)];
         }
         dmma16(c4, av, bv);
       }
@@ -351,7 +349,8 @@ __device__ __forceinline__ void phase_adj_pull(const DpgPlanDev& P, const DpgLau
 }
 
 template <int NBTM, int GTM, int BTW, int CH>
-__global__ void __launch_bounds__(NT, 1) dpg_adjoint_kernel(const __grid_constant__ DpgPlanDev P, const DpgLaunch L) {
+__global__ void __launch_bounds__(NT, 1) dpg_adjoint_kernel(const __grid_constant__ DpgPlanDev P,
+                                                                  const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x;
   Ctx X;
   double* const sm = dpg_smem;
@@ -386,7 +385,7 @@ __global__ void __launch_bounds__(NT, 1) dpg_adjoint_kernel(const __grid_constan
     phase_b<BTW>(P, L, cell, X);
     __syncthreads();
     phase_gram<GTM, CH>(P, L, cell, X);
-    phase_factor(P, X);
+    phase_factor(P);
     phase_adj_solve<NBTM>(P, L);
     phase_adj_p<NBTM>(P, L, cell);
     phase_adj_pull(P, L, cell);
@@ -406,7 +405,7 @@ __global__ void __launch_bounds__(NT, 1) dpg_adjoint_kernel(const __grid_constan
 
 #define DPG_ADJ_INSTANCES(X) X(12, 5, 4, 8) X(16, 6, 4, 8) X(20, 8, 4, 8) X(24, 12, 6, 8) X(24, 12, 6, 4)
 
-static KernelFn pick_adjoint_kernel(const DpgPlanDev* plan) {
+KernelFn pick_adjoint_kernel(const DpgPlanDev* plan) {
   const int per = (plan->ngb + DPG_NWARPS - 1) / DPG_NWARPS;
   int btw = 0;
   for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);

@@ -379,8 +379,7 @@ __device__ __forceinline__ void big_diag_block(const double* Z, int ld, int k0, 
   constexpr int NTD = NBD * (NBD + 1) / 2;    // 36 lower tiles
   double* const T = S.D;
   double* const linv = S.LI;                  // [8][64] inverse diagonal tiles
-  double* const invd = S.LI + NBD * 64;       // [64]
-  int* const tri = reinterpret_cast<int*>(S.LI + NBD * 64 + ZT);
+  int* const tri = reinterpret_cast<int*>(S.LI + NBD * 64);
   int* const flag = tri + 64;
   __syncthreads();
   for (int e = tid; e < NTD * 64; e += NT) {
@@ -397,7 +396,7 @@ __device__ __forceinline__ void big_diag_block(const double* Z, int ld, int k0, 
   if (tid == 0) *flag = 0;
   __syncthreads();
   tile_cholesky((int)(T - dpg_smem), NBD, NBD, (int)(flag - reinterpret_cast<int*>(dpg_smem)), 1,
-                (int)(reinterpret_cast<double*>(tri) - dpg_smem), (int)(invd - dpg_smem), (int)(linv - dpg_smem));
+                (int)(reinterpret_cast<double*>(tri) - dpg_smem), (int)(linv - dpg_smem));
   if (tid == 0 && *flag > 0) atomicMin(fail, k0 + *flag - 1);
   if (warp < NBD) {
     const int cb = warp;
@@ -673,7 +672,8 @@ __device__ __forceinline__ void big_cell_body(const DpgPlanDev& P, const DpgLaun
 }
 
 template <int ZK>
-__global__ void __launch_bounds__(NT, 1) dpg_big_kernel(const __grid_constant__ DpgPlanDev P, const DpgLaunch L) {
+__global__ void __launch_bounds__(NT, 1) dpg_big_kernel(const __grid_constant__ DpgPlanDev P,
+                                                                  const __grid_constant__ DpgLaunch L) {
   const BigSm S = big_views(P);
   big_cta_setup(P, S);
   for (int cell = blockIdx.x; cell < L.C; cell += gridDim.x)

@@ -24,7 +24,8 @@ __device__ __forceinline__ void energy_residual(const DpgPlanDev& P, const DpgLa
 }
 
 template <int NBTM, int GTM, int BTW, int CH>
-__global__ void __launch_bounds__(NT, 1) dpg_energy_kernel(const __grid_constant__ DpgPlanDev P, const DpgLaunch L) {
+__global__ void __launch_bounds__(NT, 1) dpg_energy_kernel(const __grid_constant__ DpgPlanDev P,
+                                                                  const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   Ctx X;
   double* const sm = dpg_smem;
@@ -46,8 +47,8 @@ __global__ void __launch_bounds__(NT, 1) dpg_energy_kernel(const __grid_constant
     energy_residual(P, L, cell);
     __syncthreads();
     phase_gram<GTM, CH>(P, L, cell, X);
-    phase_factor(P, X);
-    phase_trsm<NBTM>(P, L, cell, X);
+    phase_factor(P);
+    phase_trsm<NBTM>(P, L, cell);
     // |L^-1 r|^2: row fcol of the W^T tiles of column tile fcol / 8
     const double* WT = sm + P.sm_w + (size_t)(P.fcol >> 3) * P.NBT * 64;
     const int fr = P.fcol & 7;
@@ -96,7 +97,8 @@ static KernelFn pick_energy_kernel(const DpgPlanDev* plan) {
 // factored solve overwrites B and F in place): W = L^-1 B as (C, M, N) "trial x
 // test" and y = L^-1 F as (C, N), user numbering, L the unscaled Cholesky factor of G.
 template <int NBTM, int GTM, int BTW, int CH>
-__global__ void __launch_bounds__(NT, 1) dpg_dls_kernel(const __grid_constant__ DpgPlanDev P, const DpgLaunch L) {
+__global__ void __launch_bounds__(NT, 1) dpg_dls_kernel(const __grid_constant__ DpgPlanDev P,
+                                                                  const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x;
   Ctx X;
   double* const sm = dpg_smem;
@@ -116,8 +118,8 @@ __global__ void __launch_bounds__(NT, 1) dpg_dls_kernel(const __grid_constant__ 
     phase_b<BTW>(P, L, cell, X);
     __syncthreads();
     phase_gram<GTM, CH>(P, L, cell, X);
-    phase_factor(P, X);
-    phase_trsm<NBTM>(P, L, cell, X);
+    phase_factor(P);
+    phase_trsm<NBTM>(P, L, cell);
     // W^T tile (J, I), element (r, c) = W[I*8 + c][J*8 + r]
     const double* WT = sm + P.sm_w;
     double* Wc = L.B + (size_t)cell * P.M * P.N;

@@ -598,6 +598,7 @@ static int big_layout(HostPlan* P) {
 // DPG_OK, -1 when it needs more shared memory than one CTA has, or a failure code.
 static int smem_layout(DpgPlanDev& g, int chg, bool adj_terms_ok) {
   g.chg = chg;
+  if (g.nbt16 < (g.nfp + g.ntp + 8) / 8) return fail(DPG_ERR_UNSUPPORTED, "trial tiles outnumber test tiles: condensation workspace overlaps K");
   auto al = [](int x) { return (x + 15) & ~15; };  // 128-byte aligned regions
   int o = 0;
   // Gram phase
@@ -611,8 +612,10 @@ static int smem_layout(DpgPlanDev& g, int chg, bool adj_terms_ok) {
   int gphase = o;
   // factor
   o = 0;
-  g.sm_gt = o; o += al(g.ngt * 64);
-  g.sm_linv = o; o += al(g.NBT * 64);
+  // inverse diagonal tiles behind G's and K's tiles: the condensation factors K in place
+  const int ksz = g.MBT * (g.MBT + 1) / 2 * 64;
+  g.sm_gt = o; o += al(std::max(g.ngt * 64, ksz));
+  g.sm_linv = o; o += al(std::max(g.NBT, g.MBT) * 64);
   g.sm_scale = o; o += al(g.Np);
   int fphase = o;
   // B phase (runs first; whole body available)
@@ -626,9 +629,6 @@ static int smem_layout(DpgPlanDev& g, int chg, bool adj_terms_ok) {
   g.sm_w = 0;
   int wsz = g.MBT * g.NBT * 64;
   g.sm_k = 0;
-  int ksz = g.MBT * (g.MBT + 1) / 2 * 64;
-  if (g.sm_linv < ksz || g.sm_linv + g.MBT * 64 > g.sm_linv + al(g.NBT * 64))
-    return fail(DPG_ERR_UNSUPPORTED, "trial tiles outnumber test tiles: condensation workspace overlaps K");
   int body = std::max(std::max(gphase, bphase), std::max(std::max(wsz, ksz), fphase));
   // reverse mode: S_A, then the pull-back staging (both reuse the body after the factor)
   {
@@ -645,13 +645,15 @@ static int smem_layout(DpgPlanDev& g, int chg, bool adj_terms_ok) {
     g.a_geo = q; q += al(std::max(DPG_CHA_HOST, g.ns * g.QS) * 24);
     g.a_beta = q; q += al(DPG_CHA_HOST * g.niprows * 4 * g.ntest);
     g.a_cbar = q; q += al(std::max(1, g.nslots * g.Ptot));
-    g.adj_ok = adj_terms_ok && std::max(sa_end, q) <= body && g.QB > 0;
+    const int ngt16 = g.nbt16 * (g.nbt16 + 1) / 2;
+    const int body16 = std::max(std::max(body, g.MBT * g.nbt16 * 64), (ngt16 + g.nbt16) * 64 + g.nbt16 * 8);
+    g.adj_ok = adj_terms_ok && std::max(sa_end, q) <= body16 && g.QB > 0;
+    if (g.adj_ok) body = std::max(body, std::max(sa_end, q));
   }
   g.sm_coef = al(body);
   g.sm_tiles = g.sm_coef + al(std::max(1, g.nslots * g.Ptot));
   g.sm_nodes = g.sm_tiles + al((g.ngb * (int)sizeof(DpgGTile) + 7) / 8);
-  g.sm_invd = g.sm_nodes + 192;
-  g.sm_total = g.sm_invd + al(std::max(g.Np, g.Mp));
+  g.sm_total = g.sm_nodes + 192;
   if ((size_t)g.sm_total * 8 > 232448) {
     return -1;
   }
@@ -754,6 +756,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
   // large-bucket kernel, whose tiles need test vars padded to 8 rows only (the single-CTA
   // kernel's 16 x 8 blocks need 16).
   bool big_pre = false;
+  int nbt16 = 0;  // test tiles with every var padded to 16 rows
   {
     int np16 = 0, nf = 0, nt = 0;
     for (int a = 0; a < D->n_test; a++) {
@@ -762,6 +765,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
                                                : card_hdiv_t(topo, d, std::max(V.poly_order, 1));
       np16 += (c + 15) & ~15;
     }
+    nbt16 = np16 / 8;
     for (int b = 0; b < D->n_trial; b++) {
       const dpg_var_desc& V = D->trial[b];
       if (V.kind == DPG_VAR_FIELD)
@@ -785,13 +789,16 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
       if (n < 1) return fail(DPG_ERR_INVALID_ARGUMENT, "HDIV test order must be >= 1");
       tv.card = card_hdiv_t(topo, d, n);
     } else return fail(DPG_ERR_INVALID_ARGUMENT, "test vars must be HGRAD or HDIV");
-    // rows padded to pairs of 8-row tiles (16x8 mma blocks never straddle two vars)
-    const int rows = big_pre ? (tv.card + 7) & ~7 : (tv.card + 15) & ~15;
+    // device rows: whole 8-row tiles.  The single-CTA kernel's 16x8 mma blocks never straddle two
+    // vars: the last block of a var with an odd number of tiles computes a second tile of zero
+    // slots and drops it, so only the staged slot rows are padded to 16 (padding the device rows
+    // too cost the factorisation and the solve up to a tenth more tiles per dimension)
+    const int rows = (tv.card + 7) & ~7;
     tv.dev_off = dev_row;
     tv.user_off = user_row;
     tv.ntile0 = dev_row / 8;
     tv.ntiles = rows / 8;
-    tv.ldA = ld_pad(rows);
+    tv.ldA = ld_pad(big_pre ? rows : (tv.card + 15) & ~15);
     tv.foff = foff;
     foff += 4 * tv.ldA;
     dev_row += rows;
@@ -802,6 +809,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
   g.N = user_row;
   g.Np = dev_row;
   g.NBT = g.Np / 8;
+  g.nbt16 = nbt16;
   if (g.NBT > DPG_MAX_NBT) g.big = 1;  // the large-bucket kernel
   // staged reference slots of all test vars at a list of volume-reference points
   auto fref_table = [&](const double* pts, int npts) {
@@ -889,8 +897,10 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
   g.nfp = pad8(g.nf);
   g.ntp = pad8(g.nt);
   g.nfb = g.nfp / 8;
-  g.fcol = g.nfp + g.ntp;
-  g.Mp = g.fcol + 8;
+  // the F column follows the traces in their last tile where that has room: a column tile less
+  // in the solve and in W^T W (on the 3D hex bucket 14 instead of 15)
+  g.fcol = g.nfp + g.nt;
+  g.Mp = pad8(g.fcol + 1);
   g.MBT = g.Mp / 8;
   if (g.MBT > DPG_MAX_MBT) g.big = 1;
   {
@@ -986,8 +996,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     g.hstride = off;
     std::vector<DpgGTile> tiles;
     std::vector<char> covered(g.NBT * (g.NBT + 1) / 2, 0);
-    // 16 x 8 blocks of the single-CTA kernel (large plans have none: their test vars may
-    // have an odd number of 8-row tiles)
+    // 16 x 8 blocks of the single-CTA kernel (large plans have none)
     for (int a = 0; a < g.ntest && !g.big; a++)
       for (int rp = 0; rp < g.test[a].ntiles; rp += 2) {
         const int I = g.test[a].ntile0 + rp;
@@ -996,10 +1005,12 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
             const int J = g.test[b].ntile0 + jj;
             if (J > I + 1) continue;
             if (pidx[a * g.ntest + b] < 0) continue;
+            const bool half = rp + 1 >= g.test[a].ntiles;
+            if (half && J > I) continue;
             if (J <= I) covered[I * (I + 1) / 2 + J] = 1;
-            covered[(I + 1) * (I + 2) / 2 + J] = 1;
+            if (!half) covered[(I + 1) * (I + 2) / 2 + J] = 1;
             DpgGTile t;
-            t.I = (int16_t)I; t.J = (int16_t)J;
+            t.I = (int16_t)I; t.J = (int16_t)(J | (half ? 0x100 : 0));
             t.aoff = g.test[a].foff + rp * 8;
             t.lda = (int16_t)g.test[a].ldA;
             t.boff = g.hoff[pidx[a * g.ntest + b]] + jj * 8;
@@ -1163,7 +1174,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     // 16x8 blocks (row-tile pairs of the block's test var) of the active (var, column tile) blocks
     for (int kb = 0; kb < S.nblk; kb++) {
       const DpgTestVar& V = g.test[S.blk[kb].var];
-      for (int I = V.ntile0; I < V.ntile0 + V.ntiles; I += 2) btiles.push_back(make_int4(I, S.blk[kb].J, kb, 0));
+      for (int I = V.ntile0; I < V.ntile0 + V.ntiles; I += 2) btiles.push_back(make_int4(I, S.blk[kb].J, kb, I + 1 < V.ntile0 + V.ntiles ? 0 : 1));
     }
     S.ntile = (int)btiles.size() - S.tile0;
     if (!g.big && (S.ntile + DPG_NWARPS - 1) / DPG_NWARPS > DPG_MAX_BTW)
@@ -1414,9 +1425,9 @@ int dpg_make_solve_plan(int N, int M, DpgPlanDev* out) {
   g.d = 2; g.nv = 0; g.ns = 0;
   g.N = N; g.M = M; g.nf = M; g.nt = 0;
   g.Np = pad8(N); g.NBT = g.Np / 8;
-  g.nfp = pad8(M); g.ntp = 0; g.nfb = g.nfp / 8; g.fcol = g.nfp; g.Mp = g.nfp + 8; g.MBT = g.Mp / 8;
+  g.nfp = pad8(M); g.ntp = 0; g.nfb = g.nfp / 8; g.fcol = M; g.Mp = pad8(M + 1); g.MBT = g.Mp / 8;
   if (g.NBT > DPG_MAX_NBT) return dpg::fail(DPG_ERR_UNSUPPORTED, "N too large for the single-CTA solve (N <= 192)");
-  if (g.MBT > DPG_MAX_MBT) return dpg::fail(DPG_ERR_UNSUPPORTED, "M too large for the single-CTA solve (M <= 120)");
+  if (g.nfp + 8 > 8 * DPG_MAX_MBT) return dpg::fail(DPG_ERR_UNSUPPORTED, "M too large for the single-CTA solve (M <= 120)");
   g.ntest = 1;
   g.test[0].card = N; g.test[0].ntiles = g.NBT;
   g.ntrial = 1;
@@ -1433,8 +1444,7 @@ int dpg_make_solve_plan(int N, int M, DpgPlanDev* out) {
   g.sm_nodes = g.sm_tiles;
   g.scratch_per_cta = 0;
   g.chg = DPG_CHG;  // no Gram phase; selects the standard kernel instances
-  g.sm_invd = g.sm_nodes + 192;
-  g.sm_total = g.sm_invd + al(std::max(g.Np, g.Mp));
+  g.sm_total = g.sm_nodes + 192;
   return DPG_OK;
 }
 

@@ -53,6 +53,9 @@ struct DpgLaunch {
 };
 
 int dpg_configure_kernels(const DpgPlanDev* plan);
+int dpg_configure_adjoint(const DpgPlanDev* plan, int bytes);
+int dpg_configure_big(const DpgPlanDev* plan);
+int dpg_launch_big(const DpgPlanDev* plan, const DpgLaunch* L, cudaStream_t stream);
 int dpg_launch_assemble(const DpgPlanDev* plan, const DpgPlanDev* d_plan, const DpgLaunch* L, cudaStream_t stream);
 int dpg_host_pipeline(const DpgPlanDev* plan, const DpgPlanDev* d_plan, void** d_ws, size_t* ws_bytes,
                       cudaStream_t* streams, int C, const double* nodes, const int8_t* parity, const double* coeff,

@@ -1,0 +1,1119 @@
+// dpg_phases.cuh — the phases of the per-cell assembly and their device helpers, shared by the
+// kernels that walk cells with one CTA (assembly, work queue, reverse mode, energy error, DLS)
+// and by the large-bucket kernel.  Each kernel family is a translation unit of its own.
+#pragma once
+#include "../../include/dpg_b200.h"
+#include "dpg_internal.h"
+#include "dpg_plan.h"
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <cstring>
+#include <mutex>
+#include <vector>
+
+// The CTA's dynamic shared memory; every shared pointer below is derived from it
+// so the compiler keeps shared-space (LDS/STS) addressing inside the phase functions.
+extern __shared__ __align__(128) double dpg_smem[];
+
+namespace {
+
+constexpr int NT = DPG_NTHREADS;
+constexpr int MBAR_SPIN_LIMIT = 1 << 22;
+constexpr int ERR_TIMEOUT_FLAG = 0x7fff0000;
+constexpr int GEO = 24;  // doubles per point geometry record: J(9) Ji(9) det w*|J| n(3) 1/det
+
+__device__ __forceinline__ void dmma(double2& c, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c.x), "+d"(c.y)
+               : "d"(a), "d"(b));
+}
+
+// D(16x8) += A(16x16) B(16x8), FP64.  Fragments: a[2i] = A[g][t+4i], a[2i+1] = A[g+8][t+4i],
+// b[i] = B[t+4i][g]; c = {C[g][2t], C[g][2t+1], C[g+8][2t], C[g+8][2t+1]}.
+__device__ __forceinline__ void dmma16(double* c, const double* a, const double* b) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, "
+      "{%12,%13,%14,%15}, {%0,%1,%2,%3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]),
+        "d"(b[1]), "d"(b[2]), "d"(b[3]));
+}
+
+// D(16x8) += A(16x8) * B(8x8): a0 = A[g][t], a1 = A[g+8][t], a2 = A[g][t+4], a3 = A[g+8][t+4];
+// b0 = B[t][g], b1 = B[t+4][g]; c_lo holds rows g, c_hi rows g+8 (columns 2t, 2t+1 each).
+__device__ __forceinline__ void dmma16x8(double2& c_lo, double2& c_hi, double a0, double a1, double a2, double a3,
+                                         double b0, double b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+d"(c_lo.x), "+d"(c_lo.y), "+d"(c_hi.x), "+d"(c_hi.y)
+      : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+}
+
+// Global -> shared bulk copy completing on an mbarrier (16-byte aligned, bytes % 16 == 0).
+__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* b) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(b))
+               : "memory");
+}
+
+// Bounded wait on an mbarrier phase; false if the limit was reached.
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, int limit = MBAR_SPIN_LIMIT) {
+  for (int it = 0; it < limit; it++) {
+    uint32_t done;
+    asm volatile(
+        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(done)
+        : "r"(smem_u32(b)), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
+// AK layout index of element (r, c) of an 8x8 tile
+__device__ __forceinline__ int ak(int r, int c) { return ((c >> 2) * 8 + r) * 4 + (c & 3); }
+
+// Offset of the C-fragment pair (g, 2t..2t+1) in AK layout
+__device__ __forceinline__ int ak_cfrag(int g, int t) { return ((t >> 1) * 8 + g) * 4 + (t & 1) * 2; }
+
+// Convert a C-fragment (rows g, cols 2t, 2t+1) into the two B-fragments of the
+// same 8x8 matrix used as the k x n operand: B_h[t][g] = X[4h + t][g].
+__device__ __forceinline__ void cfrag_to_bfrag(const double2 c, int lane, double& b0, double& b1) {
+  const int g = lane >> 2, t = lane & 3;
+  const int src0 = t * 4 + (g >> 1);
+  const int src1 = 16 + t * 4 + (g >> 1);
+  double x0 = __shfl_sync(0xffffffffu, c.x, src0);
+  double y0 = __shfl_sync(0xffffffffu, c.y, src0);
+  double x1 = __shfl_sync(0xffffffffu, c.x, src1);
+  double y1 = __shfl_sync(0xffffffffu, c.y, src1);
+  b0 = (g & 1) ? y0 : x0;
+  b1 = (g & 1) ? y1 : x1;
+}
+
+// Geometry record of one point: Jacobian, inverse, determinant, weighted
+// measure (w*detJ, or w*|side Jacobian| when tang != nullptr) and, on a side,
+// the outward unit normal.  All vertex-shape derivatives are loaded up front.
+__device__ __forceinline__ void point_geometry(int d, int nv, const double* __restrict__ X,
+                                               const double* __restrict__ dN, double w,
+                                               const double* __restrict__ tang, double* gq) {
+  double dn[24];
+#pragma unroll
+  for (int i = 0; i < 24; i++) dn[i] = (i < nv * d) ? __ldg(dN + i) : 0.0;
+  double tg[6];
+  if (tang) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) tg[i] = __ldg(tang + i);
+  }
+  double J[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) J[i] = 0.0;
+  if (d == 3) {
+#pragma unroll
+    for (int a = 0; a < 8; a++) {
+      if (a < nv) {
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          double xa = X[a * 3 + i];
+#pragma unroll
+          for (int j = 0; j < 3; j++) J[i * 3 + j] += xa * dn[a * 3 + j];
+        }
+      }
+    }
+  } else {
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+      if (a < nv) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          double xa = X[a * 2 + i];
+#pragma unroll
+          for (int j = 0; j < 2; j++) J[i * 3 + j] += xa * dn[a * 2 + j];
+        }
+      }
+    }
+  }
+  double Ji[9], det;
+  if (d == 2) {
+    det = J[0] * J[4] - J[1] * J[3];
+    double id = 1.0 / det;
+    Ji[0] = J[4] * id; Ji[1] = -J[1] * id; Ji[2] = 0;
+    Ji[3] = -J[3] * id; Ji[4] = J[0] * id; Ji[5] = 0;
+    Ji[6] = 0; Ji[7] = 0; Ji[8] = 1;
+  } else {
+    double c00 = J[4] * J[8] - J[5] * J[7];
+    double c01 = J[5] * J[6] - J[3] * J[8];
+    double c02 = J[3] * J[7] - J[4] * J[6];
+    det = J[0] * c00 + J[1] * c01 + J[2] * c02;
+    double id = 1.0 / det;
+    Ji[0] = c00 * id;
+    Ji[3] = c01 * id;
+    Ji[6] = c02 * id;
+    Ji[1] = (J[2] * J[7] - J[1] * J[8]) * id;
+    Ji[4] = (J[0] * J[8] - J[2] * J[6]) * id;
+    Ji[7] = (J[1] * J[6] - J[0] * J[7]) * id;
+    Ji[2] = (J[1] * J[5] - J[2] * J[4]) * id;
+    Ji[5] = (J[2] * J[3] - J[0] * J[5]) * id;
+    Ji[8] = (J[0] * J[4] - J[1] * J[3]) * id;
+  }
+#pragma unroll
+  for (int i = 0; i < 9; i++) { gq[i] = J[i]; gq[9 + i] = Ji[i]; }
+  gq[18] = det;
+  gq[23] = 1.0 / det;
+  gq[20] = gq[21] = gq[22] = 0.0;
+  if (!tang) {
+    gq[19] = w * det;
+    return;
+  }
+  double T0[3] = {0, 0, 0}, T1[3] = {0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      T0[i] += J[i * 3 + j] * tg[j];
+      T1[i] += J[i * 3 + j] * tg[3 + j];
+    }
+  double meas;
+  if (d == 2) {
+    meas = sqrt(T0[0] * T0[0] + T0[1] * T0[1]);
+    gq[20] = T0[1] / meas;
+    gq[21] = -T0[0] / meas;
+  } else {
+    double c0 = T0[1] * T1[2] - T0[2] * T1[1];
+    double c1 = T0[2] * T1[0] - T0[0] * T1[2];
+    double c2 = T0[0] * T1[1] - T0[1] * T1[0];
+    meas = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
+    gq[20] = c0 / meas; gq[21] = c1 / meas; gq[22] = c2 / meas;
+  }
+  gq[19] = w * meas;
+}
+
+// Row `m` of the slot transform T of a test var at a point: physical value of
+// the operator in physical slot m = sum_k T[m][k] * reference slot k.
+//   HGRAD slots (value, d/dx_0..): T[0][0] = 1, T[1+c][1+j] = Ji[j][c]
+//   HDIV  slots (v_0.., div):      T[c][j] = J[c][j]/det, T[d][d] = 1/det
+__device__ __forceinline__ void trow_slot(int space, int d, int m, const double* gq, double* r) {
+  r[0] = r[1] = r[2] = r[3] = 0.0;
+  if (space == DPG_SPACE_HGRAD) {
+    if (m == 0) r[0] = 1.0;
+    else if (m <= d) {
+      int c = m - 1;
+      for (int j = 0; j < d; j++) r[1 + j] = gq[9 + j * 3 + c];
+    }
+  } else {
+    const double id = gq[23];
+    if (m < d) {
+      for (int j = 0; j < d; j++) r[j] = gq[m * 3 + j] * id;
+    } else if (m == d) {
+      r[d] = id;
+    }
+  }
+}
+
+// Row of T for a physical operator (incl. tau . n on a side; normal at gq[20..22]).
+__device__ __forceinline__ void trow_op(int space, int d, int op, const double* gq, double* r) {
+  if (space == DPG_SPACE_HGRAD) {
+    trow_slot(space, d, op == DPG_OP_VALUE ? 0 : 1 + (op - DPG_OP_DX), gq, r);
+    return;
+  }
+  if (op == DPG_OP_DOT_NORMAL) {
+    const double id = gq[23];
+    r[0] = r[1] = r[2] = r[3] = 0.0;
+    for (int c = 0; c < d; c++)
+      for (int j = 0; j < d; j++) r[j] += gq[20 + c] * gq[c * 3 + j] * id;
+    return;
+  }
+  trow_slot(space, d, op == DPG_OP_DIV ? d : op - DPG_OP_X, gq, r);
+}
+
+// Element (r, c) of the symmetric matrix stored as lower AK tiles at base.
+__device__ __forceinline__ double sym_get(const double* base, int r, int c) {
+  if (r < c) { int x = r; r = c; c = x; }
+  int I = r >> 3, J = c >> 3;
+  return base[(I * (I + 1) / 2 + J) * 64 + ak(r & 7, c & 7)];
+}
+
+struct Ctx {
+  uint32_t* phase;     // mbarrier use counters [4]
+};
+
+// Shared-memory views of the persistent region (derived from dpg_smem).
+#define DPG_SMEM_VIEWS(P)                                                              \
+  double* const sm = dpg_smem;                                                         \
+  int* const flag_s = reinterpret_cast<int*>(sm + (P).sm_nodes + 24);                  \
+  uint64_t* const mbar_s = reinterpret_cast<uint64_t*>(sm + (P).sm_nodes + 26);        \
+  const int* const tri_s = reinterpret_cast<const int*>(sm + (P).sm_nodes + 32);       \
+  const double* const nodes_s = sm + (P).sm_nodes;                                     \
+  const double* const coef_s = sm + (P).sm_coef;                                       \
+  (void)flag_s; (void)mbar_s; (void)tri_s; (void)nodes_s; (void)coef_s;
+
+// Factor the diagonal tile k (one warp) and invert the factor.  Every lane loads the lower
+// triangle and runs the whole factorisation in its own registers, so the pivot chain is eight
+// reciprocal square roots (70 cycles each), each followed by one multiply and one FMA (8), with no
+// shuffle on it; lane c forms column c of the inverse tile L_kk^-1 row by row beside it.  Only
+// the inverse (AK layout, linv[64 k]) is written: the panel and the solves multiply by it,
+// and nothing reads L_kk.  First failing pivot (1-based) -> *flag (sign sgn).
+__device__ __forceinline__ void factor_diag(const double* __restrict__ T, int k, int* flag, int sgn, double* linv) {
+  const int lane = threadIdx.x & 31;
+  const double* Tkk = T + (k * (k + 1) / 2 + k) * 64;
+  double a[36];  // a[r (r + 1) / 2 + c], c <= r
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int c = 0; c <= r; c++) a[r * (r + 1) / 2 + c] = Tkk[ak(r, c)];
+  const int c0 = lane & 7;
+  double x[8];
+  bool failed = false;
+  int fail_j = 0;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const double piv = a[j * (j + 1) / 2 + j];
+    if (!(piv > 0.0) && !failed) { failed = true; fail_j = j; }
+    const double inv = rsqrt(piv);
+#pragma unroll
+    for (int r = j + 1; r < 8; r++) a[r * (r + 1) / 2 + j] *= inv;
+#pragma unroll
+    for (int c = j + 1; c < 8; c++)
+#pragma unroll
+      for (int r = c; r < 8; r++) a[r * (r + 1) / 2 + c] -= a[r * (r + 1) / 2 + j] * a[c * (c + 1) / 2 + j];
+    // row j of the inverse's column c0
+    double v = (j == c0) ? 1.0 : 0.0;
+#pragma unroll
+    for (int m = 0; m < j; m++) v -= a[j * (j + 1) / 2 + m] * x[m];
+    x[j] = (j < c0) ? 0.0 : v * inv;
+  }
+  if (lane == 0 && failed && *flag == 0) *flag = sgn * (k * 8 + fail_j + 1);
+  if (lane < 8) {
+#pragma unroll
+    for (int r = 0; r < 8; r++) linv[k * 64 + ak(r, c0)] = x[r];
+  }
+  __syncwarp();
+}
+
+// The blocked Cholesky of 8x8 tiles (AK layout, lower tiles row by row) is left-looking: after
+// step k's panel L_ik = A_ik L_kk^-T, column k+1 receives all its updates
+// A_i,k+1 -= sum_{j <= k} L_ij L_k+1,j^T at once, each tile in one warp's registers.  A
+// right-looking update reads and writes every trailing tile in every step (7.4 K cycles for
+// the first step of 22 tiles, a dozen warps each waiting on load, two products and store per
+// tile); here a tile is loaded and stored once, its products follow one another in the
+// same order (the same sums), and the work of a step stays below the time of the diagonal tile
+// next door.  That chain of diagonal tiles is what bounds the factorisation: warp 0 does
+// nothing else, with its sub-partition to itself (warps 4, 8, 12 only keep the barriers), and it
+// needs from the others only the sum over j < k of tile (k+1, k+1), formed a step ahead.
+constexpr int CHOL_NW = DPG_NWARPS - DPG_NWARPS / 4;  // warps that update: those of the other sub-partitions
+
+__device__ __forceinline__ int chol_rank(int warp) { return warp - (warp >> 2) - 1; }
+
+// Warp 0: panel tile (k+1, k), then update and factorisation of tile (k+1, k+1).
+__device__ __forceinline__ void chol_chain(double* T, int nb, int nsteps, int* flag, int sgn, double* linv) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  factor_diag(T, 0, flag, sgn, linv);
+  asm volatile("bar.sync 0, %0;" ::"n"(NT) : "memory");
+#pragma unroll 1
+  for (int k = 0; k < nsteps; k++) {
+    const int i = k + 1;
+    double* Lik = T + (i * (i + 1) / 2 + k) * 64;
+    if (i < nb) {
+      const double* Li = linv + k * 64;
+      const double a0 = Lik[lane], a1 = Lik[32 + lane];
+      double2 c = make_double2(0.0, 0.0);
+      dmma(c, a0, Li[lane]);
+      dmma(c, a1, Li[32 + lane]);
+      __syncwarp();
+      *reinterpret_cast<double2*>(Lik + ak_cfrag(g, t)) = c;
+    }
+    asm volatile("bar.arrive 1, %0;" ::"n"(NT) : "memory");  // it needs no other warp's panel tile
+    __syncwarp();
+    if (i < nsteps) {
+      double* Tii = Lik + 64;
+      double2 c = *reinterpret_cast<const double2*>(Tii + ak_cfrag(g, t));
+      dmma(c, -Lik[lane], Lik[lane]);
+      dmma(c, -Lik[32 + lane], Lik[32 + lane]);
+      *reinterpret_cast<double2*>(Tii + ak_cfrag(g, t)) = c;
+      __syncwarp();
+      factor_diag(T, i, flag, sgn, linv);
+    }
+    asm volatile("bar.sync 0, %0;" ::"n"(NT) : "memory");
+  }
+}
+
+// Panel tiles L_ik = A_ik L_kk^-T of step k, i > k + 1 (warps of rank r).
+__device__ __forceinline__ void chol_panel(double* T, const double* Li, int nb, int k, int r, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll 1
+  for (int i = k + 2 + r; i < nb; i += CHOL_NW) {
+    double* Tik = T + (i * (i + 1) / 2 + k) * 64;
+    const double a0 = Tik[lane], a1 = Tik[32 + lane];
+    double2 c = make_double2(0.0, 0.0);
+    dmma(c, a0, Li[lane]);
+    dmma(c, a1, Li[32 + lane]);
+    __syncwarp();
+    *reinterpret_cast<double2*>(Tik + ak_cfrag(g, t)) = c;
+  }
+}
+
+// A_ij -= sum_{m < n} L_im L_jm^T of one tile.
+__device__ __forceinline__ void chol_tile(double* T, int i, int j, int n, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  const double* pa = T + (i * (i + 1) / 2) * 64 + lane;
+  const double* pb = T + (j * (j + 1) / 2) * 64 + lane;
+  double* C = T + (i * (i + 1) / 2 + j) * 64 + ak_cfrag(g, t);
+  double2 c = *reinterpret_cast<const double2*>(C);
+#pragma unroll 2
+  for (int m = 0; m < n; m++) {
+    const double a0 = -pa[m * 64], a1 = -pa[m * 64 + 32];
+    const double b0 = pb[m * 64], b1 = pb[m * 64 + 32];
+    dmma(c, a0, b0);
+    dmma(c, a1, b1);
+  }
+  *reinterpret_cast<double2*>(C) = c;
+}
+
+// After the panel of step k: column k+1 below its diagonal tile, and tile (k+2, k+2) up to
+// column k (warps of rank r).
+__device__ __forceinline__ void chol_column(double* T, int nb, int nsteps, int k, int r, int lane) {
+  if (k + 1 >= nsteps) return;
+#pragma unroll 1
+  for (int e = r; e < nb - 1 - k; e += CHOL_NW) {
+    if (e > 0) chol_tile(T, k + 1 + e, k + 1, k + 1, lane);
+    else if (k + 2 < nsteps) chol_tile(T, k + 2, k + 2, k + 1, lane);
+  }
+}
+
+// Factors the leading nsteps tiles of a tile-lower matrix with nb tiles in shared memory; the
+// trailing block is left with its Schur complement.  linv (nsteps x 64) receives the
+// inverses of the diagonal tiles.
+__device__ __noinline__ void tile_cholesky(int T_off, int nb, int nsteps, int flag_idx, int sgn, int tri_off,
+                                           int linv_off) {
+  double* const T = dpg_smem + T_off;
+  int* const flag = reinterpret_cast<int*>(dpg_smem) + flag_idx;
+  const int* const tri = reinterpret_cast<const int*>(dpg_smem + tri_off);
+  double* const linv = dpg_smem + linv_off;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (nsteps <= 0) return;
+  if (warp == 0) {
+    chol_chain(T, nb, nsteps, flag, sgn, linv);
+  } else {
+    const int r = chol_rank(warp);
+    asm volatile("bar.sync 0, %0;" ::"n"(NT) : "memory");
+#pragma unroll 1
+    for (int k = 0; k < nsteps; k++) {
+      if (warp & 3) chol_panel(T, linv + k * 64, nb, k, r, lane);
+      asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+      if (warp & 3) chol_column(T, nb, nsteps, k, r, lane);
+      asm volatile("bar.sync 0, %0;" ::"n"(NT) : "memory");
+    }
+  }
+  // the trailing block
+  const int m = nb - nsteps, ntr = m * (m + 1) / 2;
+#pragma unroll 1
+  for (int u = warp; u < ntr; u += DPG_NWARPS) chol_tile(T, nsteps + (tri[u] & 255), nsteps + (tri[u] >> 8), nsteps, lane);
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// Phase 1: B and F -> per-CTA scratch (or the B/F outputs in parts mode)
+// ---------------------------------------------------------------------------
+template <int BTW>
+__device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, int cell, const Ctx& X) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int d = P.d, nv = P.nv;
+  DPG_SMEM_VIEWS(P);
+  double* geo = sm + P.b_geo;
+  double* U = sm + P.b_u;
+  const int8_t* par_c = L.parity + (size_t)cell * P.ns;
+  double2* scr = reinterpret_cast<double2*>(L.scratch + (size_t)blockIdx.x * P.scratch_per_cta);
+  // prologue: first chunk's records in flight while the geometry is computed
+  int first_seg = 0;
+  while (first_seg < P.nseg && P.seg[first_seg].nterm == 0) first_seg++;
+  if (tid == 0 && first_seg < P.nseg) {
+    const DpgSeg& S = P.seg[first_seg];
+    const uint32_t bytes = (uint32_t)(((min(S.chunk, S.npts) + 3) & ~3) * S.rec_len * sizeof(double));
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_expect_tx(&mbar_s[2], bytes);
+    bulk_g2s(sm + P.b_rec0, S.rec, bytes, &mbar_s[2]);
+  }
+  // [B | F] tiles accumulate in this CTA's scratch slot, C-fragment layout per tile
+  for (int i = tid; i < P.MBT * P.NBT * 32; i += NT) scr[i] = make_double2(0.0, 0.0);
+  for (int q = tid; q < P.nbpts; q += NT)
+    point_geometry(d, nv, nodes_s, P.dNB + (size_t)q * nv * d, P.wB[q], q >= P.QB ? P.tangB + (size_t)q * 6 : nullptr,
+                   geo + q * GEO);
+  // separable side terms, while the first volume chunk is in flight: per-point factors,
+  // then one thread per entry (scratch element); entries are unique, and an element
+  // that a bilinear block also writes is read-modified-written (the blocks add to it
+  // after the chunk loop's barriers)
+  if (P.nse > 0) {
+    double* fac = sm + P.b_fac;  // [nse][QS]
+    __syncthreads();             // geometry complete, scratch zeroed
+    for (int task = tid; task < P.nse * P.QS; task += NT) {
+      const int se = task / P.QS, q = task - se * P.QS;
+      const DpgSideTerm& E = P.se[se];
+      const double* gq = geo + (P.QB + E.side * P.QS + q) * GEO;
+      double v = E.coef;
+      if (E.use_meas) v *= gq[19];
+      if (E.slot >= 0) v *= coef_s[E.slot * P.Ptot + E.pbase + q];
+      if (E.normal_comp >= 0) v *= gq[20 + E.normal_comp];
+      if (E.flux) v *= (double)par_c[E.side];
+      fac[task] = v;
+    }
+    __syncthreads();
+    double* scd = reinterpret_cast<double*>(scr);
+    for (int e = tid; e < P.nsent; e += NT) {
+      const int4 en = __ldg(P.sent + e);
+      double acc = 0.0;
+      if (en.z == 1) {
+        const double* f = fac + (en.w & 0xffff) * P.QS;
+        const double* w = P.scon_w + en.y;
+        for (int q = 0; q < P.QS; q++) acc += __ldg(w + (size_t)q * P.ncon) * f[q];
+      } else {
+        for (int c = en.y; c < en.y + en.z; c++) {
+          const double* f = fac + __ldg(P.scon_se + c) * P.QS;
+          for (int q = 0; q < P.QS; q++) acc += __ldg(P.scon_w + (size_t)q * P.ncon + c) * f[q];
+        }
+      }
+      if (en.w >> 16) scd[en.x] = acc;
+      else scd[en.x] += acc;
+    }
+  }
+  int gc = 0;  // global chunk counter (buffer parity)
+  for (int sgi = first_seg; sgi < P.nseg; sgi++) {
+    const DpgSeg& S = P.seg[sgi];
+    if (S.nterm == 0) continue;
+    // this warp's active 16x8 blocks of the segment: operand offsets and accumulators
+    const int bbase = S.ntile / DPG_NWARPS, bextra = S.ntile % DPG_NWARPS;
+    const int my0 = S.tile0 + warp * bbase + min(warp, bextra);
+    const int nmine = bbase + (warp < bextra ? 1 : 0);
+    uint32_t pk[BTW];
+    double acc[BTW][4];
+#pragma unroll
+    for (int u = 0; u < BTW; u++) {
+      acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0;
+      uint32_t v = 0;
+      if (u < nmine) {
+        const int4 td = P.btiles[my0 + u];
+        const DpgBBlock& Bk = S.blk[td.z];
+        const DpgTestVar& V = P.test[Bk.var];
+        v = (uint32_t)(V.foff + t * V.ldA + (td.x - V.ntile0) * 8 + g) | ((uint32_t)(Bk.off + t * DPG_ULD + g) << 16);
+      }
+      pk[u] = v;
+    }
+    for (int c = 0; c < S.nchunk; c++, gc++) {
+      const int buf = gc & 1;
+      double* rec = sm + (buf ? P.b_rec1 : P.b_rec0);
+      __syncthreads();  // the other buffer and U are free; geometry is complete
+      if (tid == 0) {
+        // prefetch the next chunk (this segment or the next one with terms)
+        int ns = sgi, nc = c + 1;
+        if (nc >= S.nchunk) {
+          ns = sgi + 1;
+          nc = 0;
+          while (ns < P.nseg && P.seg[ns].nterm == 0) ns++;
+        }
+        if (ns < P.nseg) {
+          const DpgSeg& S2 = P.seg[ns];
+          // the records of the chunk's points, rounded up to a whole k-step (the table is padded)
+          const uint32_t bytes =
+              (uint32_t)(((min(S2.chunk, S2.npts - nc * S2.chunk) + 3) & ~3) * S2.rec_len * sizeof(double));
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          mbar_expect_tx(&mbar_s[2 + (buf ^ 1)], bytes);
+          bulk_g2s(sm + (buf ? P.b_rec0 : P.b_rec1), S2.rec + (size_t)nc * S2.chunk * S2.rec_len, bytes,
+                   &mbar_s[2 + (buf ^ 1)]);
+        }
+        if (!mbar_wait(&mbar_s[2 + buf], X.phase[2 + buf] & 1)) flag_s[2] = 1;
+      }
+      X.phase[2 + buf]++;
+      const int q0 = c * S.chunk;
+      const int nq = min(S.chunk, S.npts - q0);
+      __syncthreads();
+      // U blocks: U[lq][blk][m][col] = sum over the block's terms of
+      //   (w*|J| * coef * slot * (n) * (parity) * T_op[m]) * trial value
+      for (int task = tid; task < S.chunk * S.nblk * 8; task += NT) {
+        const int lq = task / (S.nblk * 8);
+        const int rem = task - lq * S.nblk * 8;
+        const int kb = rem >> 3, cl = rem & 7;
+        const DpgBBlock& Bk = S.blk[kb];
+        const int col = Bk.J * 8 + cl;
+        double u0 = 0.0, u1 = 0.0, u2 = 0.0, u3 = 0.0;
+        if (lq < nq) {
+          const int q = q0 + lq;
+          const double* rq = rec + lq * S.rec_len;
+          const double* gq = geo + (S.geo0 + q) * GEO;
+          const int space = P.test[Bk.var].space;
+          for (int i = 0; i < Bk.nt; i++) {
+            const int lt = Bk.terms[i];
+            const DpgBTerm& Tm = P.bterm[S.term0 + lt];
+            const int mm = col - Tm.col0;
+            if (mm < 0 || mm >= Tm.ncol) continue;
+            double v = gq[19] * Tm.coef * rq[S.tvoff[lt] + mm];
+            if (Tm.slot >= 0) v *= coef_s[Tm.slot * P.Ptot + S.pbase + q];
+            if (Tm.normal_comp >= 0) v *= gq[20 + Tm.normal_comp];
+            if (Tm.kind == DPG_VAR_FLUX) v *= (double)par_c[S.side];
+            double tr[4];
+            trow_op(space, d, Tm.test_op, gq, tr);
+            u0 += tr[0] * v; u1 += tr[1] * v; u2 += tr[2] * v; u3 += tr[3] * v;
+          }
+        }
+        double* uq = U + lq * S.ustride + Bk.off + cl;
+        uq[0] = u0; uq[DPG_ULD] = u1; uq[2 * DPG_ULD] = u2; uq[3 * DPG_ULD] = u3;
+      }
+      __syncthreads();
+      // DMMA over this warp's active blocks of the segment: m16n8k16, one k-step = 4 points x 4 slots
+#pragma unroll 1
+      for (int s4 = 0; s4 < nq; s4 += 4) {
+        const double* ra = rec + s4 * S.rec_len;
+        const double* ub = U + s4 * S.ustride;
+        uint32_t prevA = 0xffffffffu;
+        double av[8];
+#pragma unroll
+        for (int u = 0; u < BTW; u++) {
+          if (u < nmine) {
+            const uint32_t ao = pk[u] & 0xffffu, bo = pk[u] >> 16;
+            if (ao != prevA) {
+#pragma unroll
+              for (int i = 0; i < 4; i++) {
+                av[2 * i] = ra[i * S.rec_len + ao];
+                av[2 * i + 1] = ra[i * S.rec_len + ao + 8];
+              }
+              prevA = ao;
+            }
+            double bv[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) bv[i] = ub[i * S.ustride + bo];
+            dmma16(acc[u], av, bv);
+          }
+        }
+      }
+    }
+    // segment contributions into the scratch tiles (each block has one owner per segment)
+#pragma unroll
+    for (int u = 0; u < BTW; u++) {
+      if (u < nmine) {
+        const int4 td = P.btiles[my0 + u];
+        const int s0 = (td.y * P.NBT + td.x) * 32 + lane;
+        double2 v0 = scr[s0];
+        v0.x += acc[u][0]; v0.y += acc[u][1];
+        scr[s0] = v0;
+        if (!td.w) {  // the block has a second row tile
+          double2 v1 = scr[s0 + 32];
+          v1.x += acc[u][2]; v1.y += acc[u][3];
+          scr[s0 + 32] = v1;
+        }
+      }
+    }
+  }
+  if (!L.parts) return;
+  __syncthreads();
+  double* Bc = L.B ? L.B + (size_t)cell * P.M * P.N : nullptr;
+  double* Fc = L.F ? L.F + (size_t)cell * P.N : nullptr;
+  for (int tile = warp; tile < P.MBT * P.NBT; tile += DPG_NWARPS) {
+    const int J = tile / P.NBT, I = tile - J * P.NBT;
+    const double2 v = scr[tile * 32 + lane];
+    const int ur = P.dev2user_test[I * 8 + g];
+    if (ur < 0) continue;
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int col = J * 8 + 2 * t + e;
+      const double x = e ? v.y : v.x;
+      const int uc = P.dev2user_trial[col];
+      if (Bc && uc >= 0) Bc[(size_t)uc * P.N + ur] = x;
+      if (Fc && col == P.fcol) Fc[ur] = x;
+    }
+  }
+}
+
+// The Gram chunk loop for CH points per chunk (compile-time, so the h and DMMA loops
+// unroll completely).
+// Every P.gflush chunks (except after the last) each thread adds the accumulators of its
+// flushed blocks (P.gflushbits) into its own running sums in gsum ([block][lane][4]; plain
+// L2 loads and stores, one writer per element, so the order of additions is fixed) and
+// restarts them from zero.
+template <int GTM, int CH>
+__device__ __forceinline__ void gram_chunks(const DpgPlanDev& P, const Ctx& X, const double* Dm, double* hb, int nunit,
+                                            int ntw, const uint32_t (&pk)[GTM], double (&acc)[GTM][4],
+                                            double* __restrict__ gsum) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  DPG_SMEM_VIEWS(P);
+  const int nch = P.QGpad / CH;
+  const uint32_t chunk_bytes = (uint32_t)(CH * P.featstride * sizeof(double));
+  for (int c = 0; c < nch; c++) {
+    const int buf = c & 1;
+    const double* fref = sm + (buf ? P.g_fref1 : P.g_fref0);
+    if (tid == 0) {
+      if (c + 1 < nch) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_expect_tx(&mbar_s[buf ^ 1], chunk_bytes);
+        bulk_g2s(sm + (buf ? P.g_fref0 : P.g_fref1), P.frefG + (size_t)(c + 1) * CH * P.featstride,
+                 chunk_bytes, &mbar_s[buf ^ 1]);
+      }
+      if (!mbar_wait(&mbar_s[buf], X.phase[buf] & 1)) flag_s[2] = 1;
+    }
+    X.phase[buf]++;
+    __syncthreads();
+    // h_{b->a}[q] = D_q (4x4, padded to 8 rows) * slots_b[q] (4 x 8 column tile): one DMMA per unit and point
+    for (int un = warp; un < nunit; un += DPG_NWARPS) {
+      int r = un, p = 0;
+      while (r >= P.test[P.pair_b[p]].ntiles) { r -= P.test[P.pair_b[p]].ntiles; p++; }
+      const int b = P.pair_b[p];
+      const int ld = P.test[b].ldA;
+      const double* dp = Dm + ((size_t)c * CH * P.npairs + p) * 16 + g * 4 + t;
+      const double* fp = fref + P.test[b].foff + t * ld + r * 8 + g;
+      double* hp = hb + P.hoff[p] + g * ld + r * 8 + 2 * t;
+#pragma unroll
+      for (int lq = 0; lq < CH; lq++) {
+        const double av = (g < 4) ? dp[lq * P.npairs * 16] : 0.0;
+        const double bv = fp[lq * P.featstride];
+        double2 hc = make_double2(0.0, 0.0);
+        dmma(hc, av, bv);
+        if (g < 4) *reinterpret_cast<double2*>(hp + lq * P.hstride) = hc;
+      }
+    }
+    __syncthreads();
+    // m16n8k16 over the owned blocks: one k16 step = 4 points x 4 slots
+#pragma unroll 1
+    for (int s4 = 0; s4 < CH; s4 += 4) {
+      const double* fa = fref + s4 * P.featstride;
+      const double* hq = hb + s4 * P.hstride;
+      uint32_t prevA = 0xffffffffu;
+      double av[8];
+#pragma unroll
+      for (int u = 0; u < GTM; u++) {
+        if (u < ntw) {
+          const uint32_t ao = pk[u] & 0xffffu, bo = pk[u] >> 16;
+          if (ao != prevA) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              av[2 * i] = fa[i * P.featstride + ao];
+              av[2 * i + 1] = fa[i * P.featstride + ao + 8];
+            }
+            prevA = ao;
+          }
+          double bv[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) bv[i] = hq[i * P.hstride + bo];
+          dmma16(acc[u], av, bv);
+        }
+      }
+    }
+    if (P.gflush > 0 && (c + 1) % P.gflush == 0 && c + 1 < nch) {
+      const bool first = (c + 1) == P.gflush;
+      const uint32_t fb = P.gflushbits[warp];
+#pragma unroll
+      for (int u = 0; u < GTM; u++) {
+        if (u < ntw && ((fb >> u) & 1u)) {
+          double2* sp = reinterpret_cast<double2*>(gsum + (u * 32 + lane) * 4);
+          double2 lo = make_double2(acc[u][0], acc[u][1]), hi = make_double2(acc[u][2], acc[u][3]);
+          if (!first) {
+            const double2 a = __ldcg(sp), b = __ldcg(sp + 1);
+            lo.x = a.x + lo.x; lo.y = a.y + lo.y; hi.x = b.x + hi.x; hi.y = b.y + hi.y;
+          }
+          __stcg(sp, lo);
+          __stcg(sp + 1, hi);
+          acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0;
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Phase 2: Gram matrix -> lower tiles in shared memory
+// ---------------------------------------------------------------------------
+template <int GTM, int CHG>
+__device__ __forceinline__ void phase_gram(const DpgPlanDev& P, const DpgLaunch& L, int cell, const Ctx& X) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int d = P.d, nv = P.nv;
+  DPG_SMEM_VIEWS(P);
+  double* geo = sm + P.g_geo;
+  double* Dm = sm + P.g_D;  // [q][pair][16]
+  double* hb = sm + P.g_h;
+  double* GT = sm + P.sm_gt;
+  const uint32_t chunk_bytes = (uint32_t)(P.chg * P.featstride * sizeof(double));
+  if (tid == 0) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_expect_tx(&mbar_s[0], chunk_bytes);
+    bulk_g2s(sm + P.g_fref0, P.frefG, chunk_bytes, &mbar_s[0]);
+  }
+  for (int q = tid; q < P.QGpad; q += NT)
+    point_geometry(d, nv, nodes_s, P.dNG + (size_t)q * nv * d, P.wG[q], nullptr, geo + q * GEO);
+  __syncthreads();
+  // beta_r,a[k] = sum over row-r entries on var a of coef * slot * T_a[slot_e][k]
+  double* beta = sm + P.g_beta;  // [q][row][4 * ntest]
+  const int F = 4 * P.ntest;
+  for (int task = tid; task < P.QGpad * P.niprows * P.ntest; task += NT) {
+    const int q = task / (P.niprows * P.ntest);
+    const int rem = task - q * P.niprows * P.ntest;
+    const int r = rem / P.ntest, a = rem - r * P.ntest;
+    const double* gq = geo + q * GEO;
+    double b0 = 0.0, b1 = 0.0, b2 = 0.0, b3 = 0.0;
+    for (int e = P.rowstart[r]; e < P.rowstart[r + 1]; e++) {
+      const DpgIPEnt& E = P.ipent[e];
+      if ((E.gslot >> 2) != a) continue;
+      double v = E.coef;
+      if (E.slot >= 0) v *= (q < P.QG) ? coef_s[E.slot * P.Ptot + q] : 0.0;
+      double tr[4];
+      trow_slot(P.test[a].space, d, E.gslot & 3, gq, tr);
+      b0 += v * tr[0]; b1 += v * tr[1]; b2 += v * tr[2]; b3 += v * tr[3];
+    }
+    double* dst = beta + (q * P.niprows + r) * F + 4 * a;
+    dst[0] = b0; dst[1] = b1; dst[2] = b2; dst[3] = b3;
+  }
+  __syncthreads();
+  // coupling D_ab[k][l] = wdet * sum_r beta_r,a[k] beta_r,b[l]
+  for (int task = tid; task < P.QGpad * P.npairs * 16; task += NT) {
+    const int q = task / (P.npairs * 16);
+    const int rem = task - q * P.npairs * 16;
+    const int p = rem >> 4, k = (rem >> 2) & 3, l = rem & 3;
+    const double* bq = beta + q * P.niprows * F;
+    const int ia = 4 * P.pair_a[p] + k, ib = 4 * P.pair_b[p] + l;
+    double sacc = 0.0;
+    for (int r = 0; r < P.niprows; r++) sacc += bq[r * F + ia] * bq[r * F + ib];
+    Dm[task] = sacc * geo[q * GEO + 19];
+  }
+  // owned 16x8 blocks: packed per-thread operand offsets (A | B << 16)
+  // balanced: warps 0 .. extra-1 take one block more, so the four SM sub-partitions
+  // (warps w, w+4, w+8, w+12) carry equal tensor work
+  const int gbase = P.ngb / DPG_NWARPS, gextra = P.ngb % DPG_NWARPS;
+  const int ntw = gbase + (warp < gextra ? 1 : 0);
+  const int tau0 = warp * gbase + min(warp, gextra);
+  const int4* tdesc = reinterpret_cast<const int4*>(sm + P.sm_tiles) + tau0;
+  uint32_t pk[GTM];
+  double acc[GTM][4];
+#pragma unroll
+  for (int u = 0; u < GTM; u++) {
+    acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0;
+    uint32_t v = 0;
+    if (u < ntw) {
+      const int4 T = tdesc[u];
+      v = (uint32_t)(T.z + t * (T.y & 0xffff) + g) | ((uint32_t)(T.w + t * (T.y >> 16) + g) << 16);
+    }
+    pk[u] = v;
+  }
+  // h work units per point: (pair, column tile of the pair's second var); warp w takes
+  // units w, w + 16, ... for every point of the chunk
+  int nunit = 0;
+  for (int p = 0; p < P.npairs; p++) nunit += P.test[P.pair_b[p]].ntiles;
+  __syncthreads();
+  double* gsum = L.scratch + (size_t)blockIdx.x * P.scratch_per_cta + P.gsum_off + (size_t)tau0 * 128;
+  if (CHG != 0) gram_chunks<GTM, CHG != 0 ? CHG : DPG_CHG>(P, X, Dm, hb, nunit, ntw, pk, acc, gsum);
+  else if (P.chg == DPG_CHG) gram_chunks<GTM, DPG_CHG>(P, X, Dm, hb, nunit, ntw, pk, acc, gsum);
+  else gram_chunks<GTM, DPG_CHG / 2>(P, X, Dm, hb, nunit, ntw, pk, acc, gsum);
+  if (P.gflush > 0 && P.gflush < P.QGpad / P.chg) {  // the last group joins the running sums
+    const uint32_t fb = P.gflushbits[warp];
+#pragma unroll
+    for (int u = 0; u < GTM; u++) {
+      if (u < ntw && ((fb >> u) & 1u)) {
+        const double2* sp = reinterpret_cast<const double2*>(gsum + (u * 32 + lane) * 4);
+        const double2 a = __ldcg(sp), b = __ldcg(sp + 1);
+        acc[u][0] = a.x + acc[u][0]; acc[u][1] = a.y + acc[u][1];
+        acc[u][2] = b.x + acc[u][2]; acc[u][3] = b.y + acc[u][3];
+      }
+    }
+  }
+  // accumulators -> tile-lower shared storage (overlaps the staging area); tiles of
+  // uncoupled var pairs are zero
+  for (int e = tid; e < P.ngz * 64; e += NT) GT[P.gzero[e >> 6] * 64 + (e & 63)] = 0.0;
+#pragma unroll
+  for (int u = 0; u < GTM; u++) {
+    if (u < ntw) {
+      const int4 T = tdesc[u];
+      const int I = T.x & 0xffff, J = (T.x >> 16) & 0xff;
+      if (J <= I)
+        *reinterpret_cast<double2*>(GT + (I * (I + 1) / 2 + J) * 64 + ak_cfrag(g, t)) = make_double2(acc[u][0], acc[u][1]);
+      if (!(T.x >> 24))
+        *reinterpret_cast<double2*>(GT + ((I + 1) * (I + 2) / 2 + J) * 64 + ak_cfrag(g, t)) =
+            make_double2(acc[u][2], acc[u][3]);
+    }
+  }
+  __syncthreads();
+  // padded rows decouple: unit diagonal
+  for (int r = tid; r < P.Np; r += NT)
+    if (P.dev2user_test[r] < 0) GT[((r >> 3) * ((r >> 3) + 1) / 2 + (r >> 3)) * 64 + ak(r & 7, r & 7)] = 1.0;
+  __syncthreads();
+  if (L.parts && L.G) {
+    double* Gc = L.G + (size_t)cell * P.N * P.N;
+    for (int e = tid; e < P.Np * P.Np; e += NT) {
+      int r = e / P.Np, c2 = e - r * P.Np;
+      int ur = P.dev2user_test[r], uc = P.dev2user_test[c2];
+      if (ur >= 0 && uc >= 0) Gc[(size_t)ur * P.N + uc] = sym_get(GT, r, c2);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Phase 3: equilibrated Cholesky of G and inverses of its diagonal tiles
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void phase_factor(const DpgPlanDev& P) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  DPG_SMEM_VIEWS(P);
+  double* GT = sm + P.sm_gt;
+  double* scale = sm + P.sm_scale;
+  double* LINV = sm + P.sm_linv;
+  for (int r = tid; r < P.Np; r += NT) {
+    int I = r >> 3;
+    double dg = GT[(I * (I + 1) / 2 + I) * 64 + ak(r & 7, r & 7)];
+    scale[r] = (dg > 0.0) ? rsqrt(dg) : 1.0;
+  }
+  __syncthreads();
+  for (int u = warp; u < P.ngt; u += DPG_NWARPS) {
+    int ij = tri_s[u];
+    int I = ij & 255, J = ij >> 8;
+    double2* p = reinterpret_cast<double2*>(GT + u * 64 + ak_cfrag(g, t));
+    double si = scale[I * 8 + g];
+    double2 v = *p;
+    v.x *= si * scale[J * 8 + 2 * t];
+    v.y *= si * scale[J * 8 + 2 * t + 1];
+    *p = v;
+  }
+  __syncthreads();
+  tile_cholesky(P.sm_gt, P.NBT, P.NBT, 2 * (P.sm_nodes + 24), 1, P.sm_nodes + 32, P.sm_linv);
+}
+
+// ---------------------------------------------------------------------------
+// Phase 4: W = L^-1 [B | F] per column tile in registers, W^T tiles to shared memory
+// ---------------------------------------------------------------------------
+
+// Column tile J of S [B | F] (S: the equilibration scales), C-fragments per row tile.
+template <int NBTM>
+__device__ __forceinline__ void solve_load(const DpgPlanDev& P, const DpgLaunch& L, int cell, int J, const double* scale,
+                                           double2 (&y)[NBTM]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  if (L.solve_only) {
+    const double* Bc = L.Bin + (size_t)cell * P.M * P.N;
+    const double* Fc = L.Fin + (size_t)cell * P.N;
+#pragma unroll
+    for (int I = 0; I < NBTM; I++) {
+      y[I] = make_double2(0.0, 0.0);
+      const int row = I * 8 + g;
+      if (I < P.NBT && row < P.N) {
+        double v[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int col = J * 8 + 2 * t + e;
+          v[e] = col < P.M ? Bc[(size_t)col * P.N + row] : (col == P.fcol ? Fc[row] : 0.0);
+        }
+        y[I] = make_double2(v[0], v[1]);
+      }
+    }
+  } else {
+    const double2* scr = reinterpret_cast<const double2*>(L.scratch + (size_t)blockIdx.x * P.scratch_per_cta) +
+                         (size_t)J * P.NBT * 32 + lane;
+#pragma unroll
+    for (int I = 0; I < NBTM; I++) y[I] = I < P.NBT ? scr[I * 32] : make_double2(0.0, 0.0);
+  }
+#pragma unroll
+  for (int I = 0; I < NBTM; I++)
+    if (I < P.NBT) {
+      const double si = scale[I * 8 + g];
+      y[I].x *= si;
+      y[I].y *= si;
+    }
+}
+
+// x_k = L_kk^-1 y_k, returned as a C-fragment and as negated B-fragments.
+__device__ __forceinline__ double2 solve_diag(const double* Li, const double2 yk, int lane, double& x0, double& x1) {
+  double y0, y1;
+  cfrag_to_bfrag(yk, lane, y0, y1);
+  double2 x = make_double2(0.0, 0.0);
+  dmma(x, Li[lane], y0);
+  dmma(x, Li[32 + lane], y1);
+  cfrag_to_bfrag(x, lane, x0, x1);
+  x0 = -x0;
+  x1 = -x1;
+  return x;
+}
+
+// y_i -= L_ik x_k for i > k: tiles (2j, 2j + 1) together, one m16n8k8 on the stacked tiles
+// [L_ik; L_i+1,k].  The pairs are the same in every step: an m16n8k8 accumulates into eight
+// consecutive registers, so pairs that shift with k would move every tile each step.
+// k is a compile-time value in the unrolled callers.
+template <int NBTM>
+__device__ __forceinline__ void solve_update(const double* __restrict__ GT, int NBT, int k, int lane, double2 (&y)[NBTM],
+                                             double x0, double x1) {
+  if (!(k & 1) && k + 1 < NBTM && k + 1 < NBT) {
+    const double* Lik = GT + ((k + 1) * (k + 2) / 2 + k) * 64;
+    dmma(y[k + 1], Lik[lane], x0);
+    dmma(y[k + 1], Lik[32 + lane], x1);
+  }
+#pragma unroll
+  for (int r = 0; r < NBTM; r += 2) {
+    if (r <= k) continue;
+    const double* Lik = GT + (r * (r + 1) / 2 + k) * 64;
+    const double* Ln = GT + ((r + 1) * (r + 2) / 2 + k) * 64;
+    if (r + 1 < NBT) {
+      dmma16x8(y[r], y[r + 1], Lik[lane], Ln[lane], Lik[32 + lane], Ln[32 + lane], x0, x1);
+    } else if (r < NBT) {
+      dmma(y[r], Lik[lane], x0);
+      dmma(y[r], Lik[32 + lane], x1);
+    }
+  }
+}
+
+// W^T tiles (trial J, test I) in AK layout, over L's tiles.
+template <int NBTM>
+__device__ __forceinline__ void solve_store(double* WT, int NBT, int J, const double2 (&y)[NBTM]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double* tile = WT + J * NBT * 64 + ((g >> 2) * 8 + 2 * t) * 4 + (g & 3);
+#pragma unroll
+  for (int I = 0; I < NBTM; I++) {
+    if (I < NBT) {
+      tile[I * 64] = y[I].x;
+      tile[I * 64 + 4] = y[I].y;
+    }
+  }
+}
+
+// W = Ls^-1 S [B | F] = L^-1 [B | F], one warp per column tile; then W^T over L's tiles.
+template <int NBTM>
+__device__ __forceinline__ void phase_trsm(const DpgPlanDev& P, const DpgLaunch& L, int cell) {
+  const int lane = threadIdx.x & 31, J = threadIdx.x >> 5;
+  const double* const GT = dpg_smem + P.sm_gt;
+  const double* const LINV = dpg_smem + P.sm_linv;
+  const int NBT = P.NBT;
+  if (J < P.MBT) {
+    double2 y[NBTM];
+    solve_load<NBTM>(P, L, cell, J, dpg_smem + P.sm_scale, y);
+#pragma unroll
+    for (int k = 0; k < NBTM; k++) {
+      if (k >= NBT) break;
+      double x0, x1;
+      y[k] = solve_diag(LINV + k * 64, y[k], lane, x0, x1);
+      solve_update<NBTM>(GT, NBT, k, lane, y, x0, x1);
+    }
+    asm volatile("bar.sync 0, %0;" ::"n"(NT) : "memory");
+    solve_store<NBTM>(dpg_smem + P.sm_w, NBT, J, y);
+  } else {
+    asm volatile("bar.sync 0, %0;" ::"n"(NT) : "memory");
+  }
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// Phase 5/6: K_ext = W^T W, outputs, condensation
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void phase_syrk_out(const DpgPlanDev& P, const DpgLaunch& L, int cell, const Ctx& X) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  DPG_SMEM_VIEWS(P);
+  const double* WT = sm + P.sm_w;
+  double* KT = sm + P.sm_k;
+  {
+    const int nk = P.MBT * (P.MBT + 1) / 2;
+    const int kbase = nk / DPG_NWARPS, kextra = nk % DPG_NWARPS;
+    const int k0 = warp * kbase + min(warp, kextra);
+    const int nkw = kbase + (warp < kextra ? 1 : 0);
+    double2 kacc[DPG_MAX_KT];
+    int kI[DPG_MAX_KT], kJ[DPG_MAX_KT];
+#pragma unroll
+    for (int u = 0; u < DPG_MAX_KT; u++) {
+      kacc[u] = make_double2(0.0, 0.0);
+      int ij = (u < nkw) ? tri_s[k0 + u] : 0;
+      kI[u] = ij & 255;
+      kJ[u] = ij >> 8;
+    }
+    for (int R = 0; R < P.NBT; R++) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        int lastI = -1;
+        double afr = 0.0;
+#pragma unroll
+        for (int u = 0; u < DPG_MAX_KT; u++) {
+          if (u < nkw) {
+            if (kI[u] != lastI) { afr = WT[(kI[u] * P.NBT + R) * 64 + h * 32 + lane]; lastI = kI[u]; }
+            double bfr = WT[(kJ[u] * P.NBT + R) * 64 + h * 32 + lane];
+            dmma(kacc[u], afr, bfr);
+          }
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < DPG_MAX_KT; u++)
+      if (u < nkw) *reinterpret_cast<double2*>(KT + (k0 + u) * 64 + ak_cfrag(g, t)) = kacc[u];
+    __syncthreads();
+  }
+  // K and l out (user numbering; fields first: dev = i for i < nf, nfp + (i - nf) otherwise);
+  // streaming stores, so the outputs do not evict the CTA's scratch slot from L2
+  if (L.K) {
+    double* Kc = L.K + (size_t)cell * P.M * P.M;
+    for (int i = warp; i < P.M; i += DPG_NWARPS) {
+      const int di = i < P.nf ? i : P.nfp + (i - P.nf);
+      for (int j = lane; j < P.M; j += 32) {
+        const int dj = j < P.nf ? j : P.nfp + (j - P.nf);
+        __stcs(&Kc[(size_t)i * P.M + j], sym_get(KT, di, dj));
+      }
+    }
+    double* lc = L.l + (size_t)cell * P.M;
+    for (int i = tid; i < P.M; i += NT) {
+      int di = i < P.nf ? i : P.nfp + (i - P.nf);
+      __stcs(&lc[i], sym_get(KT, P.fcol, di));
+    }
+  }
+  if (L.S && P.nt > 0) {
+    if (P.nfb > 0) {
+      __syncthreads();
+      for (int r = P.nf + tid; r < P.nfp; r += NT) {
+        int I = r >> 3;
+        KT[(I * (I + 1) / 2 + I) * 64 + ak(r & 7, r & 7)] = 1.0;
+      }
+      __syncthreads();
+      tile_cholesky(P.sm_k, P.MBT, P.nfb, 2 * (P.sm_nodes + 24) + 1, -1, P.sm_nodes + 32, P.sm_linv);
+    }
+    double* Sc = L.S + (size_t)cell * P.nt * P.nt;
+    for (int i = warp; i < P.nt; i += DPG_NWARPS)
+      for (int j = lane; j < P.nt; j += 32) __stcs(&Sc[(size_t)i * P.nt + j], sym_get(KT, P.nfp + i, P.nfp + j));
+    double* sc = L.s + (size_t)cell * P.nt;
+    for (int i = tid; i < P.nt; i += NT) __stcs(&sc[i], sym_get(KT, P.fcol, P.nfp + i));
+  }
+}
+
+// Element (r, c) of a C-fragment tiled N x (M+1) matrix in a scratch slot
+// (tile (I, J) at ((J * NBT + I) * 32 + lane) double2, lane = r * 4 + c / 2).
+__device__ __forceinline__ size_t cfrag_index(int NBT, int r, int c) {
+  return ((size_t)((c >> 3) * NBT + (r >> 3)) * 32 + (r & 7) * 4 + ((c & 7) >> 1)) * 2 + (c & 1);
+}
+
+__device__ __forceinline__ void mbar_inval(uint64_t* b) {
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(b)) : "memory");
+}
+
+// Per-CTA tables of one plan: triangular tile index, G block list, mbarriers.
+__device__ __forceinline__ void cta_setup(const DpgPlanDev& P) {
+  const int tid = threadIdx.x;
+  double* const sm = dpg_smem;
+  int* tri_s = reinterpret_cast<int*>(sm + P.sm_nodes + 32);
+  DpgGTile* tiles_s = reinterpret_cast<DpgGTile*>(sm + P.sm_tiles);
+  uint64_t* mbar_s = reinterpret_cast<uint64_t*>(sm + P.sm_nodes + 26);
+  const int ntri = DPG_MAX_NBT * (DPG_MAX_NBT + 1) / 2;
+  for (int u = tid; u < ntri; u += NT) {
+    int I = (int)((sqrt(8.0 * u + 1.0) - 1.0) * 0.5);
+    while ((I + 1) * (I + 2) / 2 <= u) I++;
+    while (I * (I + 1) / 2 > u) I--;
+    tri_s[u] = I | ((u - I * (I + 1) / 2) << 8);
+  }
+  for (int u = tid; u < P.ngb; u += NT) tiles_s[u] = P.gtiles[u];
+  if (tid == 0) {
+    for (int i = 0; i < 4; i++) mbar_init(&mbar_s[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+}
+
+typedef void (*KernelFn)(const DpgPlanDev, const DpgLaunch);
+
+}  // namespace

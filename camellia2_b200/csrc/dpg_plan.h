@@ -117,9 +117,10 @@ struct DpgTestVar {
 
 // One 16x8 block of G for mma.m16n8k16: rows of test tiles (I, I+1) of one
 // var, columns of test tile J.  The upper tile (I, I+1) of a diagonal block is
-// computed and dropped.
+// computed and dropped, and so is the second tile of a var whose last block has
+// one tile only.
 struct DpgGTile {
-  int16_t I, J;
+  int16_t I, J;    // J | 0x100: one row tile only
   int16_t lda, ldb;
   int aoff, boff;  // A operand / B operand offsets inside a point's feature / h block
 };
@@ -128,6 +129,7 @@ struct DpgPlanDev {
   int d, nv, ns;
   int N, M, nf, nt;
   int Np, NBT;              // padded test rows, test tiles
+  int nbt16;                // test tiles with every var padded to whole 16-row blocks
   int nfp, ntp, Mp, MBT;    // padded fields/traces, device trial columns incl F tile, trial tiles
   int nfb;                  // field tiles
   int fcol;                 // device column of F
@@ -188,7 +190,7 @@ struct DpgPlanDev {
   int sm_nodes;   // persistent: cell vertices, flags, mbarriers, triangular index table (192 doubles)
   int sm_coef;    // per cell: coefficients [nslots][Ptot]
   int g_fref0, g_fref1, g_h, g_geo, g_D, g_beta;   // Gram phase (g_beta overlaps g_h)
-  int sm_gt, sm_linv, sm_scale, sm_invd;           // factor
+  int sm_gt, sm_linv, sm_scale;                    // factor
   int b_rec0, b_rec1, b_u, b_geo, b_fac;      // B phase
   int sm_w, sm_k;                                  // solve / Gram of W
   int a_sa, a_ldS;                                 // adjoint: S_A [MBT*8][a_ldS]
