@@ -348,33 +348,15 @@ __device__ __forceinline__ void phase_adj_pull(const DpgPlanDev& P, const DpgLau
   __syncthreads();
 }
 
-template <int NBTM, int GTM, int BTW, int CH>
+template <int NBTM, int GTM, int BTW>
 __global__ void __launch_bounds__(NT, 1) dpg_adjoint_kernel(const __grid_constant__ DpgPlanDev P,
                                                                   const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x;
-  Ctx X;
   double* const sm = dpg_smem;
   double* nodes_s = sm + P.sm_nodes;
   int* flag_s = reinterpret_cast<int*>(sm + P.sm_nodes + 24);
-  uint64_t* mbar_s = reinterpret_cast<uint64_t*>(sm + P.sm_nodes + 26);
-  int* tri_s = reinterpret_cast<int*>(sm + P.sm_nodes + 32);
-  DpgGTile* tiles_s = reinterpret_cast<DpgGTile*>(sm + P.sm_tiles);
   double* coef_s = sm + P.sm_coef;
-  uint32_t phase[4] = {0, 0, 0, 0};
-  X.phase = phase;
-  const int ntri = DPG_MAX_NBT * (DPG_MAX_NBT + 1) / 2;
-  for (int u = tid; u < ntri; u += NT) {
-    int I = (int)((sqrt(8.0 * u + 1.0) - 1.0) * 0.5);
-    while ((I + 1) * (I + 2) / 2 <= u) I++;
-    while (I * (I + 1) / 2 > u) I--;
-    tri_s[u] = I | ((u - I * (I + 1) / 2) << 8);
-  }
-  for (int u = tid; u < P.ngb; u += NT) tiles_s[u] = P.gtiles[u];
-  if (tid == 0) {
-    for (int i = 0; i < 4; i++) mbar_init(&mbar_s[i], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
+  cta_setup(P);
   for (int cell = blockIdx.x; cell < L.C; cell += gridDim.x) {
     if (tid == 0) { flag_s[0] = 0; flag_s[1] = 0; flag_s[2] = 0; }
     if (tid < P.nv * P.d) nodes_s[tid] = L.nodes[(size_t)cell * P.nv * P.d + tid];
@@ -382,9 +364,9 @@ __global__ void __launch_bounds__(NT, 1) dpg_adjoint_kernel(const __grid_constan
     if (L.coeff)
       for (int i = tid; i < nco; i += NT) coef_s[i] = L.coeff[(size_t)cell * nco + i];
     __syncthreads();
-    phase_b<BTW>(P, L, cell, X);
+    phase_b<BTW>(P, L, cell);
     __syncthreads();
-    phase_gram<GTM, CH>(P, L, cell, X);
+    phase_gram<GTM>(P, L, cell);
     phase_factor(P);
     phase_adj_solve<NBTM>(P, L);
     phase_adj_p<NBTM>(P, L, cell);
@@ -403,14 +385,14 @@ __global__ void __launch_bounds__(NT, 1) dpg_adjoint_kernel(const __grid_constan
   }
 }
 
-#define DPG_ADJ_INSTANCES(X) X(12, 5, 4, 8) X(16, 6, 4, 8) X(20, 8, 4, 8) X(24, 12, 6, 8) X(24, 12, 6, 4)
+#define DPG_ADJ_INSTANCES(X) X(12, 5, 4) X(16, 6, 4) X(20, 8, 4) X(24, 12, 6)
 
 KernelFn pick_adjoint_kernel(const DpgPlanDev* plan) {
   const int per = (plan->ngb + DPG_NWARPS - 1) / DPG_NWARPS;
   int btw = 0;
   for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);
-#define DPG_PICK(NB, GT, BT, CH) \
-  if (plan->NBT <= NB && per <= GT && btw <= BT && plan->chg == CH) return dpg_adjoint_kernel<NB, GT, BT, CH>;
+#define DPG_PICK(NB, GT, BT) \
+  if (plan->NBT <= NB && per <= GT && btw <= BT) return dpg_adjoint_kernel<NB, GT, BT>;
   DPG_ADJ_INSTANCES(DPG_PICK)
 #undef DPG_PICK
   return nullptr;

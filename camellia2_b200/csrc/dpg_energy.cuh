@@ -23,17 +23,14 @@ __device__ __forceinline__ void energy_residual(const DpgPlanDev& P, const DpgLa
   }
 }
 
-template <int NBTM, int GTM, int BTW, int CH>
+template <int NBTM, int GTM, int BTW>
 __global__ void __launch_bounds__(NT, 1) dpg_energy_kernel(const __grid_constant__ DpgPlanDev P,
                                                                   const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  Ctx X;
   double* const sm = dpg_smem;
   double* nodes_s = sm + P.sm_nodes;
   int* flag_s = reinterpret_cast<int*>(sm + P.sm_nodes + 24);
   double* coef_s = sm + P.sm_coef;
-  uint32_t phase[4] = {0, 0, 0, 0};
-  X.phase = phase;
   cta_setup(P);
   for (int cell = blockIdx.x; cell < L.C; cell += gridDim.x) {
     if (tid == 0) { flag_s[0] = 0; flag_s[1] = 0; flag_s[2] = 0; }
@@ -42,11 +39,11 @@ __global__ void __launch_bounds__(NT, 1) dpg_energy_kernel(const __grid_constant
     if (L.coeff)
       for (int i = tid; i < nco; i += NT) coef_s[i] = L.coeff[(size_t)cell * nco + i];
     __syncthreads();
-    phase_b<BTW>(P, L, cell, X);
+    phase_b<BTW>(P, L, cell);
     __syncthreads();
     energy_residual(P, L, cell);
     __syncthreads();
-    phase_gram<GTM, CH>(P, L, cell, X);
+    phase_gram<GTM>(P, L, cell);
     phase_factor(P);
     phase_trsm<NBTM>(P, L, cell);
     // |L^-1 r|^2: row fcol of the W^T tiles of column tile fcol / 8
@@ -77,17 +74,14 @@ __global__ void __launch_bounds__(NT, 1) dpg_energy_kernel(const __grid_constant
   }
 }
 
-// Gram points per chunk (CH) fixed at compile time, as in the assembly kernel; the
-// picker takes the first instance whose sizes and chunk length fit the plan.
-#define DPG_ENERGY_INSTANCES(X) \
-  X(12, 5, 4, 8) X(16, 6, 4, 8) X(20, 8, 4, 8) X(22, 9, 3, 8) X(24, 12, 6, 8) X(24, 12, 6, 4)
+#define DPG_ENERGY_INSTANCES(X) X(12, 5, 4) X(16, 6, 4) X(20, 8, 4) X(22, 9, 3) X(24, 12, 6)
 
 static KernelFn pick_energy_kernel(const DpgPlanDev* plan) {
   const int per = (plan->ngb + DPG_NWARPS - 1) / DPG_NWARPS;
   int btw = 0;
   for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);
-#define DPG_PICK(NB, GT, BT, CH) \
-  if (plan->NBT <= NB && per <= GT && btw <= BT && plan->chg == CH) return dpg_energy_kernel<NB, GT, BT, CH>;
+#define DPG_PICK(NB, GT, BT) \
+  if (plan->NBT <= NB && per <= GT && btw <= BT) return dpg_energy_kernel<NB, GT, BT>;
   DPG_ENERGY_INSTANCES(DPG_PICK)
 #undef DPG_PICK
   return nullptr;
@@ -96,17 +90,14 @@ static KernelFn pick_energy_kernel(const DpgPlanDev* plan) {
 // DLS local matrices (TBF::localStiffnessMatrixAndRHS_DLS, BF.cpp:1169-1306: the
 // factored solve overwrites B and F in place): W = L^-1 B as (C, M, N) "trial x
 // test" and y = L^-1 F as (C, N), user numbering, L the unscaled Cholesky factor of G.
-template <int NBTM, int GTM, int BTW, int CH>
+template <int NBTM, int GTM, int BTW>
 __global__ void __launch_bounds__(NT, 1) dpg_dls_kernel(const __grid_constant__ DpgPlanDev P,
                                                                   const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x;
-  Ctx X;
   double* const sm = dpg_smem;
   double* nodes_s = sm + P.sm_nodes;
   int* flag_s = reinterpret_cast<int*>(sm + P.sm_nodes + 24);
   double* coef_s = sm + P.sm_coef;
-  uint32_t phase[4] = {0, 0, 0, 0};
-  X.phase = phase;
   cta_setup(P);
   for (int cell = blockIdx.x; cell < L.C; cell += gridDim.x) {
     if (tid == 0) { flag_s[0] = 0; flag_s[1] = 0; flag_s[2] = 0; }
@@ -115,9 +106,9 @@ __global__ void __launch_bounds__(NT, 1) dpg_dls_kernel(const __grid_constant__ 
     if (L.coeff)
       for (int i = tid; i < nco; i += NT) coef_s[i] = L.coeff[(size_t)cell * nco + i];
     __syncthreads();
-    phase_b<BTW>(P, L, cell, X);
+    phase_b<BTW>(P, L, cell);
     __syncthreads();
-    phase_gram<GTM, CH>(P, L, cell, X);
+    phase_gram<GTM>(P, L, cell);
     phase_factor(P);
     phase_trsm<NBTM>(P, L, cell);
     // W^T tile (J, I), element (r, c) = W[I*8 + c][J*8 + r]
@@ -150,8 +141,8 @@ static KernelFn pick_dls_kernel(const DpgPlanDev* plan) {
   const int per = (plan->ngb + DPG_NWARPS - 1) / DPG_NWARPS;
   int btw = 0;
   for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);
-#define DPG_PICK(NB, GT, BT, CH) \
-  if (plan->NBT <= NB && per <= GT && btw <= BT && plan->chg == CH) return dpg_dls_kernel<NB, GT, BT, CH>;
+#define DPG_PICK(NB, GT, BT) \
+  if (plan->NBT <= NB && per <= GT && btw <= BT) return dpg_dls_kernel<NB, GT, BT>;
   DPG_ENERGY_INSTANCES(DPG_PICK)
 #undef DPG_PICK
   return nullptr;

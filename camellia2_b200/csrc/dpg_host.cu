@@ -594,21 +594,24 @@ static int big_layout(HostPlan* P) {
   return DPG_OK;
 }
 
-// Shared-memory layout (doubles) of the single-CTA kernels for Gram chunks of chg points:
+// Shared-memory layout (doubles) of the single-CTA kernels for Gram chunks of chg points in a ring of
+// `stages`:
 // DPG_OK, -1 when it needs more shared memory than one CTA has, or a failure code.
-static int smem_layout(DpgPlanDev& g, int chg, bool adj_terms_ok) {
+static int smem_layout_stages(DpgPlanDev& g, int chg, int stages, bool adj_terms_ok) {
   g.chg = chg;
   if (g.nbt16 < (g.nfp + g.ntp + 8) / 8) return fail(DPG_ERR_UNSUPPORTED, "trial tiles outnumber test tiles: condensation workspace overlaps K");
   auto al = [](int x) { return (x + 15) & ~15; };  // 128-byte aligned regions
   int o = 0;
   // Gram phase
-  g.g_fref0 = o; o += al(g.chg * g.featstride);
-  g.g_fref1 = o; o += al(g.chg * g.featstride);
-  g.g_h = o;
-  g.g_beta = o;  // per-point IP rows in reference slots; dead before the first h chunk
-  o += al(std::max(g.chg * g.hstride, g.QGpad * g.niprows * 4 * g.ntest));
-  g.g_geo = o; o += al(g.QGpad * 24);
-  g.g_D = o; o += al(g.QGpad * g.npairs * 16);
+  // the ring of staged chunks; the per-point IP rows (beta) lie over the stages after the first
+  const int qg4 = (g.QG + 3) & ~3, nch = (g.QG + chg - 1) / chg;
+  g.gstages = nch >= stages ? stages : (nch >= 2 ? 2 : 1);  // a power of two
+  g.gstage = al(g.chg * g.featstride);
+  g.g_fref = o;
+  g.g_beta = o + g.gstage;
+  o += std::max(g.gstages * g.gstage, g.gstage + al(qg4 * g.niprows * 4 * g.ntest));
+  g.g_geo = o; o += al(qg4 * 24);
+  g.g_D = o; o += al(qg4 * (g.npairs * 16 + 2));
   int gphase = o;
   // factor
   o = 0;
@@ -653,10 +656,10 @@ static int smem_layout(DpgPlanDev& g, int chg, bool adj_terms_ok) {
   g.sm_coef = al(body);
   g.sm_tiles = g.sm_coef + al(std::max(1, g.nslots * g.Ptot));
   g.sm_nodes = g.sm_tiles + al((g.ngb * (int)sizeof(DpgGTile) + 7) / 8);
-  g.sm_total = g.sm_nodes + 192;
-  if ((size_t)g.sm_total * 8 > 232448) {
-    return -1;
-  }
+  g.sm_total = g.sm_nodes + DPG_SM_PERSIST;
+  // the larger rings leave room for the work queue's claim slot behind the plan's layout
+  const int reserve = chg * stages > DPG_CHG ? 4 : 0;
+  if ((size_t)(g.sm_total + reserve) * 8 > 232448) return -1;
   // Gram sums in two levels: after every 32 points the warps' DMMA accumulators of the
   // blocks that several graph-norm terms feed are added into FP64 running sums in the
   // CTA's scratch slot and restart from zero.  A single running sum over all points and
@@ -667,6 +670,17 @@ static int smem_layout(DpgPlanDev& g, int chg, bool adj_terms_ok) {
   g.gsum_off = (size_t)g.MBT * g.NBT * 64;
   g.scratch_per_cta = g.gsum_off + (size_t)g.ngb * 128;
   return DPG_OK;
+}
+
+// The largest ring that fits: 16-point chunks in two stages or 8-point ones in four or two (chg 8), 4-point
+// ones (chg 4).  A chunk costs its warps ~1 K cycles of barrier and parameter reads whatever its size.
+static int smem_layout(DpgPlanDev& g, int chg, bool adj_terms_ok) {
+  if (chg == DPG_CHG) {
+    const int rc = smem_layout_stages(g, 2 * DPG_CHG, 2, adj_terms_ok);
+    if (rc != -1) return rc;
+  }
+  const int rc = smem_layout_stages(g, chg, 4, adj_terms_ok);
+  return rc != -1 ? rc : smem_layout_stages(g, chg, 2, adj_terms_ok);
 }
 
 static int build(HostPlan* P, const dpg_bucket_desc* D) {
@@ -694,7 +708,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
   g.QG = rG.n; g.QB = rB.n; g.QS = rS.n;
   if (g.QG > DPG_MAX_QG) return fail(DPG_ERR_UNSUPPORTED, "Gram cubature rule too large");
   auto padc = [](int n, int c) { return (n + c - 1) / c * c; };
-  g.QGpad = padc(g.QG, DPG_CHG);
+  g.QGpad = padc(g.QG, 2 * DPG_CHG);  // whole Gram chunks
   g.QBpad = padc(g.QB, 8);
   g.QSpad = padc(g.QS, 8);
   g.Ptot = g.QG + g.QB + g.ns * g.QS;
@@ -805,7 +819,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     user_row += tv.card;
   }
   g.ntest = D->n_test;
-  g.featstride = foff;
+  g.featstride = foff + 4;  // Gram points: four points' slots in four different bank groups
   g.N = user_row;
   g.Np = dev_row;
   g.NBT = g.Np / 8;
@@ -980,20 +994,17 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
       return n >= 2;
     };
     std::vector<char> tile_multi;
-    int off = 0, np = 0;
+    int np = 0;
     for (int a = 0; a < g.ntest; a++)
       for (int b = 0; b <= a; b++) {
         if (!coupled[a * g.ntest + b]) continue;
         if (np >= DPG_MAX_PAIRS) return fail(DPG_ERR_UNSUPPORTED, "too many test var pairs");
         g.pair_a[np] = a;
         g.pair_b[np] = b;
-        g.hoff[np] = off;
         pidx[a * g.ntest + b] = np;
-        off += 4 * g.test[b].ldA;
         np++;
       }
     g.npairs = np;
-    g.hstride = off;
     std::vector<DpgGTile> tiles;
     std::vector<char> covered(g.NBT * (g.NBT + 1) / 2, 0);
     // 16 x 8 blocks of the single-CTA kernel (large plans have none)
@@ -1011,9 +1022,9 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
             if (!half) covered[(I + 1) * (I + 2) / 2 + J] = 1;
             DpgGTile t;
             t.I = (int16_t)I; t.J = (int16_t)(J | (half ? 0x100 : 0));
-            t.aoff = g.test[a].foff + rp * 8;
+            t.aoff = (g.test[a].foff + rp * 8) | (pidx[a * g.ntest + b] << 16);
             t.lda = (int16_t)g.test[a].ldA;
-            t.boff = g.hoff[pidx[a * g.ntest + b]] + jj * 8;
+            t.boff = g.test[b].foff + jj * 8;
             t.ldb = (int16_t)g.test[b].ldA;
             tiles.push_back(t);
             tile_multi.push_back(multi_term(a, b) ? 1 : 0);
@@ -1129,7 +1140,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
   }
   // shared-memory budget for the B phase: two record buffers, U, geometry of all
   // B points, per-point term rows R, coefficients
-  const int budget = 232448 / 8 - 192 - 2 * ((g.ngb * (int)sizeof(DpgGTile) + 7) / 8) - 64 - g.Np - g.Mp - 64;
+  const int budget = 232448 / 8 - DPG_SM_PERSIST - 2 * ((g.ngb * (int)sizeof(DpgGTile) + 7) / 8) - 64 - g.Np - g.Mp - 64;
   g.max_rec = 0; g.max_chunk = 0; g.max_ustride = 0; g.max_nterm = 0;
   std::vector<int4> btiles;
   for (int sg = 0; sg < g.nseg; sg++) {
@@ -1141,7 +1152,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     S.term0 = -1;
     S.nterm = 0;
     S.nblk = 0;
-    int off = 0, tv = g.featstride;
+    int off = 0, tv = foff;
     for (int i = 0; i < g.nbterm; i++) {
       if (terms[i].first != sg) continue;
       if (S.term0 < 0) S.term0 = i;
@@ -1227,8 +1238,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     std::vector<double> slots = fref_table(xs.data(), npad);
     std::vector<double> rec((size_t)npad * S.rec_len, 0.0);
     for (int q = 0; q < npad; q++) {
-      std::copy(slots.begin() + (size_t)q * g.featstride, slots.begin() + (size_t)(q + 1) * g.featstride,
-                rec.begin() + (size_t)q * S.rec_len);
+      std::copy_n(slots.begin() + (size_t)q * g.featstride, foff, rec.begin() + (size_t)q * S.rec_len);
       if (q >= S.npts) continue;
       for (int lt = 0; lt < S.nterm; lt++) {
         const DpgBTerm& t = g.bterm[S.term0 + lt];
@@ -1444,7 +1454,7 @@ int dpg_make_solve_plan(int N, int M, DpgPlanDev* out) {
   g.sm_nodes = g.sm_tiles;
   g.scratch_per_cta = 0;
   g.chg = DPG_CHG;  // no Gram phase; selects the standard kernel instances
-  g.sm_total = g.sm_nodes + 192;
+  g.sm_total = g.sm_nodes + DPG_SM_PERSIST;
   return DPG_OK;
 }
 
@@ -1693,7 +1703,7 @@ int dpg_plan_autotune(dpg_plan* p, int C, const double* nodes, const int8_t* par
     return fail(DPG_ERR_CUDA, "plan upload");
   rc = dpg_configure_kernels(&p->hp.dev);
   if (rc != DPG_OK) return rc;
-  *chosen = p->hp.dev.big ? p->hp.dev.big_zk : p->hp.dev.chg;
+  *chosen = p->hp.dev.big ? p->hp.dev.big_zk : std::min(p->hp.dev.chg, DPG_CHG);
   return DPG_OK;
 }
 

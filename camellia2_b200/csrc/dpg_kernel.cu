@@ -29,36 +29,16 @@
 
 namespace {
 
-template <int NBTM, int GTM, int BTW, int CHG>
+template <int NBTM, int GTM, int BTW>
 __global__ void __launch_bounds__(NT, 1) dpg_cell_kernel(const __grid_constant__ DpgPlanDev P,
                                                                   const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x;
-  Ctx X;
   double* const sm = dpg_smem;
   double* nodes_s = sm + P.sm_nodes;
   int* flag_s = reinterpret_cast<int*>(sm + P.sm_nodes + 24);
-  uint64_t* mbar_s = reinterpret_cast<uint64_t*>(sm + P.sm_nodes + 26);
   int* tri_s = reinterpret_cast<int*>(sm + P.sm_nodes + 32);
-  DpgGTile* tiles_s = reinterpret_cast<DpgGTile*>(sm + P.sm_tiles);
   double* coef_s = sm + P.sm_coef;
-  uint32_t phase[4] = {0, 0, 0, 0};
-  X.phase = phase;
-
-  // per-CTA set-up: triangular index table, tile table, mbarriers
-  const int ntri = DPG_MAX_NBT * (DPG_MAX_NBT + 1) / 2;
-  for (int u = tid; u < ntri; u += NT) {
-    int I = (int)((sqrt(8.0 * u + 1.0) - 1.0) * 0.5);
-    while ((I + 1) * (I + 2) / 2 <= u) I++;
-    while (I * (I + 1) / 2 > u) I--;
-    tri_s[u] = I | ((u - I * (I + 1) / 2) << 8);
-  }
-  if (!L.solve_only)
-    for (int u = tid; u < P.ngb; u += NT) tiles_s[u] = P.gtiles[u];
-  if (tid == 0) {
-    for (int i = 0; i < 4; i++) mbar_init(&mbar_s[i], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
+  cta_setup(P);
 
   for (int cell = blockIdx.x; cell < L.C; cell += gridDim.x) {
     if (tid == 0) { flag_s[0] = 0; flag_s[1] = 0; flag_s[2] = 0; }
@@ -85,9 +65,9 @@ __global__ void __launch_bounds__(NT, 1) dpg_cell_kernel(const __grid_constant__
       }
       __syncthreads();
     } else {
-      phase_b<BTW>(P, L, cell, X);
+      phase_b<BTW>(P, L, cell);
       __syncthreads();
-      phase_gram<GTM, CHG>(P, L, cell, X);
+      phase_gram<GTM>(P, L, cell);
       if (L.parts) {
         __syncthreads();
         continue;
@@ -95,7 +75,7 @@ __global__ void __launch_bounds__(NT, 1) dpg_cell_kernel(const __grid_constant__
     }
     phase_factor(P);
     phase_trsm<NBTM>(P, L, cell);
-    phase_syrk_out(P, L, cell, X);
+    phase_syrk_out(P, L, cell);
     __syncthreads();
     if (tid == 0 && L.info) {
       int f0 = flag_s[0], f1 = flag_s[1];
@@ -115,18 +95,16 @@ __global__ void __launch_bounds__(NT, 1) dpg_cell_kernel(const __grid_constant__
   }
 }
 
-// Instances: register arrays sized for the test-tile count of the bucket; the last
-// argument is the Gram chunk size (plans short of shared memory use half chunks).
+// Instances: register arrays sized for the test-tile count of the bucket.
 #define DPG_INSTANCES(X) \
-  X(8, 3, 4, 8) X(12, 5, 4, 8) X(16, 6, 4, 8) X(18, 8, 4, 8) X(20, 8, 4, 8) X(22, 9, 3, 8) X(24, 12, 4, 8) \
-  X(24, 12, 6, 8) X(24, 12, 6, 4)
+  X(8, 3, 4) X(12, 5, 4) X(16, 6, 4) X(18, 8, 4) X(20, 8, 4) X(22, 9, 3) X(24, 12, 4) X(24, 12, 6)
 
 static KernelFn pick_kernel(const DpgPlanDev* plan) {
   const int per = (plan->ngb + DPG_NWARPS - 1) / DPG_NWARPS;
   int btw = 0;
   for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);
-#define DPG_PICK(NB, GT, BT, CH) \
-  if (plan->NBT <= NB && per <= GT && btw <= BT && plan->chg == CH) return dpg_cell_kernel<NB, GT, BT, CH>;
+#define DPG_PICK(NB, GT, BT) \
+  if (plan->NBT <= NB && per <= GT && btw <= BT) return dpg_cell_kernel<NB, GT, BT>;
   DPG_INSTANCES(DPG_PICK)
 #undef DPG_PICK
   return nullptr;

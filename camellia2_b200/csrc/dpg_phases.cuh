@@ -41,6 +41,20 @@ __device__ __forceinline__ void dmma16(double* c, const double* a, const double*
         "d"(b[1]), "d"(b[2]), "d"(b[3]));
 }
 
+// D(16x8) += A(16x4) B(4x8): a0 = A[g][t], a1 = A[g+8][t]; b = B[t][g].
+__device__ __forceinline__ void dmma16x4(double* c, double a0, double a1, double b) {
+  asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a0), "d"(a1), "d"(b));
+}
+
+// D(16x8) += A(16x8) B(8x8), operands as dmma16x8's.
+__device__ __forceinline__ void dmma16k8(double* c, double a0, double a1, double a2, double a3, double b0, double b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
+
 // D(16x8) += A(16x8) * B(8x8): a0 = A[g][t], a1 = A[g+8][t], a2 = A[g][t+4], a3 = A[g+8][t+4];
 // b0 = B[t][g], b1 = B[t+4][g]; c_lo holds rows g, c_hi rows g+8 (columns 2t, 2t+1 each).
 __device__ __forceinline__ void dmma16x8(double2& c_lo, double2& c_hi, double a0, double a1, double a2, double a3,
@@ -58,6 +72,10 @@ __device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
 
 // Global -> shared bulk copy completing on an mbarrier (16-byte aligned, bytes % 16 == 0).
@@ -244,15 +262,11 @@ __device__ __forceinline__ double sym_get(const double* base, int r, int c) {
   return base[(I * (I + 1) / 2 + J) * 64 + ak(r & 7, c & 7)];
 }
 
-struct Ctx {
-  uint32_t* phase;     // mbarrier use counters [4]
-};
-
 // Shared-memory views of the persistent region (derived from dpg_smem).
 #define DPG_SMEM_VIEWS(P)                                                              \
   double* const sm = dpg_smem;                                                         \
   int* const flag_s = reinterpret_cast<int*>(sm + (P).sm_nodes + 24);                  \
-  uint64_t* const mbar_s = reinterpret_cast<uint64_t*>(sm + (P).sm_nodes + 26);        \
+  uint64_t* const mbar_s = reinterpret_cast<uint64_t*>(sm + (P).sm_nodes + DPG_SM_BARS); \
   const int* const tri_s = reinterpret_cast<const int*>(sm + (P).sm_nodes + 32);       \
   const double* const nodes_s = sm + (P).sm_nodes;                                     \
   const double* const coef_s = sm + (P).sm_coef;                                       \
@@ -426,7 +440,7 @@ __device__ __noinline__ void tile_cholesky(int T_off, int nb, int nsteps, int fl
 // Phase 1: B and F -> per-CTA scratch (or the B/F outputs in parts mode)
 // ---------------------------------------------------------------------------
 template <int BTW>
-__device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, int cell, const Ctx& X) {
+__device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, int cell) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int d = P.d, nv = P.nv;
@@ -442,8 +456,8 @@ __device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, in
     const DpgSeg& S = P.seg[first_seg];
     const uint32_t bytes = (uint32_t)(((min(S.chunk, S.npts) + 3) & ~3) * S.rec_len * sizeof(double));
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(&mbar_s[2], bytes);
-    bulk_g2s(sm + P.b_rec0, S.rec, bytes, &mbar_s[2]);
+    mbar_expect_tx(&mbar_s[DPG_BAR_B], bytes);
+    bulk_g2s(sm + P.b_rec0, S.rec, bytes, &mbar_s[DPG_BAR_B]);
   }
   // [B | F] tiles accumulate in this CTA's scratch slot, C-fragment layout per tile
   for (int i = tid; i < P.MBT * P.NBT * 32; i += NT) scr[i] = make_double2(0.0, 0.0);
@@ -527,13 +541,14 @@ __device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, in
           const uint32_t bytes =
               (uint32_t)(((min(S2.chunk, S2.npts - nc * S2.chunk) + 3) & ~3) * S2.rec_len * sizeof(double));
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          mbar_expect_tx(&mbar_s[2 + (buf ^ 1)], bytes);
+          mbar_expect_tx(&mbar_s[DPG_BAR_B + (buf ^ 1)], bytes);
           bulk_g2s(sm + (buf ? P.b_rec0 : P.b_rec1), S2.rec + (size_t)nc * S2.chunk * S2.rec_len, bytes,
-                   &mbar_s[2 + (buf ^ 1)]);
+                   &mbar_s[DPG_BAR_B + (buf ^ 1)]);
         }
-        if (!mbar_wait(&mbar_s[2 + buf], X.phase[2 + buf] & 1)) flag_s[2] = 1;
+        const int par = flag_s[3];  // bit i: parity of the next wait on buffer i
+        if (!mbar_wait(&mbar_s[DPG_BAR_B + buf], (par >> buf) & 1)) flag_s[2] = 1;
+        flag_s[3] = par ^ (1 << buf);
       }
-      X.phase[2 + buf]++;
       const int q0 = c * S.chunk;
       const int nq = min(S.chunk, S.npts - q0);
       __syncthreads();
@@ -633,87 +648,162 @@ __device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, in
   }
 }
 
-// The Gram chunk loop for CH points per chunk (compile-time, so the h and DMMA loops
-// unroll completely).
-// Every P.gflush chunks (except after the last) each thread adds the accumulators of its
-// flushed blocks (P.gflushbits) into its own running sums in gsum ([block][lane][4]; plain
-// L2 loads and stores, one writer per element, so the order of additions is fixed) and
-// restarts them from zero.
-template <int GTM, int CH>
-__device__ __forceinline__ void gram_chunks(const DpgPlanDev& P, const Ctx& X, const double* Dm, double* hb, int nunit,
-                                            int ntw, const uint32_t (&pk)[GTM], double (&acc)[GTM][4],
-                                            double* __restrict__ gsum) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  DPG_SMEM_VIEWS(P);
-  const int nch = P.QGpad / CH;
-  const uint32_t chunk_bytes = (uint32_t)(CH * P.featstride * sizeof(double));
-  for (int c = 0; c < nch; c++) {
-    const int buf = c & 1;
-    const double* fref = sm + (buf ? P.g_fref1 : P.g_fref0);
-    if (tid == 0) {
-      if (c + 1 < nch) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(&mbar_s[buf ^ 1], chunk_bytes);
-        bulk_g2s(sm + (buf ? P.g_fref0 : P.g_fref1), P.frefG + (size_t)(c + 1) * CH * P.featstride,
-                 chunk_bytes, &mbar_s[buf ^ 1]);
+// One k-step of the Gram products over a warp's blocks.  The row var's slots f_a go through the
+// point's coupling D first (A' = f_a D, formed when the row pair or the column var changes), so the
+// column var's slots are the B operand as staged.  blk[u]: offset of block u's column slots | slot
+// stride << 16 | 1 << 31 where A' changes; tdesc: the block table (lane-independent).
+// 3D, two points: A' is an m16n8k8 of the two points' slots with the block diagonal of
+// their couplings; its columns 2t, 2t + 1 = (point t >> 1, slots 2 (t & 1), + 1) leave the lane that holds
+// them as A operand of the products, which take k = t and k = t + 4 from those columns.
+template <int GTM>
+__device__ __forceinline__ void gram_step3d(const double* __restrict__ f, const double* __restrict__ Dm, int fs, int dstride,
+                                            const int4* tdesc, const uint32_t (&blk)[GTM], int ntw,
+                                            double (&acc)[GTM][4]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double av[4];
+#pragma unroll
+  for (int u = 0; u < GTM; u++) {
+    if (u < ntw) {
+      const uint32_t v = blk[u];
+      if (v >> 31) {
+        const int4 T = tdesc[u];
+        const double* fa = f + (T.z & 0xffff) + t * (T.y & 0xffff) + g;
+        const double d = Dm[(g >> 2) * dstride + (T.z >> 16) * 16 + t * 4 + (g & 3)];
+        av[0] = av[1] = av[2] = av[3] = 0.0;
+        dmma16k8(av, fa[0], fa[8], fa[fs], fa[fs + 8], g < 4 ? d : 0.0, g < 4 ? 0.0 : d);
       }
-      if (!mbar_wait(&mbar_s[buf], X.phase[buf] & 1)) flag_s[2] = 1;
+      const int ldb = (v >> 16) & 0x7fff;
+      const double* b = f + (t >> 1) * fs + 2 * (t & 1) * ldb + g + (v & 0xffffu);
+      dmma16k8(acc[u], av[0], av[2], av[1], av[3], b[0], b[ldb]);
     }
-    X.phase[buf]++;
-    __syncthreads();
-    // h_{b->a}[q] = D_q (4x4, padded to 8 rows) * slots_b[q] (4 x 8 column tile): one DMMA per unit and point
-    for (int un = warp; un < nunit; un += DPG_NWARPS) {
-      int r = un, p = 0;
-      while (r >= P.test[P.pair_b[p]].ntiles) { r -= P.test[P.pair_b[p]].ntiles; p++; }
-      const int b = P.pair_b[p];
-      const int ld = P.test[b].ldA;
-      const double* dp = Dm + ((size_t)c * CH * P.npairs + p) * 16 + g * 4 + t;
-      const double* fp = fref + P.test[b].foff + t * ld + r * 8 + g;
-      double* hp = hb + P.hoff[p] + g * ld + r * 8 + 2 * t;
+  }
+}
+
+// 2D, four points with three slots each (lane t: point t), three m16n8k4: a fourth slot would be
+// zeros, a quarter of the tensor work.  A' by FMAs (lane t has its point's slots and coupling).
+template <int GTM>
+__device__ __forceinline__ void gram_step2d(const double* __restrict__ f, const double* __restrict__ Dm, int fs, int dstride,
+                                            const int4* tdesc, const uint32_t (&blk)[GTM], int ntw,
+                                            double (&acc)[GTM][4]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double av[6];
 #pragma unroll
-      for (int lq = 0; lq < CH; lq++) {
-        const double av = (g < 4) ? dp[lq * P.npairs * 16] : 0.0;
-        const double bv = fp[lq * P.featstride];
-        double2 hc = make_double2(0.0, 0.0);
-        dmma(hc, av, bv);
-        if (g < 4) *reinterpret_cast<double2*>(hp + lq * P.hstride) = hc;
-      }
-    }
-    __syncthreads();
-    // m16n8k16 over the owned blocks: one k16 step = 4 points x 4 slots
-#pragma unroll 1
-    for (int s4 = 0; s4 < CH; s4 += 4) {
-      const double* fa = fref + s4 * P.featstride;
-      const double* hq = hb + s4 * P.hstride;
-      uint32_t prevA = 0xffffffffu;
-      double av[8];
+  for (int u = 0; u < GTM; u++) {
+    if (u < ntw) {
+      const uint32_t v = blk[u];
+      if (v >> 31) {
+        const int4 T = tdesc[u];
+        const int ld = T.y & 0xffff;
+        const double* fa = f + (T.z & 0xffff) + t * fs + g;
+        const double* D = Dm + (T.z >> 16) * 16 + t * dstride;
 #pragma unroll
-      for (int u = 0; u < GTM; u++) {
-        if (u < ntw) {
-          const uint32_t ao = pk[u] & 0xffffu, bo = pk[u] >> 16;
-          if (ao != prevA) {
+        for (int k = 0; k < 3; k++) {
+          const double lo = fa[k * ld], hi = fa[k * ld + 8];
+          const double2 d01 = *reinterpret_cast<const double2*>(D + k * 4);
+          const double dk[3] = {d01.x, d01.y, D[k * 4 + 2]};
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-              av[2 * i] = fa[i * P.featstride + ao];
-              av[2 * i + 1] = fa[i * P.featstride + ao + 8];
-            }
-            prevA = ao;
+          for (int l = 0; l < 3; l++) {
+            av[2 * l] = k == 0 ? lo * dk[l] : fma(lo, dk[l], av[2 * l]);
+            av[2 * l + 1] = k == 0 ? hi * dk[l] : fma(hi, dk[l], av[2 * l + 1]);
           }
-          double bv[4];
-#pragma unroll
-          for (int i = 0; i < 4; i++) bv[i] = hq[i * P.hstride + bo];
-          dmma16(acc[u], av, bv);
         }
       }
+      const int ldb = (v >> 16) & 0x7fff;
+      const double* b = f + t * fs + g + (v & 0xffffu);
+      const double b0 = b[0], b1 = b[ldb], b2 = b[2 * ldb];
+      dmma16x4(acc[u], av[0], av[1], b0);
+      dmma16x4(acc[u], av[2], av[3], b1);
+      dmma16x4(acc[u], av[4], av[5], b2);
     }
-    if (P.gflush > 0 && (c + 1) % P.gflush == 0 && c + 1 < nch) {
-      const bool first = (c + 1) == P.gflush;
-      const uint32_t fb = P.gflushbits[warp];
+  }
+}
+
+// What the chunk loop needs of the plan, in shared memory (cta_setup): read again once a chunk
+// (volatile), because kept in registers it would push accumulators to local memory.  GP_PAR: bit i
+// is the parity of the next first use of ring stage i.
+enum { GP_CHG, GP_QG, GP_RING, GP_STAGE, GP_STAGES, GP_FLUSH, GP_D, GP_NGB, GP_TILES, GP_FS, GP_DS, GP_GT, GP_PAR, GP_N };
+
+// The Gram chunk loop.  (The earlier form wrote D x slots of every column tile to shared memory before
+// the products: two block barriers per chunk and 30 K of the phase's 165 K cycles on the 48^3
+// hex workload.)  The chunks travel through a ring of stages: warps arrive on a stage's empty
+// mbarrier and warp 0 refills it while the next chunk is worked on, so no block barrier is left in
+// the loop and the warps drift apart by up to a ring.  Every GP_FLUSH chunks (except after the last)
+// each thread adds the accumulators of its flushed blocks (P.gflushbits) into its own running sums
+// in the scratch slot ([block][lane][4]; plain L2 loads and stores, one writer per element, so the
+// order of additions is fixed) and restarts them from zero.
+template <int GTM, int DIM>
+__device__ __forceinline__ void gram_body(const DpgPlanDev& P, const DpgLaunch& L, int sm_nodes) {
+  const volatile int* const gp = reinterpret_cast<const volatile int*>(dpg_smem + sm_nodes + DPG_SM_GRAM);
+  double acc[GTM][4];
+#pragma unroll
+  for (int u = 0; u < GTM; u++) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0;
+  // owned 16x8 blocks, balanced: warps 0 .. extra-1 take one block more, so the four SM
+  // sub-partitions (warps w, w+4, w+8, w+12) carry equal tensor work
+  int ntw, tau0;
+  {
+    const int ngb = gp[GP_NGB], warp = threadIdx.x >> 5;
+    ntw = ngb / DPG_NWARPS + (warp < ngb % DPG_NWARPS ? 1 : 0);
+    tau0 = warp * (ngb / DPG_NWARPS) + min(warp, ngb % DPG_NWARPS);
+  }
+  const int4* const tdesc = reinterpret_cast<const int4*>(dpg_smem + gp[GP_TILES]) + tau0;
+  const int fs = gp[GP_FS], dstride = gp[GP_DS];
+  uint32_t blk[GTM];
+  {
+    int lastA = -1;
+#pragma unroll
+    for (int u = 0; u < GTM; u++) {
+      blk[u] = 0;
+      if (u < ntw) {
+        const int4 T = tdesc[u];
+        blk[u] = (uint32_t)T.w | ((uint32_t)(T.y >> 16) << 16) | (T.z != lastA ? 0x80000000u : 0u);
+        lastA = T.z;
+      }
+    }
+  }
+#pragma unroll 1
+  for (int c = 0; c * gp[GP_CHG] < gp[GP_QG]; c++) {
+    const double* f;
+    const double* Dm;
+    int nq;  // points of the chunk, in whole k-steps of four
+    {
+      const int chg = gp[GP_CHG], stages = gp[GP_STAGES], use = c >> (stages >> 1), st = c & (stages - 1);  // 1, 2 or 4 stages
+      uint64_t* const full = reinterpret_cast<uint64_t*>(dpg_smem + sm_nodes + DPG_SM_BARS);
+      if (c > 0 && threadIdx.x == 0 && (c - 1 + stages) * chg < gp[GP_QG]) {
+        // refill the stage of chunk c - 1 with chunk c - 1 + stages
+        const int pu = (c - 1) >> (stages >> 1), ps = (c - 1) & (stages - 1);
+        const uint32_t par = (uint32_t)gp[GP_PAR] >> (DPG_GSTAGES + ps);
+        if (!mbar_wait(&full[DPG_BAR_EMPTY + ps], (par ^ pu) & 1u)) reinterpret_cast<int*>(dpg_smem + sm_nodes + 24)[2] = 1;
+        const uint32_t bytes = (uint32_t)(chg * fs * sizeof(double));
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_expect_tx(&full[ps], bytes);
+        bulk_g2s(dpg_smem + gp[GP_RING] + ps * gp[GP_STAGE], P.frefG + (size_t)(c - 1 + stages) * chg * fs, bytes, &full[ps]);
+      }
+      __syncwarp();
+      if (!mbar_wait(&full[st], (((uint32_t)gp[GP_PAR] >> st) ^ use) & 1u)) reinterpret_cast<int*>(dpg_smem + sm_nodes + 24)[2] = 1;
+      f = dpg_smem + gp[GP_RING] + st * gp[GP_STAGE];
+      Dm = dpg_smem + gp[GP_D] + c * chg * dstride;
+      nq = (min(chg, gp[GP_QG] - c * chg) + 3) & ~3;
+    }
+    constexpr int STEP = DIM == 3 ? 2 : 4;
+#pragma unroll 1
+    for (; nq > 0; nq -= STEP, f += STEP * fs, Dm += STEP * dstride) {
+      if (DIM == 3) gram_step3d<GTM>(f, Dm, fs, dstride, tdesc, blk, ntw, acc);
+      else gram_step2d<GTM>(f, Dm, fs, dstride, tdesc, blk, ntw, acc);
+    }
+    const int chg = gp[GP_CHG], stages = gp[GP_STAGES], gflush = gp[GP_FLUSH];
+    if ((c + stages) * chg < gp[GP_QG]) {  // the stage will be refilled
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0)
+        mbar_arrive(reinterpret_cast<uint64_t*>(dpg_smem + sm_nodes + DPG_SM_BARS) + DPG_BAR_EMPTY + (c & (stages - 1)));
+    }
+    if ((c + 1) % gflush == 0 && (c + 1) * chg < gp[GP_QG]) {
+      const bool first = (c + 1) == gflush;
+      const uint32_t fb = P.gflushbits[threadIdx.x >> 5];
+      double* const gsum = L.scratch + (size_t)blockIdx.x * P.scratch_per_cta + P.gsum_off + tau0 * 128 + (threadIdx.x & 31) * 4;
 #pragma unroll
       for (int u = 0; u < GTM; u++) {
         if (u < ntw && ((fb >> u) & 1u)) {
-          double2* sp = reinterpret_cast<double2*>(gsum + (u * 32 + lane) * 4);
+          double2* sp = reinterpret_cast<double2*>(gsum + u * 128);
           double2 lo = make_double2(acc[u][0], acc[u][1]), hi = make_double2(acc[u][2], acc[u][3]);
           if (!first) {
             const double2 a = __ldcg(sp), b = __ldcg(sp + 1);
@@ -725,36 +815,70 @@ __device__ __forceinline__ void gram_chunks(const DpgPlanDev& P, const Ctx& X, c
         }
       }
     }
-    __syncthreads();
   }
+  __syncthreads();  // every warp is done with the ring, which the tiles overlap
+  if (threadIdx.x == 0) {
+    const int chg = gp[GP_CHG], stages = gp[GP_STAGES], nch = (gp[GP_QG] + chg - 1) / chg;
+    int par = gp[GP_PAR];
+    for (int i = 0; i < stages; i++) {
+      const int uses = (nch - i + stages - 1) / stages;  // a stage is emptied once less than it is filled
+      par ^= ((uses & 1) << i) | (((uses - 1) & 1) << (DPG_GSTAGES + i));
+    }
+    reinterpret_cast<int*>(dpg_smem + sm_nodes + DPG_SM_GRAM)[GP_PAR] = par;
+  }
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double* const GT = dpg_smem + gp[GP_GT];
+  const bool join = gp[GP_FLUSH] * gp[GP_CHG] < gp[GP_QG];  // the last group joins the running sums
+  const uint32_t fb = P.gflushbits[threadIdx.x >> 5];
+  const double* const gsum = L.scratch + (size_t)blockIdx.x * P.scratch_per_cta + P.gsum_off + tau0 * 128 + lane * 4;
+#pragma unroll
+  for (int u = 0; u < GTM; u++) {
+    if (u < ntw) {
+      double2 lo = make_double2(acc[u][0], acc[u][1]), hi = make_double2(acc[u][2], acc[u][3]);
+      if (join && ((fb >> u) & 1u)) {
+        const double2* sp = reinterpret_cast<const double2*>(gsum + u * 128);
+        const double2 a = __ldcg(sp), b = __ldcg(sp + 1);
+        lo.x = a.x + lo.x; lo.y = a.y + lo.y; hi.x = b.x + hi.x; hi.y = b.y + hi.y;
+      }
+      const int T = tdesc[u].x;
+      const int I = T & 0xffff, J = (T >> 16) & 0xff;
+      if (J <= I) *reinterpret_cast<double2*>(GT + (I * (I + 1) / 2 + J) * 64 + ak_cfrag(g, t)) = lo;
+      if (!(T >> 24)) *reinterpret_cast<double2*>(GT + ((I + 1) * (I + 2) / 2 + J) * 64 + ak_cfrag(g, t)) = hi;
+    }
+  }
+}
+
+// A function of its own in 3D, where inlining beside the other phases spills accumulators.
+template <int GTM>
+__device__ __noinline__ void gram_chunks3d(const DpgPlanDev& P, const DpgLaunch& L, int sm_nodes) {
+  gram_body<GTM, 3>(P, L, sm_nodes);
 }
 
 // ---------------------------------------------------------------------------
 // Phase 2: Gram matrix -> lower tiles in shared memory
 // ---------------------------------------------------------------------------
-template <int GTM, int CHG>
-__device__ __forceinline__ void phase_gram(const DpgPlanDev& P, const DpgLaunch& L, int cell, const Ctx& X) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
+template <int GTM>
+__device__ __forceinline__ void phase_gram(const DpgPlanDev& P, const DpgLaunch& L, int cell) {
+  const int tid = threadIdx.x;
   const int d = P.d, nv = P.nv;
   DPG_SMEM_VIEWS(P);
   double* geo = sm + P.g_geo;
-  double* Dm = sm + P.g_D;  // [q][pair][16]
-  double* hb = sm + P.g_h;
+  double* Dm = sm + P.g_D;  // [q][pair][16], points 2 doubles apart in bank position
   double* GT = sm + P.sm_gt;
   const uint32_t chunk_bytes = (uint32_t)(P.chg * P.featstride * sizeof(double));
   if (tid == 0) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_expect_tx(&mbar_s[0], chunk_bytes);
-    bulk_g2s(sm + P.g_fref0, P.frefG, chunk_bytes, &mbar_s[0]);
+    bulk_g2s(sm + P.g_fref, P.frefG, chunk_bytes, &mbar_s[0]);
   }
-  for (int q = tid; q < P.QGpad; q += NT)
+  const int qg4 = (P.QG + 3) & ~3;
+  for (int q = tid; q < qg4; q += NT)
     point_geometry(d, nv, nodes_s, P.dNG + (size_t)q * nv * d, P.wG[q], nullptr, geo + q * GEO);
   __syncthreads();
   // beta_r,a[k] = sum over row-r entries on var a of coef * slot * T_a[slot_e][k]
   double* beta = sm + P.g_beta;  // [q][row][4 * ntest]
   const int F = 4 * P.ntest;
-  for (int task = tid; task < P.QGpad * P.niprows * P.ntest; task += NT) {
+  for (int task = tid; task < qg4 * P.niprows * P.ntest; task += NT) {
     const int q = task / (P.niprows * P.ntest);
     const int rem = task - q * P.niprows * P.ntest;
     const int r = rem / P.ntest, a = rem - r * P.ntest;
@@ -774,7 +898,7 @@ __device__ __forceinline__ void phase_gram(const DpgPlanDev& P, const DpgLaunch&
   }
   __syncthreads();
   // coupling D_ab[k][l] = wdet * sum_r beta_r,a[k] beta_r,b[l]
-  for (int task = tid; task < P.QGpad * P.npairs * 16; task += NT) {
+  for (int task = tid; task < qg4 * P.npairs * 16; task += NT) {
     const int q = task / (P.npairs * 16);
     const int rem = task - q * P.npairs * 16;
     const int p = rem >> 4, k = (rem >> 2) & 3, l = rem & 3;
@@ -782,63 +906,20 @@ __device__ __forceinline__ void phase_gram(const DpgPlanDev& P, const DpgLaunch&
     const int ia = 4 * P.pair_a[p] + k, ib = 4 * P.pair_b[p] + l;
     double sacc = 0.0;
     for (int r = 0; r < P.niprows; r++) sacc += bq[r * F + ia] * bq[r * F + ib];
-    Dm[task] = sacc * geo[q * GEO + 19];
+    Dm[q * (P.npairs * 16 + 2) + rem] = sacc * geo[q * GEO + 19];
   }
-  // owned 16x8 blocks: packed per-thread operand offsets (A | B << 16)
-  // balanced: warps 0 .. extra-1 take one block more, so the four SM sub-partitions
-  // (warps w, w+4, w+8, w+12) carry equal tensor work
-  const int gbase = P.ngb / DPG_NWARPS, gextra = P.ngb % DPG_NWARPS;
-  const int ntw = gbase + (warp < gextra ? 1 : 0);
-  const int tau0 = warp * gbase + min(warp, gextra);
-  const int4* tdesc = reinterpret_cast<const int4*>(sm + P.sm_tiles) + tau0;
-  uint32_t pk[GTM];
-  double acc[GTM][4];
-#pragma unroll
-  for (int u = 0; u < GTM; u++) {
-    acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0;
-    uint32_t v = 0;
-    if (u < ntw) {
-      const int4 T = tdesc[u];
-      v = (uint32_t)(T.z + t * (T.y & 0xffff) + g) | ((uint32_t)(T.w + t * (T.y >> 16) + g) << 16);
-    }
-    pk[u] = v;
-  }
-  // h work units per point: (pair, column tile of the pair's second var); warp w takes
-  // units w, w + 16, ... for every point of the chunk
-  int nunit = 0;
-  for (int p = 0; p < P.npairs; p++) nunit += P.test[P.pair_b[p]].ntiles;
   __syncthreads();
-  double* gsum = L.scratch + (size_t)blockIdx.x * P.scratch_per_cta + P.gsum_off + (size_t)tau0 * 128;
-  if (CHG != 0) gram_chunks<GTM, CHG != 0 ? CHG : DPG_CHG>(P, X, Dm, hb, nunit, ntw, pk, acc, gsum);
-  else if (P.chg == DPG_CHG) gram_chunks<GTM, DPG_CHG>(P, X, Dm, hb, nunit, ntw, pk, acc, gsum);
-  else gram_chunks<GTM, DPG_CHG / 2>(P, X, Dm, hb, nunit, ntw, pk, acc, gsum);
-  if (P.gflush > 0 && P.gflush < P.QGpad / P.chg) {  // the last group joins the running sums
-    const uint32_t fb = P.gflushbits[warp];
-#pragma unroll
-    for (int u = 0; u < GTM; u++) {
-      if (u < ntw && ((fb >> u) & 1u)) {
-        const double2* sp = reinterpret_cast<const double2*>(gsum + (u * 32 + lane) * 4);
-        const double2 a = __ldcg(sp), b = __ldcg(sp + 1);
-        acc[u][0] = a.x + acc[u][0]; acc[u][1] = a.y + acc[u][1];
-        acc[u][2] = b.x + acc[u][2]; acc[u][3] = b.y + acc[u][3];
-      }
+  if (tid == 0) {  // the stages that beta overlapped
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (int c = 1; c < P.gstages && c * P.chg < P.QG; c++) {
+      mbar_expect_tx(&mbar_s[c], chunk_bytes);
+      bulk_g2s(sm + P.g_fref + c * P.gstage, P.frefG + (size_t)c * P.chg * P.featstride, chunk_bytes, &mbar_s[c]);
     }
   }
-  // accumulators -> tile-lower shared storage (overlaps the staging area); tiles of
-  // uncoupled var pairs are zero
+  if (d == 3) gram_chunks3d<GTM>(P, L, P.sm_nodes);
+  else gram_body<GTM, 2>(P, L, P.sm_nodes);
+  // tiles of uncoupled var pairs are zero
   for (int e = tid; e < P.ngz * 64; e += NT) GT[P.gzero[e >> 6] * 64 + (e & 63)] = 0.0;
-#pragma unroll
-  for (int u = 0; u < GTM; u++) {
-    if (u < ntw) {
-      const int4 T = tdesc[u];
-      const int I = T.x & 0xffff, J = (T.x >> 16) & 0xff;
-      if (J <= I)
-        *reinterpret_cast<double2*>(GT + (I * (I + 1) / 2 + J) * 64 + ak_cfrag(g, t)) = make_double2(acc[u][0], acc[u][1]);
-      if (!(T.x >> 24))
-        *reinterpret_cast<double2*>(GT + ((I + 1) * (I + 2) / 2 + J) * 64 + ak_cfrag(g, t)) =
-            make_double2(acc[u][2], acc[u][3]);
-    }
-  }
   __syncthreads();
   // padded rows decouple: unit diagonal
   for (int r = tid; r < P.Np; r += NT)
@@ -863,7 +944,6 @@ __device__ __forceinline__ void phase_factor(const DpgPlanDev& P) {
   DPG_SMEM_VIEWS(P);
   double* GT = sm + P.sm_gt;
   double* scale = sm + P.sm_scale;
-  double* LINV = sm + P.sm_linv;
   for (int r = tid; r < P.Np; r += NT) {
     int I = r >> 3;
     double dg = GT[(I * (I + 1) / 2 + I) * 64 + ak(r & 7, r & 7)];
@@ -1006,7 +1086,7 @@ __device__ __forceinline__ void phase_trsm(const DpgPlanDev& P, const DpgLaunch&
 // ---------------------------------------------------------------------------
 // Phase 5/6: K_ext = W^T W, outputs, condensation
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void phase_syrk_out(const DpgPlanDev& P, const DpgLaunch& L, int cell, const Ctx& X) {
+__device__ __forceinline__ void phase_syrk_out(const DpgPlanDev& P, const DpgLaunch& L, int cell) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   DPG_SMEM_VIEWS(P);
@@ -1098,7 +1178,7 @@ __device__ __forceinline__ void cta_setup(const DpgPlanDev& P) {
   double* const sm = dpg_smem;
   int* tri_s = reinterpret_cast<int*>(sm + P.sm_nodes + 32);
   DpgGTile* tiles_s = reinterpret_cast<DpgGTile*>(sm + P.sm_tiles);
-  uint64_t* mbar_s = reinterpret_cast<uint64_t*>(sm + P.sm_nodes + 26);
+  uint64_t* mbar_s = reinterpret_cast<uint64_t*>(sm + P.sm_nodes + DPG_SM_BARS);
   const int ntri = DPG_MAX_NBT * (DPG_MAX_NBT + 1) / 2;
   for (int u = tid; u < ntri; u += NT) {
     int I = (int)((sqrt(8.0 * u + 1.0) - 1.0) * 0.5);
@@ -1106,9 +1186,14 @@ __device__ __forceinline__ void cta_setup(const DpgPlanDev& P) {
     while (I * (I + 1) / 2 > u) I--;
     tri_s[u] = I | ((u - I * (I + 1) / 2) << 8);
   }
-  for (int u = tid; u < P.ngb; u += NT) tiles_s[u] = P.gtiles[u];
+  for (int u = tid; u < P.ngb && P.gtiles; u += NT) tiles_s[u] = P.gtiles[u];
   if (tid == 0) {
-    for (int i = 0; i < 4; i++) mbar_init(&mbar_s[i], 1);
+    for (int i = 0; i < DPG_NBARS; i++) mbar_init(&mbar_s[i], i < DPG_BAR_EMPTY ? 1 : DPG_NWARPS);
+    int* const gp = reinterpret_cast<int*>(sm + P.sm_nodes + DPG_SM_GRAM);
+    reinterpret_cast<int*>(sm + P.sm_nodes + 24)[3] = 0;
+    gp[GP_CHG] = P.chg; gp[GP_QG] = P.QG; gp[GP_RING] = P.g_fref; gp[GP_STAGE] = P.gstage; gp[GP_STAGES] = P.gstages;
+    gp[GP_FLUSH] = P.gflush; gp[GP_D] = P.g_D; gp[GP_NGB] = P.ngb; gp[GP_TILES] = P.sm_tiles; gp[GP_FS] = P.featstride;
+    gp[GP_DS] = P.npairs * 16 + 2; gp[GP_GT] = P.sm_gt; gp[GP_PAR] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();

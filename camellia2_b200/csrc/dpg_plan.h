@@ -31,6 +31,13 @@
 #define DPG_NWARPS 16
 #define DPG_NTHREADS (DPG_NWARPS * 32)
 #define DPG_CHG 8         // Gram quadrature points per staged chunk (4 when shared memory is short)
+#define DPG_GSTAGES 4     // most stages of the Gram chunk ring
+#define DPG_BAR_B DPG_GSTAGES            // mbarriers: Gram stages full, the two B-phase buffers,
+#define DPG_BAR_EMPTY (DPG_GSTAGES + 2)  // Gram stages empty
+#define DPG_NBARS (2 * DPG_GSTAGES + 2)
+#define DPG_SM_BARS 182   // their place (doubles) in the persistent region
+#define DPG_SM_GRAM 192   // chunk loop parameters (ints)
+#define DPG_SM_PERSIST 208  // doubles of the persistent region
 #define DPG_MAX_CHB 16    // max B quadrature points per staged chunk
 #define DPG_MAX_BT 12     // max terms feeding one B block
 #define DPG_MAX_BTW 12    // max active B tiles per warp per segment
@@ -122,7 +129,8 @@ struct DpgTestVar {
 struct DpgGTile {
   int16_t I, J;    // J | 0x100: one row tile only
   int16_t lda, ldb;
-  int aoff, boff;  // A operand / B operand offsets inside a point's feature / h block
+  int aoff, boff;  // row var's slots at the block's rows | var pair << 16, column var's slots at its columns
+                   // (offsets inside a point's staged slots)
 };
 
 struct DpgPlanDev {
@@ -143,16 +151,16 @@ struct DpgPlanDev {
   DpgIPEnt ipent[DPG_MAX_IP];
   int npairs;
   int pair_a[DPG_MAX_PAIRS], pair_b[DPG_MAX_PAIRS];
-  int hoff[DPG_MAX_PAIRS];  // offset of h_{b->a} inside a point's h block
   int rowstart[DPG_MAX_IPROWS + 1];  // IP entries of row r: [rowstart[r], rowstart[r+1])
   int ngt;                  // lower 8x8 tiles of G: NBT (NBT + 1) / 2
   int ngb;                  // 16x8 G blocks
   const DpgGTile* gtiles;   // [ngb]
   int ngz;                  // lower tiles of G that no block writes (uncoupled test var pairs)
   const int* gzero;         // [ngz] their indices I (I + 1) / 2 + J
-  int chg;                  // Gram points per staged chunk (DPG_CHG or DPG_CHG / 2)
-  int featstride;           // doubles per point of staged slots (sum over vars of 4*ldA)
-  int hstride;              // doubles per point of staged h blocks (sum over pairs)
+  int chg;                  // Gram points per staged chunk (2 DPG_CHG, DPG_CHG or DPG_CHG / 2)
+  int gstages, gstage;      // stages of the chunk ring, doubles per stage
+  int featstride;           // doubles per point of staged slots (sum over vars of 4*ldA, then 4: points
+                            // 4 doubles apart in bank position)
   const double* frefG;      // [QGpad][featstride]
   const double* wG;         // [QGpad]
   const double* dNG;        // [QGpad][nv][d]
@@ -187,9 +195,9 @@ struct DpgPlanDev {
   // shared memory layout (doubles)
   int sm_total;
   int sm_tiles;   // persistent: tile table copy
-  int sm_nodes;   // persistent: cell vertices, flags, mbarriers, triangular index table (192 doubles)
+  int sm_nodes;   // persistent: cell vertices, flags, mbarriers, triangular index table (DPG_SM_PERSIST doubles)
   int sm_coef;    // per cell: coefficients [nslots][Ptot]
-  int g_fref0, g_fref1, g_h, g_geo, g_D, g_beta;   // Gram phase (g_beta overlaps g_h)
+  int g_fref, g_geo, g_D, g_beta;   // Gram phase (g_beta overlaps the stages after the first)
   int sm_gt, sm_linv, sm_scale;                    // factor
   int b_rec0, b_rec1, b_u, b_geo, b_fac;      // B phase
   int sm_w, sm_k;                                  // solve / Gram of W

@@ -36,9 +36,6 @@ __global__ void __launch_bounds__(NT, 1) dpg_queue_kernel(const DpgPlanDev* __re
                                                           const int* __restrict__ cstart, int nb,
                                                           int* __restrict__ counters, int claim, int claim_slot) {
   const int tid = threadIdx.x;
-  Ctx X;
-  uint32_t phase[4] = {0, 0, 0, 0};
-  X.phase = phase;
   double* const sm = dpg_smem;
   volatile int* const claim_s = reinterpret_cast<volatile int*>(sm + claim_slot);
   int cur = -1;
@@ -55,12 +52,11 @@ __global__ void __launch_bounds__(NT, 1) dpg_queue_kernel(const DpgPlanDev* __re
       if (b != cur) {
         __syncthreads();
         if (cur >= 0 && tid == 0) {
-          uint64_t* old = reinterpret_cast<uint64_t*>(sm + plans[cur].sm_nodes + 26);
-          for (int k = 0; k < 4; k++) mbar_inval(&old[k]);
+          uint64_t* old = reinterpret_cast<uint64_t*>(sm + plans[cur].sm_nodes + DPG_SM_BARS);
+          for (int k = 0; k < DPG_NBARS; k++) mbar_inval(&old[k]);
         }
         __syncthreads();
         cta_setup(P);
-        for (int k = 0; k < 4; k++) phase[k] = 0;
         cur = b;
       }
       const int cell = i - cstart[b];
@@ -73,12 +69,12 @@ __global__ void __launch_bounds__(NT, 1) dpg_queue_kernel(const DpgPlanDev* __re
       if (L.coeff)
         for (int k = tid; k < nco; k += NT) coef_s[k] = L.coeff[(size_t)cell * nco + k];
       __syncthreads();
-      phase_b<BTW>(P, L, cell, X);
+      phase_b<BTW>(P, L, cell);
       __syncthreads();
-      phase_gram<GTM, 0>(P, L, cell, X);
+      phase_gram<GTM>(P, L, cell);
       phase_factor(P);
     phase_trsm<NBTM>(P, L, cell);
-      phase_syrk_out(P, L, cell, X);
+      phase_syrk_out(P, L, cell);
       __syncthreads();
       if (tid == 0 && L.info) {
         int v = 0;
