@@ -10,7 +10,7 @@ import sys
 import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = [os.path.join(HERE, "csrc", f"dpg_{f}.cu") for f in ("host", "kernel", "queue", "adjoint", "energy", "big", "maps")]
+SRC = [os.path.join(HERE, "csrc", f"dpg_{f}.cu") for f in ("host", "kernel", "small", "queue", "adjoint", "energy", "big", "maps")]
 OUT = os.path.join(HERE, "libdpg_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

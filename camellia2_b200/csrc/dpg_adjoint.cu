@@ -5,10 +5,19 @@ namespace {
 #include "dpg_adjoint.cuh"
 }  // namespace
 
+static DpgKernelChoice choose_adjoint_kernel(const DpgPlanDev* plan) {
+  DpgKernelChoice c = dpg_small_kernel(plan, DPG_KIND_ADJOINT);
+  if (!c.k) c = DpgKernelChoice{pick_adjoint_kernel(plan), NT, 1};
+  return c;
+}
+
 int dpg_configure_adjoint(const DpgPlanDev* plan, int bytes) {
-  KernelFn k = pick_adjoint_kernel(plan);
+  const DpgKernelChoice kc = choose_adjoint_kernel(plan);
+  KernelFn k = kc.k;
   if (!k) return DPG_OK;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && kc.per_sm > 1)
+    e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
   return DPG_OK;
 }
@@ -16,9 +25,10 @@ int dpg_configure_adjoint(const DpgPlanDev* plan, int bytes) {
 int dpg_launch_adjoint(const DpgPlanDev* plan, const DpgLaunch* Lin, cudaStream_t stream) {
   if (Lin->C <= 0) return DPG_OK;
   if (!plan->adj_ok) return dpg::fail(DPG_ERR_UNSUPPORTED, "reverse mode is not available for this bucket");
-  KernelFn k = pick_adjoint_kernel(plan);
+  const DpgKernelChoice kc = choose_adjoint_kernel(plan);
+  KernelFn k = kc.k;
   if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no adjoint kernel instance for this bucket size");
-  const int grid = std::min(Lin->C, dpg::num_sms());
+  const int grid = std::min(Lin->C, dpg::num_sms() * kc.per_sm);
   DpgLaunch L = *Lin;
   void* scratch = nullptr;
   const size_t per = plan->scratch_per_cta;
@@ -30,7 +40,7 @@ int dpg_launch_adjoint(const DpgPlanDev* plan, const DpgLaunch* Lin, cudaStream_
   L.scratch = (double*)scratch;
   L.scratch2 = L.scratch + (size_t)grid * per;
   size_t bytes = (size_t)plan->sm_total * sizeof(double);
-  k<<<grid, NT, bytes, stream>>>(*plan, L);
+  k<<<grid, kc.threads, bytes, stream>>>(*plan, L);
   cudaError_t e = cudaGetLastError();
   cudaFreeAsync(scratch, stream);
   if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));

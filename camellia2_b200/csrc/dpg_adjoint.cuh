@@ -153,7 +153,7 @@ __device__ __forceinline__ void adj_feature_gemm(const DpgPlanDev& P, const DpgL
   const double* xe = L.scratch + (size_t)blockIdx.x * P.scratch_per_cta;
   const double* pm = L.scratch2 + (size_t)blockIdx.x * P.scratch_per_cta;
   const int q0 = g >> 2, q1 = 2 + (g >> 2), k = g & 3;
-  for (int ct = warp; ct < nct; ct += DPG_NWARPS) {
+  for (int ct = warp; ct < nct; ct += NW) {
     const bool from_xe = ct < ncx;
     const int J = from_xe ? ct : ct - ncx;
     const double* src = from_xe ? xe : pm;
@@ -239,7 +239,7 @@ __device__ __forceinline__ void phase_adj_pull(const DpgPlanDev& P, const DpgLau
       adj_feature_gemm(P, L, fs, P.featstride, nq, 2 * P.MBT, P.MBT, xpf);
       __syncthreads();
       // one warp per (point, slot): sum over the IP entries carrying the slot
-      for (int task = warp; task < nq * P.nslots; task += DPG_NWARPS) {
+      for (int task = warp; task < nq * P.nslots; task += NW) {
         const int q = task / P.nslots, s = task - q * P.nslots;
         const double* gq = geo + q * GEO;
         double val = 0.0;
@@ -282,7 +282,7 @@ __device__ __forceinline__ void phase_adj_pull(const DpgPlanDev& P, const DpgLau
       __syncthreads();
       adj_feature_gemm(P, L, fs, S.rec_len, nq, P.MBT, 0, xpf);
       __syncthreads();
-      for (int task = warp; task < nq * P.nslots; task += DPG_NWARPS) {
+      for (int task = warp; task < nq * P.nslots; task += NW) {
         const int q = task / P.nslots, s = task - q * P.nslots;
         const double* gq = geo + q * GEO;
         double val = 0.0;
@@ -317,7 +317,7 @@ __device__ __forceinline__ void phase_adj_pull(const DpgPlanDev& P, const DpgLau
       point_geometry(d, nv, nodes_s, P.dNB + (size_t)(P.QB + i) * nv * d, P.wB[P.QB + i], P.tangB + (size_t)(P.QB + i) * 6,
                      geo + i * GEO);
     __syncthreads();
-    for (int task = warp; task < nsp * P.nslots; task += DPG_NWARPS) {
+    for (int task = warp; task < nsp * P.nslots; task += NW) {
       const int sp = task / P.nslots, s = task - sp * P.nslots;
       const int sd = sp / P.QS, q = sp - sd * P.QS;
       const double* gq = geo + sp * GEO;
@@ -349,7 +349,7 @@ __device__ __forceinline__ void phase_adj_pull(const DpgPlanDev& P, const DpgLau
 }
 
 template <int NBTM, int GTM, int BTW>
-__global__ void __launch_bounds__(NT, 1) dpg_adjoint_kernel(const __grid_constant__ DpgPlanDev P,
+__global__ void __launch_bounds__(NT, CTAS_PER_SM) dpg_adjoint_kernel(const __grid_constant__ DpgPlanDev P,
                                                                   const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x;
   double* const sm = dpg_smem;
@@ -385,12 +385,16 @@ __global__ void __launch_bounds__(NT, 1) dpg_adjoint_kernel(const __grid_constan
   }
 }
 
+#if DPG_CTA_WARPS == DPG_NWARPS
 #define DPG_ADJ_INSTANCES(X) X(12, 5, 4) X(16, 6, 4) X(20, 8, 4) X(24, 12, 6)
+#else
+#define DPG_ADJ_INSTANCES(X) X(9, 4, 4) X(14, 8, 6)
+#endif
 
 KernelFn pick_adjoint_kernel(const DpgPlanDev* plan) {
-  const int per = (plan->ngb + DPG_NWARPS - 1) / DPG_NWARPS;
+  const int per = (plan->ngb + NW - 1) / NW;
   int btw = 0;
-  for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);
+  for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + NW - 1) / NW);
 #define DPG_PICK(NB, GT, BT) \
   if (plan->NBT <= NB && per <= GT && btw <= BT) return dpg_adjoint_kernel<NB, GT, BT>;
   DPG_ADJ_INSTANCES(DPG_PICK)

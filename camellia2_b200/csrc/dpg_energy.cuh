@@ -24,7 +24,7 @@ __device__ __forceinline__ void energy_residual(const DpgPlanDev& P, const DpgLa
 }
 
 template <int NBTM, int GTM, int BTW>
-__global__ void __launch_bounds__(NT, 1) dpg_energy_kernel(const __grid_constant__ DpgPlanDev P,
+__global__ void __launch_bounds__(NT, CTAS_PER_SM) dpg_energy_kernel(const __grid_constant__ DpgPlanDev P,
                                                                   const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* const sm = dpg_smem;
@@ -74,12 +74,16 @@ __global__ void __launch_bounds__(NT, 1) dpg_energy_kernel(const __grid_constant
   }
 }
 
+#if DPG_CTA_WARPS == DPG_NWARPS
 #define DPG_ENERGY_INSTANCES(X) X(12, 5, 4) X(16, 6, 4) X(20, 8, 4) X(22, 9, 3) X(24, 12, 6)
+#else
+#define DPG_ENERGY_INSTANCES(X) X(9, 4, 4) X(14, 8, 6)
+#endif
 
 static KernelFn pick_energy_kernel(const DpgPlanDev* plan) {
-  const int per = (plan->ngb + DPG_NWARPS - 1) / DPG_NWARPS;
+  const int per = (plan->ngb + NW - 1) / NW;
   int btw = 0;
-  for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);
+  for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + NW - 1) / NW);
 #define DPG_PICK(NB, GT, BT) \
   if (plan->NBT <= NB && per <= GT && btw <= BT) return dpg_energy_kernel<NB, GT, BT>;
   DPG_ENERGY_INSTANCES(DPG_PICK)
@@ -91,7 +95,7 @@ static KernelFn pick_energy_kernel(const DpgPlanDev* plan) {
 // factored solve overwrites B and F in place): W = L^-1 B as (C, M, N) "trial x
 // test" and y = L^-1 F as (C, N), user numbering, L the unscaled Cholesky factor of G.
 template <int NBTM, int GTM, int BTW>
-__global__ void __launch_bounds__(NT, 1) dpg_dls_kernel(const __grid_constant__ DpgPlanDev P,
+__global__ void __launch_bounds__(NT, CTAS_PER_SM) dpg_dls_kernel(const __grid_constant__ DpgPlanDev P,
                                                                   const __grid_constant__ DpgLaunch L) {
   const int tid = threadIdx.x;
   double* const sm = dpg_smem;
@@ -138,9 +142,9 @@ __global__ void __launch_bounds__(NT, 1) dpg_dls_kernel(const __grid_constant__ 
 }
 
 static KernelFn pick_dls_kernel(const DpgPlanDev* plan) {
-  const int per = (plan->ngb + DPG_NWARPS - 1) / DPG_NWARPS;
+  const int per = (plan->ngb + NW - 1) / NW;
   int btw = 0;
-  for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);
+  for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + NW - 1) / NW);
 #define DPG_PICK(NB, GT, BT) \
   if (plan->NBT <= NB && per <= GT && btw <= BT) return dpg_dls_kernel<NB, GT, BT>;
   DPG_ENERGY_INSTANCES(DPG_PICK)

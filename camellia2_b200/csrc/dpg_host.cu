@@ -589,7 +589,7 @@ static int big_layout(HostPlan* P) {
   g.bs_int = s; s += 256;  // 512 ints: flags, chunk point maps, relevance lists
   g.bs_nodes = s; s += 32;
   g.bs_total = s;
-  if ((size_t)s * 8 > 232448) return fail(DPG_ERR_UNSUPPORTED, "large-bucket kernel: shared memory exceeded");
+  if (s * 8 > DPG_SMEM) return fail(DPG_ERR_UNSUPPORTED, "large-bucket kernel: shared memory exceeded");
   g.sm_total = s;
   return DPG_OK;
 }
@@ -650,7 +650,8 @@ static int smem_layout_stages(DpgPlanDev& g, int chg, int stages, bool adj_terms
     g.a_cbar = q; q += al(std::max(1, g.nslots * g.Ptot));
     const int ngt16 = g.nbt16 * (g.nbt16 + 1) / 2;
     const int body16 = std::max(std::max(body, g.MBT * g.nbt16 * 64), (ngt16 + g.nbt16) * 64 + g.nbt16 * 8);
-    g.adj_ok = adj_terms_ok && std::max(sa_end, q) <= body16 && g.QB > 0;
+    // a small layout makes room for the reverse mode wherever the full one has it
+    g.adj_ok = g.small ? g.adj_ok : adj_terms_ok && std::max(sa_end, q) <= body16 && g.QB > 0;
     if (g.adj_ok) body = std::max(body, std::max(sa_end, q));
   }
   g.sm_coef = al(body);
@@ -659,7 +660,7 @@ static int smem_layout_stages(DpgPlanDev& g, int chg, int stages, bool adj_terms
   g.sm_total = g.sm_nodes + DPG_SM_PERSIST;
   // the larger rings leave room for the work queue's claim slot behind the plan's layout
   const int reserve = chg * stages > DPG_CHG ? 4 : 0;
-  if ((size_t)(g.sm_total + reserve) * 8 > 232448) return -1;
+  if ((g.sm_total + reserve) * 8 > (g.small ? DPG_SMALL_SMEM : DPG_SMEM)) return -1;
   // Gram sums in two levels: after every 32 points the warps' DMMA accumulators of the
   // blocks that several graph-norm terms feed are added into FP64 running sums in the
   // CTA's scratch slot and restart from zero.  A single running sum over all points and
@@ -1032,16 +1033,8 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
       }
     g.ngb = (int)tiles.size();
     g.ngt = g.NBT * (g.NBT + 1) / 2;
-    {  // the kernel's balanced block ownership: warp w owns blocks [tau0, tau0 + ntw)
-      const int gbase = g.ngb / DPG_NWARPS, gextra = g.ngb % DPG_NWARPS;
-      for (int w = 0; w < DPG_NWARPS; w++) {
-        const int ntw = gbase + (w < gextra ? 1 : 0), tau0 = w * gbase + std::min(w, gextra);
-        uint32_t bits = 0;
-        for (int u = 0; u < ntw && u < 32; u++)
-          if (tile_multi[tau0 + u]) bits |= 1u << u;
-        g.gflushbits[w] = bits;
-      }
-    }
+    for (int b = 0; b < g.ngb && b < DPG_MAX_GT * DPG_NWARPS; b++)
+      if (tile_multi[b]) g.gflushmask[b >> 5] |= 1u << (b & 31);
     std::vector<int> gz;  // lower tiles no block writes (uncoupled var pairs)
     for (int u = 0; u < g.ngt && !g.big; u++)
       if (!covered[u]) gz.push_back(u);
@@ -1138,9 +1131,6 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     g.wB = upload(P, wall);
     g.tangB = upload(P, tall);
   }
-  // shared-memory budget for the B phase: two record buffers, U, geometry of all
-  // B points, per-point term rows R, coefficients
-  const int budget = 232448 / 8 - DPG_SM_PERSIST - 2 * ((g.ngb * (int)sizeof(DpgGTile) + 7) / 8) - 64 - g.Np - g.Mp - 64;
   g.max_rec = 0; g.max_chunk = 0; g.max_ustride = 0; g.max_nterm = 0;
   std::vector<int4> btiles;
   for (int sg = 0; sg < g.nseg; sg++) {
@@ -1203,18 +1193,57 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     P->allocs.push_back(p);
     g.btiles = (const int4*)p;
   }
+  // coefficient uses the reverse mode covers: IP entries, volume B and load terms,
+  // separable side terms
+  for (int e = 0; e < g.nipent; e++) g.ip_slots |= g.ipent[e].slot >= 0;
+  bool adj_terms_ok = true;
+  for (int sg = 0; sg < g.nseg; sg++)
+    for (int lt = 0; lt < g.seg[sg].nterm; lt++) {
+      const DpgBTerm& t = g.bterm[g.seg[sg].term0 + lt];
+      if (t.slot < 0) continue;
+      if (sg == 0) g.b_slots = 1;
+      else adj_terms_ok = false;  // a non-separable side term with a coefficient
+    }
+  P->adj_terms_ok = adj_terms_ok;
   // chunk size: all points of a side in one chunk when it fits; the volume in equal chunks
   {
-    auto fits = [&](int ch) {
+    // shared-memory budget for the B phase: two record buffers, U, geometry of all
+    // B points, per-point term rows R, coefficients
+    auto fits = [&](int ch, int smem) {
+      const int budget = smem / 8 - DPG_SM_PERSIST - 2 * ((g.ngb * (int)sizeof(DpgGTile) + 7) / 8) - 64 - g.Np - g.Mp - 64;
       int need = 2 * ch * g.max_rec + ch * g.max_ustride + g.nbpts * 24 + g.nslots * g.Ptot + 64 +
                  (int)sterms.size() * g.QS + 16;
       return need <= budget;
     };
     // chunks are multiples of 4 points (one m16n8k16 k-step = 4 points x 4 slots)
-    int ch = DPG_MAX_CHB;
-    while (ch > 4 && !fits(ch)) ch -= 4;
+    auto largest = [&](int smem) {
+      int ch = DPG_MAX_CHB;
+      while (ch > 4 && !fits(ch, smem)) ch -= 4;
+      return ch;
+    };
+    int ch = largest(DPG_SMEM);
+    // small buckets (at most one column tile per warp of an 8-warp CTA, eight G blocks and six B blocks):
+    // two CTAs per SM when every phase fits half the shared memory
+    int btw = 0;
+    for (int sg = 0; sg < g.nseg; sg++) btw = std::max(btw, g.seg[sg].ntile);
+    if (!g.big && g.NBT <= 14 && g.MBT <= DPG_SMALL_WARPS && g.ngb <= 8 * DPG_SMALL_WARPS && btw <= 6 * DPG_SMALL_WARPS) {
+      const int chs = largest(DPG_SMALL_SMEM);
+      if (fits(chs, DPG_SMALL_SMEM)) {
+        g.nse = (int)sterms.size();
+        g.max_chunk = std::min(ch, (g.seg[0].npts + 3) & ~3);
+        for (int sg = 1; sg < g.nseg; sg++)
+          if (g.seg[sg].nterm > 0) g.max_chunk = std::max(g.max_chunk, std::min(ch, (g.seg[sg].npts + 3) & ~3));
+        if (smem_layout(g, DPG_CHG, adj_terms_ok) != DPG_OK) smem_layout(g, DPG_CHG / 2, adj_terms_ok);  // adj_ok
+        g.small = 1;
+        g.max_chunk = chs;
+        if (smem_layout(g, DPG_CHG, adj_terms_ok) == DPG_OK || smem_layout(g, DPG_CHG / 2, adj_terms_ok) == DPG_OK) ch = chs;
+        else g.small = 0;
+        g.max_chunk = 0;
+      }
+    }
     if (g.big) ch = 1 << 20;  // no staging: one chunk per segment
-    else if (!fits(ch)) return fail(DPG_ERR_UNSUPPORTED, "B-phase staging does not fit in shared memory");
+    else if (!fits(ch, g.small ? DPG_SMALL_SMEM : DPG_SMEM))
+      return fail(DPG_ERR_UNSUPPORTED, "B-phase staging does not fit in shared memory");
     for (int sg = 0; sg < g.nseg; sg++) {
       DpgSeg& S = g.seg[sg];
       if (S.nterm == 0) continue;
@@ -1381,18 +1410,6 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     g.scon_rc = (const int2*)p;
     for (const DpgSideTerm& st : ses) g.se_slots |= st.slot >= 0;
   }
-  // coefficient uses the reverse mode covers: IP entries, volume B and load terms,
-  // separable side terms
-  for (int e = 0; e < g.nipent; e++) g.ip_slots |= g.ipent[e].slot >= 0;
-  bool adj_terms_ok = true;
-  for (int sg = 0; sg < g.nseg; sg++)
-    for (int lt = 0; lt < g.seg[sg].nterm; lt++) {
-      const DpgBTerm& t = g.bterm[g.seg[sg].term0 + lt];
-      if (t.slot < 0) continue;
-      if (sg == 0) g.b_slots = 1;
-      else adj_terms_ok = false;  // a non-separable side term with a coefficient
-    }
-
   if (g.big) {
     int rc = big_layout(P);
     if (rc != DPG_OK) return rc;
@@ -1404,7 +1421,6 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     if (rc == -1) return fail(DPG_ERR_UNSUPPORTED, "bucket needs more shared memory than one CTA has");
     if (rc != DPG_OK) return rc;
   }
-  P->adj_terms_ok = adj_terms_ok;
   // info
   dpg_plan_info& I = P->info;
   I.N = g.N; I.M = g.M; I.n_field = g.nf; I.n_trace = g.nt;

@@ -52,6 +52,15 @@ struct DpgLaunch {
   double* energy;
 };
 
+// A kernel instance, its threads per CTA and CTAs per SM.
+typedef void (*DpgKernelFn)(const DpgPlanDev, const DpgLaunch);
+struct DpgKernelChoice {
+  DpgKernelFn k;
+  int threads, per_sm;
+};
+enum { DPG_KIND_ASSEMBLE, DPG_KIND_ADJOINT, DPG_KIND_ENERGY, DPG_KIND_DLS };
+DpgKernelChoice dpg_small_kernel(const DpgPlanDev* plan, int kind);  // k null: not a small bucket
+
 int dpg_configure_kernels(const DpgPlanDev* plan);
 int dpg_configure_adjoint(const DpgPlanDev* plan, int bytes);
 int dpg_configure_big(const DpgPlanDev* plan);

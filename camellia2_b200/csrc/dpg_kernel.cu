@@ -29,86 +29,7 @@
 
 namespace {
 
-template <int NBTM, int GTM, int BTW>
-__global__ void __launch_bounds__(NT, 1) dpg_cell_kernel(const __grid_constant__ DpgPlanDev P,
-                                                                  const __grid_constant__ DpgLaunch L) {
-  const int tid = threadIdx.x;
-  double* const sm = dpg_smem;
-  double* nodes_s = sm + P.sm_nodes;
-  int* flag_s = reinterpret_cast<int*>(sm + P.sm_nodes + 24);
-  int* tri_s = reinterpret_cast<int*>(sm + P.sm_nodes + 32);
-  double* coef_s = sm + P.sm_coef;
-  cta_setup(P);
-
-  for (int cell = blockIdx.x; cell < L.C; cell += gridDim.x) {
-    if (tid == 0) { flag_s[0] = 0; flag_s[1] = 0; flag_s[2] = 0; }
-    if (!L.solve_only) {
-      if (tid < P.nv * P.d) nodes_s[tid] = L.nodes[(size_t)cell * P.nv * P.d + tid];
-      const int nco = P.nslots * P.Ptot;
-      if (L.coeff)
-        for (int i = tid; i < nco; i += NT) coef_s[i] = L.coeff[(size_t)cell * nco + i];
-    }
-    __syncthreads();
-    double* GT = sm + P.sm_gt;
-    if (L.solve_only) {
-      const double* Gc = L.Gin + (size_t)cell * P.N * P.N;
-      for (int e = tid; e < P.ngt * 64; e += NT) {
-        int tau = e >> 6, idx = e & 63;
-        int ij = tri_s[tau];
-        int I = ij & 255, J = ij >> 8;
-        int r = (idx >> 2) & 7, c = (idx >> 5) * 4 + (idx & 3);
-        int gr = I * 8 + r, gc = J * 8 + c;
-        double v = 0.0;
-        if (gr < P.N && gc < P.N) v = Gc[(size_t)gr * P.N + gc];
-        else if (gr == gc) v = 1.0;
-        GT[e] = v;
-      }
-      __syncthreads();
-    } else {
-      phase_b<BTW>(P, L, cell);
-      __syncthreads();
-      phase_gram<GTM>(P, L, cell);
-      if (L.parts) {
-        __syncthreads();
-        continue;
-      }
-    }
-    phase_factor(P);
-    phase_trsm<NBTM>(P, L, cell);
-    phase_syrk_out(P, L, cell);
-    __syncthreads();
-    if (tid == 0 && L.info) {
-      int f0 = flag_s[0], f1 = flag_s[1];
-      int v = 0;
-      if (flag_s[2]) {
-        v = ERR_TIMEOUT_FLAG;
-      } else if (f0 != 0) {
-        int r = f0 - 1;
-        int u = L.solve_only ? r : P.dev2user_test[r];
-        v = (u >= 0 ? u : r) + 1;
-      } else if (f1 != 0) {
-        v = f1;
-      }
-      L.info[cell] = v;
-    }
-    __syncthreads();
-  }
-}
-
-// Instances: register arrays sized for the test-tile count of the bucket.
-#define DPG_INSTANCES(X) \
-  X(8, 3, 4) X(12, 5, 4) X(16, 6, 4) X(18, 8, 4) X(20, 8, 4) X(22, 9, 3) X(24, 12, 4) X(24, 12, 6)
-
-static KernelFn pick_kernel(const DpgPlanDev* plan) {
-  const int per = (plan->ngb + DPG_NWARPS - 1) / DPG_NWARPS;
-  int btw = 0;
-  for (int s = 0; s < plan->nseg; s++) btw = std::max(btw, (plan->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);
-#define DPG_PICK(NB, GT, BT) \
-  if (plan->NBT <= NB && per <= GT && btw <= BT) return dpg_cell_kernel<NB, GT, BT>;
-  DPG_INSTANCES(DPG_PICK)
-#undef DPG_PICK
-  return nullptr;
-}
+#include "dpg_cell.cuh"
 
 }  // namespace
 
@@ -168,9 +89,17 @@ cudaError_t ws_alloc(void** p, size_t bytes, cudaStream_t s) {
 }
 }  // namespace dpg
 
+// The small buckets run two CTAs per SM.
+static DpgKernelChoice choose_kernel(const DpgPlanDev* plan) {
+  DpgKernelChoice c = dpg_small_kernel(plan, DPG_KIND_ASSEMBLE);
+  if (!c.k) c = DpgKernelChoice{pick_kernel(plan), NT, 1};
+  return c;
+}
+
 int dpg_configure_kernels(const DpgPlanDev* plan) {
   if (plan->big) return dpg_configure_big(plan);
-  KernelFn k = pick_kernel(plan);
+  const DpgKernelChoice kc = choose_kernel(plan);
+  KernelFn k = kc.k;
   if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no kernel instance for this bucket size");
   // Several plans may share a kernel instance: the opt-in limit is the device's
   // maximum, so configuring one plan never lowers another's.
@@ -181,6 +110,8 @@ int dpg_configure_kernels(const DpgPlanDev* plan) {
   if (optin > 0 && bytes > (size_t)optin) return dpg::fail(DPG_ERR_UNSUPPORTED, "bucket needs more shared memory than one CTA has");
   if (optin > 0) bytes = (size_t)optin;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess && kc.per_sm > 1)
+    e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
   return plan->adj_ok ? dpg_configure_adjoint(plan, (int)bytes) : DPG_OK;
 }
@@ -189,9 +120,10 @@ int dpg_launch_assemble(const DpgPlanDev* plan, const DpgPlanDev* d_plan, const 
   (void)d_plan;
   if (Lin->C <= 0) return DPG_OK;
   if (plan->big) return dpg_launch_big(plan, Lin, stream);
-  KernelFn k = pick_kernel(plan);
+  const DpgKernelChoice kc = choose_kernel(plan);
+  KernelFn k = kc.k;
   if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no kernel instance for this bucket size");
-  const int grid = std::min(Lin->C, dpg::num_sms());
+  const int grid = std::min(Lin->C, dpg::num_sms() * kc.per_sm);
   DpgLaunch L = *Lin;
   void* scratch = nullptr;
   const bool need_scratch = !L.solve_only && plan->scratch_per_cta > 0 && !L.scratch;
@@ -204,7 +136,7 @@ int dpg_launch_assemble(const DpgPlanDev* plan, const DpgPlanDev* d_plan, const 
     L.scratch = (double*)scratch;
   }
   size_t bytes = (size_t)plan->sm_total * sizeof(double);
-  k<<<grid, NT, bytes, stream>>>(*plan, L);
+  k<<<grid, kc.threads, bytes, stream>>>(*plan, L);
   cudaError_t e = cudaGetLastError();
   if (scratch) cudaFreeAsync(scratch, stream);
   if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
@@ -519,7 +451,8 @@ unsigned long long current_context_id() {
 int dpg_launch_assemble_noalloc(const DpgPlanDev* plan, const DpgLaunch* Lin, cudaStream_t stream) {
   if (Lin->C <= 0) return DPG_OK;
   if (plan->big) return dpg::fail(DPG_ERR_UNSUPPORTED, "dpg_assemble_noalloc: large-bucket plans need dpg_assemble");
-  KernelFn k = pick_kernel(plan);
+  const DpgKernelChoice kc = choose_kernel(plan);
+  KernelFn k = kc.k;
   if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no kernel instance for this bucket size");
   if (plan->scratch_per_cta > DPG_NOALLOC_SCRATCH_DOUBLES)
     return dpg::fail(DPG_ERR_UNSUPPORTED,
@@ -547,12 +480,12 @@ int dpg_launch_assemble_noalloc(const DpgPlanDev* plan, const DpgLaunch* Lin, cu
     base = g_noalloc_ptr[dev];
   }
   const size_t fit = plan->scratch_per_cta > 0 ? DPG_NOALLOC_SCRATCH_DOUBLES / plan->scratch_per_cta : (size_t)Lin->C;
-  int grid = std::min(Lin->C, dpg::num_sms());
+  int grid = std::min(Lin->C, dpg::num_sms() * kc.per_sm);
   grid = (int)std::min<size_t>((size_t)grid, fit);
   DpgLaunch L = *Lin;
   L.scratch = base;
   size_t bytes = (size_t)plan->sm_total * sizeof(double);
-  k<<<grid, NT, bytes, stream>>>(*plan, L);
+  k<<<grid, kc.threads, bytes, stream>>>(*plan, L);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
   return DPG_OK;

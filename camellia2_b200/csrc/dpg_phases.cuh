@@ -20,7 +20,16 @@ extern __shared__ __align__(128) double dpg_smem[];
 
 namespace {
 
-constexpr int NT = DPG_NTHREADS;
+// Warps per CTA and CTAs per SM of this translation unit: 16 and one, or (DPG_CTA_WARPS defined) the
+// small buckets' 8 and two.
+#ifndef DPG_CTA_WARPS
+#define DPG_CTA_WARPS DPG_NWARPS
+#endif
+constexpr int NW = DPG_CTA_WARPS;
+constexpr int NT = NW * 32;
+constexpr int CTAS_PER_SM = DPG_NWARPS / NW;
+constexpr int MAX_MBT = NW == DPG_NWARPS ? DPG_MAX_MBT : NW;  // trial tiles: one column tile per warp
+constexpr int MAX_KT = (MAX_MBT * (MAX_MBT + 1) / 2 + NW - 1) / NW;  // lower K_ext tiles per warp
 constexpr int MBAR_SPIN_LIMIT = 1 << 22;
 constexpr int ERR_TIMEOUT_FLAG = 0x7fff0000;
 constexpr int GEO = 24;  // doubles per point geometry record: J(9) Ji(9) det w*|J| n(3) 1/det
@@ -325,7 +334,7 @@ __device__ __forceinline__ void factor_diag(const double* __restrict__ T, int k,
 // next door.  That chain of diagonal tiles is what bounds the factorisation: warp 0 does
 // nothing else, with its sub-partition to itself (warps 4, 8, 12 only keep the barriers), and it
 // needs from the others only the sum over j < k of tile (k+1, k+1), formed a step ahead.
-constexpr int CHOL_NW = DPG_NWARPS - DPG_NWARPS / 4;  // warps that update: those of the other sub-partitions
+constexpr int CHOL_NW = NW - NW / 4;  // warps that update: those of the other sub-partitions
 
 __device__ __forceinline__ int chol_rank(int warp) { return warp - (warp >> 2) - 1; }
 
@@ -432,7 +441,7 @@ __device__ __noinline__ void tile_cholesky(int T_off, int nb, int nsteps, int fl
   // the trailing block
   const int m = nb - nsteps, ntr = m * (m + 1) / 2;
 #pragma unroll 1
-  for (int u = warp; u < ntr; u += DPG_NWARPS) chol_tile(T, nsteps + (tri[u] & 255), nsteps + (tri[u] >> 8), nsteps, lane);
+  for (int u = warp; u < ntr; u += NW) chol_tile(T, nsteps + (tri[u] & 255), nsteps + (tri[u] >> 8), nsteps, lane);
   __syncthreads();
 }
 
@@ -506,7 +515,7 @@ __device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, in
     const DpgSeg& S = P.seg[sgi];
     if (S.nterm == 0) continue;
     // this warp's active 16x8 blocks of the segment: operand offsets and accumulators
-    const int bbase = S.ntile / DPG_NWARPS, bextra = S.ntile % DPG_NWARPS;
+    const int bbase = S.ntile / NW, bextra = S.ntile % NW;
     const int my0 = S.tile0 + warp * bbase + min(warp, bextra);
     const int nmine = bbase + (warp < bextra ? 1 : 0);
     uint32_t pk[BTW];
@@ -632,7 +641,7 @@ __device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, in
   __syncthreads();
   double* Bc = L.B ? L.B + (size_t)cell * P.M * P.N : nullptr;
   double* Fc = L.F ? L.F + (size_t)cell * P.N : nullptr;
-  for (int tile = warp; tile < P.MBT * P.NBT; tile += DPG_NWARPS) {
+  for (int tile = warp; tile < P.MBT * P.NBT; tile += NW) {
     const int J = tile / P.NBT, I = tile - J * P.NBT;
     const double2 v = scr[tile * 32 + lane];
     const int ur = P.dev2user_test[I * 8 + g];
@@ -728,9 +737,13 @@ enum { GP_CHG, GP_QG, GP_RING, GP_STAGE, GP_STAGES, GP_FLUSH, GP_D, GP_NGB, GP_T
 // hex workload.)  The chunks travel through a ring of stages: warps arrive on a stage's empty
 // mbarrier and warp 0 refills it while the next chunk is worked on, so no block barrier is left in
 // the loop and the warps drift apart by up to a ring.  Every GP_FLUSH chunks (except after the last)
-// each thread adds the accumulators of its flushed blocks (P.gflushbits) into its own running sums
+// each thread adds the accumulators of its flushed blocks (P.gflushmask) into its own running sums
 // in the scratch slot ([block][lane][4]; plain L2 loads and stores, one writer per element, so the
 // order of additions is fixed) and restarts them from zero.
+__device__ __forceinline__ uint32_t gram_flush_bits(const DpgPlanDev& P, int tau0) {
+  return __funnelshift_r(P.gflushmask[tau0 >> 5], P.gflushmask[(tau0 >> 5) + 1], tau0 & 31);
+}
+
 template <int GTM, int DIM>
 __device__ __forceinline__ void gram_body(const DpgPlanDev& P, const DpgLaunch& L, int sm_nodes) {
   const volatile int* const gp = reinterpret_cast<const volatile int*>(dpg_smem + sm_nodes + DPG_SM_GRAM);
@@ -742,8 +755,8 @@ __device__ __forceinline__ void gram_body(const DpgPlanDev& P, const DpgLaunch& 
   int ntw, tau0;
   {
     const int ngb = gp[GP_NGB], warp = threadIdx.x >> 5;
-    ntw = ngb / DPG_NWARPS + (warp < ngb % DPG_NWARPS ? 1 : 0);
-    tau0 = warp * (ngb / DPG_NWARPS) + min(warp, ngb % DPG_NWARPS);
+    ntw = ngb / NW + (warp < ngb % NW ? 1 : 0);
+    tau0 = warp * (ngb / NW) + min(warp, ngb % NW);
   }
   const int4* const tdesc = reinterpret_cast<const int4*>(dpg_smem + gp[GP_TILES]) + tau0;
   const int fs = gp[GP_FS], dstride = gp[GP_DS];
@@ -798,7 +811,7 @@ __device__ __forceinline__ void gram_body(const DpgPlanDev& P, const DpgLaunch& 
     }
     if ((c + 1) % gflush == 0 && (c + 1) * chg < gp[GP_QG]) {
       const bool first = (c + 1) == gflush;
-      const uint32_t fb = P.gflushbits[threadIdx.x >> 5];
+      const uint32_t fb = gram_flush_bits(P, tau0);
       double* const gsum = L.scratch + (size_t)blockIdx.x * P.scratch_per_cta + P.gsum_off + tau0 * 128 + (threadIdx.x & 31) * 4;
 #pragma unroll
       for (int u = 0; u < GTM; u++) {
@@ -829,7 +842,7 @@ __device__ __forceinline__ void gram_body(const DpgPlanDev& P, const DpgLaunch& 
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   double* const GT = dpg_smem + gp[GP_GT];
   const bool join = gp[GP_FLUSH] * gp[GP_CHG] < gp[GP_QG];  // the last group joins the running sums
-  const uint32_t fb = P.gflushbits[threadIdx.x >> 5];
+  const uint32_t fb = gram_flush_bits(P, tau0);
   const double* const gsum = L.scratch + (size_t)blockIdx.x * P.scratch_per_cta + P.gsum_off + tau0 * 128 + lane * 4;
 #pragma unroll
   for (int u = 0; u < GTM; u++) {
@@ -950,7 +963,7 @@ __device__ __forceinline__ void phase_factor(const DpgPlanDev& P) {
     scale[r] = (dg > 0.0) ? rsqrt(dg) : 1.0;
   }
   __syncthreads();
-  for (int u = warp; u < P.ngt; u += DPG_NWARPS) {
+  for (int u = warp; u < P.ngt; u += NW) {
     int ij = tri_s[u];
     int I = ij & 255, J = ij >> 8;
     double2* p = reinterpret_cast<double2*>(GT + u * 64 + ak_cfrag(g, t));
@@ -1094,13 +1107,13 @@ __device__ __forceinline__ void phase_syrk_out(const DpgPlanDev& P, const DpgLau
   double* KT = sm + P.sm_k;
   {
     const int nk = P.MBT * (P.MBT + 1) / 2;
-    const int kbase = nk / DPG_NWARPS, kextra = nk % DPG_NWARPS;
+    const int kbase = nk / NW, kextra = nk % NW;
     const int k0 = warp * kbase + min(warp, kextra);
     const int nkw = kbase + (warp < kextra ? 1 : 0);
-    double2 kacc[DPG_MAX_KT];
-    int kI[DPG_MAX_KT], kJ[DPG_MAX_KT];
+    double2 kacc[MAX_KT];
+    int kI[MAX_KT], kJ[MAX_KT];
 #pragma unroll
-    for (int u = 0; u < DPG_MAX_KT; u++) {
+    for (int u = 0; u < MAX_KT; u++) {
       kacc[u] = make_double2(0.0, 0.0);
       int ij = (u < nkw) ? tri_s[k0 + u] : 0;
       kI[u] = ij & 255;
@@ -1112,7 +1125,7 @@ __device__ __forceinline__ void phase_syrk_out(const DpgPlanDev& P, const DpgLau
         int lastI = -1;
         double afr = 0.0;
 #pragma unroll
-        for (int u = 0; u < DPG_MAX_KT; u++) {
+        for (int u = 0; u < MAX_KT; u++) {
           if (u < nkw) {
             if (kI[u] != lastI) { afr = WT[(kI[u] * P.NBT + R) * 64 + h * 32 + lane]; lastI = kI[u]; }
             double bfr = WT[(kJ[u] * P.NBT + R) * 64 + h * 32 + lane];
@@ -1123,7 +1136,7 @@ __device__ __forceinline__ void phase_syrk_out(const DpgPlanDev& P, const DpgLau
     }
     __syncthreads();
 #pragma unroll
-    for (int u = 0; u < DPG_MAX_KT; u++)
+    for (int u = 0; u < MAX_KT; u++)
       if (u < nkw) *reinterpret_cast<double2*>(KT + (k0 + u) * 64 + ak_cfrag(g, t)) = kacc[u];
     __syncthreads();
   }
@@ -1131,7 +1144,7 @@ __device__ __forceinline__ void phase_syrk_out(const DpgPlanDev& P, const DpgLau
   // streaming stores, so the outputs do not evict the CTA's scratch slot from L2
   if (L.K) {
     double* Kc = L.K + (size_t)cell * P.M * P.M;
-    for (int i = warp; i < P.M; i += DPG_NWARPS) {
+    for (int i = warp; i < P.M; i += NW) {
       const int di = i < P.nf ? i : P.nfp + (i - P.nf);
       for (int j = lane; j < P.M; j += 32) {
         const int dj = j < P.nf ? j : P.nfp + (j - P.nf);
@@ -1155,7 +1168,7 @@ __device__ __forceinline__ void phase_syrk_out(const DpgPlanDev& P, const DpgLau
       tile_cholesky(P.sm_k, P.MBT, P.nfb, 2 * (P.sm_nodes + 24) + 1, -1, P.sm_nodes + 32, P.sm_linv);
     }
     double* Sc = L.S + (size_t)cell * P.nt * P.nt;
-    for (int i = warp; i < P.nt; i += DPG_NWARPS)
+    for (int i = warp; i < P.nt; i += NW)
       for (int j = lane; j < P.nt; j += 32) __stcs(&Sc[(size_t)i * P.nt + j], sym_get(KT, P.nfp + i, P.nfp + j));
     double* sc = L.s + (size_t)cell * P.nt;
     for (int i = tid; i < P.nt; i += NT) __stcs(&sc[i], sym_get(KT, P.fcol, P.nfp + i));
@@ -1188,7 +1201,7 @@ __device__ __forceinline__ void cta_setup(const DpgPlanDev& P) {
   }
   for (int u = tid; u < P.ngb && P.gtiles; u += NT) tiles_s[u] = P.gtiles[u];
   if (tid == 0) {
-    for (int i = 0; i < DPG_NBARS; i++) mbar_init(&mbar_s[i], i < DPG_BAR_EMPTY ? 1 : DPG_NWARPS);
+    for (int i = 0; i < DPG_NBARS; i++) mbar_init(&mbar_s[i], i < DPG_BAR_EMPTY ? 1 : NW);
     int* const gp = reinterpret_cast<int*>(sm + P.sm_nodes + DPG_SM_GRAM);
     reinterpret_cast<int*>(sm + P.sm_nodes + 24)[3] = 0;
     gp[GP_CHG] = P.chg; gp[GP_QG] = P.QG; gp[GP_RING] = P.g_fref; gp[GP_STAGE] = P.gstage; gp[GP_STAGES] = P.gstages;
@@ -1199,6 +1212,6 @@ __device__ __forceinline__ void cta_setup(const DpgPlanDev& P) {
   __syncthreads();
 }
 
-typedef void (*KernelFn)(const DpgPlanDev, const DpgLaunch);
+typedef DpgKernelFn KernelFn;
 
 }  // namespace

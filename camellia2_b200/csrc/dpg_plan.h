@@ -29,7 +29,9 @@
 #define DPG_MAX_BLK 24    // active (test var, trial column tile) blocks per segment
 #define DPG_MAX_PAIRS 36  // test var pairs a >= b
 #define DPG_NWARPS 16
-#define DPG_NTHREADS (DPG_NWARPS * 32)
+#define DPG_SMEM 232448   // shared memory of one CTA
+#define DPG_SMALL_WARPS 8 // warps per CTA of the small buckets, two CTAs per SM
+#define DPG_SMALL_SMEM 115712  // shared memory of one of two CTAs (228 KB per SM, 1 KB reserved for each)
 #define DPG_CHG 8         // Gram quadrature points per staged chunk (4 when shared memory is short)
 #define DPG_GSTAGES 4     // most stages of the Gram chunk ring
 #define DPG_BAR_B DPG_GSTAGES            // mbarriers: Gram stages full, the two B-phase buffers,
@@ -45,7 +47,6 @@
 #define DPG_MAX_NBT 24    // max test tiles (N <= 192)
 #define DPG_MAX_MBT 16    // max trial tiles incl. the F tile (one column tile per warp)
 #define DPG_MAX_GT 12     // max 16x8 G blocks per warp
-#define DPG_MAX_KT 9      // max lower K_ext tiles per warp: ceil(16*17/2 / 16)
 #define DPG_ULD 12        // leading dim of a staged 8-column U block (conflict-free B-fragments)
 
 struct DpgIPEnt {
@@ -208,9 +209,9 @@ struct DpgPlanDev {
   size_t gsum_off;                                 // [ngb][32 lanes][4] Gram partial sums
   int gflush;                                      // staged Gram chunks between two flushes of the
                                                    // accumulators into the running sums (0: none)
-  uint32_t gflushbits[DPG_NWARPS];                 // per warp: its blocks (bit u = its u-th) that
-                                                   // take part in the flushes (var pairs that two
-                                                   // or more graph-norm terms couple)
+  uint32_t gflushmask[DPG_MAX_GT * DPG_NWARPS / 32 + 1];  // bit b: block b takes part in the flushes (var
+                                                   // pairs that two or more graph-norm terms couple)
+  int small;                // two CTAs of DPG_SMALL_WARPS warps per SM (layout within DPG_SMALL_SMEM)
   // Large buckets (N > 192 or M > 120 after padding) run on dpg_big_kernel: per cell the
   // lower triangle of Z = [[G, E], [E^T, 0]] (E = [B^T | F]; rows/columns: device test rows,
   // then device trial columns) in a per-CTA global workspace.

@@ -31,7 +31,7 @@ __device__ __forceinline__ void queue_leave(int* counters) {
 // first and the short ones fill the tail.  Switching buckets rebuilds the CTA's tables and
 // mbarriers.  claim_slot: a shared-memory double beyond every plan's layout.
 template <int NBTM, int GTM, int BTW>
-__global__ void __launch_bounds__(NT, 1) dpg_queue_kernel(const DpgPlanDev* __restrict__ plans,
+__global__ void __launch_bounds__(NT, CTAS_PER_SM) dpg_queue_kernel(const DpgPlanDev* __restrict__ plans,
                                                           const DpgLaunch* __restrict__ launches,
                                                           const int* __restrict__ cstart, int nb,
                                                           int* __restrict__ counters, int claim, int claim_slot) {
@@ -101,8 +101,8 @@ static QueueFn pick_queue_kernel(const DpgPlanDev* plans, int nb) {
   for (int b = 0; b < nb; b++) {
     const DpgPlanDev* p = &plans[b];
     nbt = std::max(nbt, p->NBT);
-    per = std::max(per, (p->ngb + DPG_NWARPS - 1) / DPG_NWARPS);
-    for (int s = 0; s < p->nseg; s++) btw = std::max(btw, (p->seg[s].ntile + DPG_NWARPS - 1) / DPG_NWARPS);
+    per = std::max(per, (p->ngb + NW - 1) / NW);
+    for (int s = 0; s < p->nseg; s++) btw = std::max(btw, (p->seg[s].ntile + NW - 1) / NW);
   }
 #define DPG_PICK(NB, GT, BT) \
   if (nbt <= NB && per <= GT && btw <= BT) return dpg_queue_kernel<NB, GT, BT>;
