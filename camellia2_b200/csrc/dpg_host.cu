@@ -1491,7 +1491,13 @@ int dpg_host_pipeline(const DpgPlanDev* plan, const DpgPlanDev* d_plan, void** d
   const size_t nb_K = wantK ? (size_t)g.M * g.M * 8 : 0, nb_l = wantK ? (size_t)g.M * 8 : 0;
   const size_t nb_S = wantS ? (size_t)g.nt * g.nt * 8 : 0, nb_s = wantS ? (size_t)g.nt * 8 : 0;
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const int chunk = std::min(C, 4096);
+  // cells per chunk: whole waves of the kernel, about 64 MB of outputs.  The copies out are the slower
+  // side, so what counts is how soon the first one starts (4096-cell chunks kept it waiting for 6 ms
+  // of kernel on the 3D hex bucket).
+  const size_t cell_out = nb_K + nb_l + nb_S + nb_s + 4;
+  const size_t wave = 2 * (size_t)dpg::num_sms();
+  const size_t want = std::min<size_t>(4096, ((64u << 20) / cell_out + wave - 1) / wave * wave);
+  const int chunk = (int)std::min<size_t>(C, std::max<size_t>(want, g.big ? wave / 2 : wave));
   const size_t per_buf = al(chunk * nb_nodes) + al(chunk * nb_par) + al(chunk * nb_co) + al(chunk * nb_K) +
                          al(chunk * nb_l) + al(chunk * nb_S) + al(chunk * nb_s) + al(chunk * 4);
   if (*ws_bytes < 2 * per_buf) {

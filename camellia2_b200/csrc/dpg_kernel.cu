@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(RF_MAXW * 32) recover_fields_warp_kernel(int C
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   constexpr int ld = 33;                // odd row stride: conflict-free column reads
-  double* st = rs + (size_t)warp * (32 * ld + M);
+  double* st = rs + (size_t)warp * (32 * ld + M + 72);
   double* ts = st + 32 * ld;            // trace values
   const int nt = M - nf;
   for (int cell = blockIdx.x * nwarps + warp; cell < C; cell += gridDim.x * nwarps) {
@@ -295,17 +295,23 @@ __global__ void __launch_bounds__(RF_MAXW * 32) recover_fields_warp_kernel(int C
       sc = d > 0.0 ? rsqrt(d) : 1.0;
     }
     // rows and columns nf..31 are padded with the identity, so every step below runs
-    // unguarded on all 32 lanes and leaves the padding unchanged
+    // unguarded on all 32 lanes and leaves the padding unchanged.  Values that every lane needs
+    // go through shared memory two at a time (a 64-bit shuffle is two instructions on a unit the
+    // four sub-partitions share; the 1,400 of the shuffled form bound the kernel).
+    double* const bc = ts + ((nt + 1) & ~1);  // two rows of 34: column k of L, then z_k
+    bc[lane] = sc;
+    __syncwarp();
     double a[32];
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
-      const double sj = __shfl_sync(FULL, sc, j);
-      a[j] = (i < nf && j < nf) ? sc * st[i * ld + j] * sj : (i == j ? 1.0 : 0.0);
+    for (int j = 0; j < 32; j += 2) {
+      const double2 s2 = *reinterpret_cast<const double2*>(bc + j);
+      a[j] = (i < nf && j < nf) ? sc * st[i * ld + j] * s2.x : (i == j ? 1.0 : 0.0);
+      a[j + 1] = (i < nf && j + 1 < nf) ? sc * st[i * ld + j + 1] * s2.y : (i == j + 1 ? 1.0 : 0.0);
     }
     __syncwarp();
     bi = i < nf ? bi * sc : 0.0;
-    // right-looking Cholesky: at step k lane k holds the pivot, lanes i > k column k;
-    // entries above the diagonal are left unused
+    // right-looking Cholesky with L z = b beside it: at step k lane k holds the pivot, lanes i > k
+    // column k; entries above the diagonal are left unused
     int fail = 0;
     double dinv = 0.0;  // 1 / L_ii
 #pragma unroll
@@ -315,16 +321,23 @@ __global__ void __launch_bounds__(RF_MAXW * 32) recover_fields_warp_kernel(int C
       const double inv = rsqrt(piv);
       const double lik = (i == k) ? piv * inv : a[k] * inv;
       a[k] = lik;
-      if (i == k) dinv = inv;
+      double* const bk = bc + (k & 1) * 34;
+      bk[lane] = lik;
+      if (i == k) {
+        dinv = inv;
+        bi = bi * inv;
+        bk[32] = bi;
+      }
+      __syncwarp();
+      const double zk = bk[32];
+      if (i > k) bi -= lik * zk;
+      if ((k & 1) == 0) a[k + 1] -= lik * bk[k + 1];
 #pragma unroll
-      for (int j = k + 1; j < 32; j++) a[j] -= lik * __shfl_sync(FULL, lik, j);
-    }
-    // L z = b
-#pragma unroll
-    for (int k = 0; k < 32; k++) {
-      const double zk = __shfl_sync(FULL, bi * dinv, k);
-      if (i == k) bi = zk;
-      else if (i > k) bi -= a[k] * zk;
+      for (int j = (k + 2) & ~1; j < 32; j += 2) {
+        const double2 l2 = *reinterpret_cast<const double2*>(bk + j);
+        a[j] -= lik * l2.x;
+        a[j + 1] -= lik * l2.y;
+      }
     }
     // L^T y = z, column by column: L's rows go back to the (now free) shared tile, y_k is
     // broadcast and lanes j < k take L_kj y_k off their z_j
@@ -350,7 +363,7 @@ __global__ void __launch_bounds__(RF_MAXW * 32) recover_fields_warp_kernel(int C
 int dpg_launch_recover_fields(int C, int M, int nf, const double* K, const double* l, const double* t, double* u,
                               int32_t* info, cudaStream_t stream) {
   if (C <= 0) return DPG_OK;
-  const size_t per_warp = ((size_t)32 * 33 + M) * sizeof(double);
+  const size_t per_warp = ((size_t)32 * 33 + M + 72) * sizeof(double);
   if (nf <= 32 && per_warp <= 100 * 1024) {
     // one-warp blocks: as many resident per SM as the staging tiles allow
     static int wconfigured = 0;
