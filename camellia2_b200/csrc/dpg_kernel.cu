@@ -229,49 +229,59 @@ __global__ void __launch_bounds__(256) recover_fields_kernel(int C, int M, int n
   }
 }
 
-// nf <= 32: one warp per cell.  K_ff goes to a per-warp shared tile by 8-byte
-// asynchronous copies (all in flight at once); K_ft t is formed from coalesced reads of
-// the K_ft rows, each lane holding partial sums of all rows, which one butterfly
-// reduce-scatter (31 shuffles) turns into lane i's row sum.  Lane i then holds row i of
-// the equilibrated K_ff in registers and the Cholesky factorisation, both triangular
-// solves and the unscaling run on shuffles, without a block barrier.  Same results and
-// info as the block kernel above.
-constexpr int RF_MAXW = 1;  // warps per block
+// nf <= 32: one warp per cell, no block barrier.  The lower 8x8 tiles of K_ff go to shared memory by
+// 8-byte asynchronous copies, K_ft t is formed meanwhile from coalesced reads of the K_ft rows, each
+// lane holding partial sums of all rows, which one butterfly reduce-scatter (31 shuffles) turns into
+// lane i's row sum.  K_ff is then equilibrated and factored as tiles like G (factor_diag, panels and
+// updates by m8n8k4), four diagonal tiles of ~1 K cycles: a row per lane in registers takes 32 steps of
+// pivot, reciprocal square root, broadcast and update (200-300 cycles each), and the kernel is bound by
+// that chain.  The two solves multiply by the inverse diagonal tiles.  Same info as the block kernel.
+// 64,000 hex cells (nf 32, M 110; HBM floor 0.29 ms): 0.96 ms with rows in registers and shuffles, 0.68 ms now;
+// 20 warps per SM at 96 registers spill: 0.71 ms
+constexpr int RF_TILES = 10;  // lower tiles of a 32 x 32 matrix
+constexpr int RF_SM = RF_TILES * 64 + 4 * 64 + 3 * 32 + 2;  // tiles, inverses, scales, two vectors, flag (then t)
 
-__global__ void __launch_bounds__(RF_MAXW * 32) recover_fields_warp_kernel(int C, int M, int nf,
-                                                                         const double* __restrict__ K,
-                                                                         const double* __restrict__ l,
-                                                                         const double* __restrict__ t_in,
-                                                                         double* __restrict__ u,
-                                                                         int32_t* __restrict__ info) {
-  extern __shared__ double rs[];
+__global__ void __launch_bounds__(32) recover_fields_warp_kernel(int C, int M, int nf, const double* __restrict__ K,
+                                                                 const double* __restrict__ l,
+                                                                 const double* __restrict__ t_in,
+                                                                 double* __restrict__ u, int32_t* __restrict__ info) {
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  constexpr int ld = 33;                // odd row stride: conflict-free column reads
-  double* st = rs + (size_t)warp * (32 * ld + M + 72);
-  double* ts = st + 32 * ld;            // trace values
-  const int nt = M - nf;
-  for (int cell = blockIdx.x * nwarps + warp; cell < C; cell += gridDim.x * nwarps) {
+  const int lane = threadIdx.x, i = lane, g = lane >> 2, t = lane & 3;
+  double* const T = dpg_smem;
+  double* const linv = T + RF_TILES * 64;
+  double* const scl = linv + 4 * 64;
+  double* const vb = scl + 32;
+  double* const vz = vb + 32;
+  int* const flag = reinterpret_cast<int*>(vz + 32);
+  double* const ts = vz + 34;
+  const int nt = M - nf, nb = (nf + 7) >> 3;
+  for (int cell = blockIdx.x; cell < C; cell += gridDim.x) {
     const double* Kc = K + (size_t)cell * M * M;
     const double* tc = t_in + (size_t)cell * nt;
-    for (int r = 0; r < nf; r++)
-      if (lane < nf)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(st + r * ld + lane)),
-                     "l"(Kc + (size_t)r * M + lane)
-                     : "memory");
+    if (lane == 0) *flag = 0;
+    for (int r = 0; r < nb * 8; r++) {
+      const int I = r >> 3;
+      if ((lane >> 3) <= I) {
+        double* dst = T + (I * (I + 1) / 2 + (lane >> 3)) * 64 + ak(r & 7, lane & 7);
+        if (r < nf && lane < nf)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(Kc + (size_t)r * M + lane)
+                       : "memory");
+        else *dst = r == lane ? 1.0 : 0.0;
+      }
+    }
     for (int j = lane; j < nt; j += 32)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(ts + j)), "l"(tc + j) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
     // partial sums of K_ft(i,:) t over this lane's columns, all rows
     double p[32];
 #pragma unroll
-    for (int i = 0; i < 32; i++) p[i] = 0.0;
+    for (int r = 0; r < 32; r++) p[r] = 0.0;
     for (int c0 = 0; c0 < nt; c0 += 32) {
       const int c = c0 + lane;
       const double tv = c < nt ? tc[c] : 0.0;
 #pragma unroll
-      for (int i = 0; i < 32; i++)
-        if (i < nf && c < nt) p[i] += Kc[(size_t)i * M + nf + c] * tv;
+      for (int r = 0; r < 32; r++)
+        if (r < nf && c < nt) p[r] += Kc[(size_t)r * M + nf + c] * tv;
     }
     // reduce-scatter: after the step with offset o a lane keeps the rows whose bit o
     // matches its own; at the end lane i holds row i's sum in p[0]
@@ -285,77 +295,88 @@ __global__ void __launch_bounds__(RF_MAXW * 32) recover_fields_warp_kernel(int C
         p[r] = keep + __shfl_xor_sync(FULL, send, o);
       }
     }
+    const double li = i < nf ? l[(size_t)cell * M + i] : 0.0;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();
-    const int i = lane;
-    double bi = 0.0, sc = 1.0;  // lane i: l_i - K_ft(i,:) t and s_i = K_ii^-1/2
+    // equilibrate (rows and columns nf .. are padded with the identity)
+    double sc = 1.0;
     if (i < nf) {
-      bi = l[(size_t)cell * M + i] - p[0];
-      const double d = st[i * ld + i];
-      sc = d > 0.0 ? rsqrt(d) : 1.0;
+      const double d = T[((i >> 3) * ((i >> 3) + 1) / 2 + (i >> 3)) * 64 + ak(i & 7, i & 7)];
+      if (d > 0.0) sc = rsqrt(d);
     }
-    // rows and columns nf..31 are padded with the identity, so every step below runs
-    // unguarded on all 32 lanes and leaves the padding unchanged.  Values that every lane needs
-    // go through shared memory two at a time (a 64-bit shuffle is two instructions on a unit the
-    // four sub-partitions share; the 1,400 of the shuffled form bound the kernel).
-    double* const bc = ts + ((nt + 1) & ~1);  // two rows of 34: column k of L, then z_k
-    bc[lane] = sc;
+    scl[i] = sc;
+    vb[i] = i < nf ? (li - p[0]) * sc : 0.0;
     __syncwarp();
-    double a[32];
-#pragma unroll
-    for (int j = 0; j < 32; j += 2) {
-      const double2 s2 = *reinterpret_cast<const double2*>(bc + j);
-      a[j] = (i < nf && j < nf) ? sc * st[i * ld + j] * s2.x : (i == j ? 1.0 : 0.0);
-      a[j + 1] = (i < nf && j + 1 < nf) ? sc * st[i * ld + j + 1] * s2.y : (i == j + 1 ? 1.0 : 0.0);
-    }
+    for (int I = 0, tau = 0; I < nb; I++)
+      for (int J = 0; J <= I; J++, tau++) {
+        double2* q = reinterpret_cast<double2*>(T + tau * 64 + ak_cfrag(g, t));
+        double2 v = *q;
+        const double si = scl[I * 8 + g];
+        v.x *= si * scl[J * 8 + 2 * t];
+        v.y *= si * scl[J * 8 + 2 * t + 1];
+        *q = v;
+      }
     __syncwarp();
-    bi = i < nf ? bi * sc : 0.0;
-    // right-looking Cholesky with L z = b beside it: at step k lane k holds the pivot, lanes i > k
-    // column k; entries above the diagonal are left unused
-    int fail = 0;
-    double dinv = 0.0;  // 1 / L_ii
-#pragma unroll
-    for (int k = 0; k < 32; k++) {
-      const double piv = __shfl_sync(FULL, a[k], k);
-      if (!(piv > 0.0) && fail == 0) fail = k + 1;
-      const double inv = rsqrt(piv);
-      const double lik = (i == k) ? piv * inv : a[k] * inv;
-      a[k] = lik;
-      double* const bk = bc + (k & 1) * 34;
-      bk[lane] = lik;
-      if (i == k) {
-        dinv = inv;
-        bi = bi * inv;
-        bk[32] = bi;
+    for (int k = 0; k < nb; k++) {
+      factor_diag(T, k, flag, 1, linv);
+      const double* Li = linv + k * 64;
+      for (int I = k + 1; I < nb; I++) {  // panel
+        double* Tik = T + (I * (I + 1) / 2 + k) * 64;
+        const double a0 = Tik[lane], a1 = Tik[32 + lane];
+        double2 c = make_double2(0.0, 0.0);
+        dmma(c, a0, Li[lane]);
+        dmma(c, a1, Li[32 + lane]);
+        __syncwarp();
+        *reinterpret_cast<double2*>(Tik + ak_cfrag(g, t)) = c;
       }
       __syncwarp();
-      const double zk = bk[32];
-      if (i > k) bi -= lik * zk;
-      if ((k & 1) == 0) a[k + 1] -= lik * bk[k + 1];
+      for (int I = k + 1; I < nb; I++)  // trailing update
+        for (int J = k + 1; J <= I; J++) {
+          const double* Lik = T + (I * (I + 1) / 2 + k) * 64;
+          const double* Ljk = T + (J * (J + 1) / 2 + k) * 64;
+          double2* q = reinterpret_cast<double2*>(T + (I * (I + 1) / 2 + J) * 64 + ak_cfrag(g, t));
+          double2 c = *q;
+          dmma(c, -Lik[lane], Ljk[lane]);
+          dmma(c, -Lik[32 + lane], Ljk[32 + lane]);
+          *q = c;
+        }
+      // z_k = L_kk^-1 b_k (four lanes per row), then b_I -= L_Ik z_k, a lane per row
+      double z = Li[ak(g, t)] * vb[k * 8 + t] + Li[ak(g, t + 4)] * vb[k * 8 + t + 4];
+      z += __shfl_xor_sync(FULL, z, 1);
+      z += __shfl_xor_sync(FULL, z, 2);
+      if (t == 0) vz[k * 8 + g] = z;
+      __syncwarp();
+      if ((i >> 3) > k && (i >> 3) < nb) {
+        const double* Lik = T + ((i >> 3) * ((i >> 3) + 1) / 2 + k) * 64;
+        double b = vb[i];
 #pragma unroll
-      for (int j = (k + 2) & ~1; j < 32; j += 2) {
-        const double2 l2 = *reinterpret_cast<const double2*>(bk + j);
-        a[j] -= lik * l2.x;
-        a[j + 1] -= lik * l2.y;
+        for (int m = 0; m < 8; m++) b -= Lik[ak(i & 7, m)] * vz[k * 8 + m];
+        vb[i] = b;
       }
+      __syncwarp();
     }
-    // L^T y = z, column by column: L's rows go back to the (now free) shared tile, y_k is
-    // broadcast and lanes j < k take L_kj y_k off their z_j
+    // y_k = L_kk^-T z_k, then z_J -= L_kJ^T y_k for J < k
+    for (int k = nb - 1; k >= 0; k--) {
+      const double* Li = linv + k * 64;
+      double y = Li[ak(t, g)] * vz[k * 8 + t] + Li[ak(t + 4, g)] * vz[k * 8 + t + 4];
+      y += __shfl_xor_sync(FULL, y, 1);
+      y += __shfl_xor_sync(FULL, y, 2);
+      if (t == 0) vb[k * 8 + g] = y;
+      __syncwarp();
+      if ((i >> 3) < k) {
+        const double* Lk = T + (k * (k + 1) / 2 + (i >> 3)) * 64;
+        double z = vz[i];
 #pragma unroll
-    for (int j = 0; j < 32; j++)
-      if (i < nf && j <= i) st[i * ld + j] = a[j];
-    __syncwarp();
-    double y = bi;
-    for (int k = nf - 1; k >= 0; k--) {
-      const double yk = __shfl_sync(FULL, y * dinv, k);
-      if (i == k) y = yk;
-      else if (i < k) y -= st[k * ld + i] * yk;
+        for (int m = 0; m < 8; m++) z -= Lk[ak(m, i & 7)] * vb[k * 8 + m];
+        vz[i] = z;
+      }
+      __syncwarp();
     }
-    __syncwarp();
     double* uc = u + (size_t)cell * M;
-    if (i < nf) uc[i] = sc * y;
-    for (int j = lane; j < nt; j += 32) uc[nf + j] = tc[j];
-    if (lane == 0 && info) info[cell] = fail;
+    if (i < nf) uc[i] = sc * vb[i];
+    for (int j = lane; j < nt; j += 32) uc[nf + j] = ts[j];
+    if (lane == 0 && info) info[cell] = *flag;
+    __syncwarp();
   }
 }
 }  // namespace
@@ -363,7 +384,7 @@ __global__ void __launch_bounds__(RF_MAXW * 32) recover_fields_warp_kernel(int C
 int dpg_launch_recover_fields(int C, int M, int nf, const double* K, const double* l, const double* t, double* u,
                               int32_t* info, cudaStream_t stream) {
   if (C <= 0) return DPG_OK;
-  const size_t per_warp = ((size_t)32 * 33 + M + 72) * sizeof(double);
+  const size_t per_warp = ((size_t)RF_SM + M) * sizeof(double);
   if (nf <= 32 && per_warp <= 100 * 1024) {
     // one-warp blocks: as many resident per SM as the staging tiles allow
     static int wconfigured = 0;
