@@ -14,18 +14,65 @@ int dpg_configure_big(const DpgPlanDev* plan) {
   // every large plan shares the kernel: opt in to the device maximum so that configuring one
   // plan never lowers the limit another plan needs
   if (optin > 0) bytes = (size_t)optin;
-  for (KernelFn k : {dpg_big_kernel<16>, dpg_big_kernel<32>}) {
+  for (KernelFn k : {dpg_big_kernel<16, false>, dpg_big_kernel<32, false>, dpg_big_kernel<16, true>, dpg_big_kernel<32, true>}) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
   }
   return DPG_OK;
 }
 
-// Large buckets: one CTA per SM, each with its own workspace (Z and the per-point factors).
+static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int grid, int size, size_t smem,
+                           cudaStream_t stream) {
+  std::memset(&cfg, 0, sizeof(cfg));
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+}
+
+// CTAs per cell of a call of C cells, and the clusters that run at once.  With at most half as many
+// cells as SMs the others would idle, so a cluster shares each cell: the size with the least waves x
+// (serial tenth + rest / size), at most half the cell's 64-row blocks (a step's panels and trailing tiles
+// are what is dealt out).  37 Stokes quads of p = 6: 4.98 ms with a CTA per cell, 1.96 ms so.  With more cells than that one CTA per cell is faster: a cluster
+// reloads a step's panels in every CTA and waits at two cluster barriers per step.
+static int team_size(const DpgPlanDev* plan, int C, KernelFn k, int* clusters) {
+  const int sms = dpg::num_sms();
+  *clusters = std::min(C, sms);
+  int best = 1;
+  double cost = 1.0;
+  if (2 * C > sms) return best;
+  for (int size = 2; size <= 8 && size <= (plan->Zn + 127) / 128; size++) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    cluster_config(cfg, attr, size, size, (size_t)plan->bs_total * sizeof(double), nullptr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      break;
+    }
+    const double c = ((C + n - 1) / n) * (0.1 + 0.9 / size);
+    if (c < cost) {
+      cost = c;
+      best = size;
+      *clusters = std::min(C, n);
+    }
+  }
+  return best;
+}
+
+// Large buckets: one CTA per SM, or a cluster per cell, each with its own workspace (Z and the per-point
+// factors).
 int dpg_launch_big(const DpgPlanDev* plan, const DpgLaunch* Lin, cudaStream_t stream) {
   if (Lin->solve_only)
     return dpg::fail(DPG_ERR_UNSUPPORTED, "large-bucket plans support the assembly entry points only");
-  const int grid = std::min(Lin->C, dpg::num_sms());
+  KernelFn kt = plan->big_zk == 16 ? dpg_big_kernel<16, true> : dpg_big_kernel<32, true>;
+  int grid = 0;  // workspaces: CTAs or clusters
+  const int team = team_size(plan, Lin->C, kt, &grid);
   DpgLaunch L = *Lin;
   void* ws = nullptr;
   if (!L.scratch) {  // a caller-provided workspace holds dpg_big_workspace_bytes(plan, C)
@@ -36,9 +83,18 @@ int dpg_launch_big(const DpgPlanDev* plan, const DpgLaunch* Lin, cudaStream_t st
     }
     L.scratch = (double*)ws;
   }
-  KernelFn k = plan->big_zk == 16 ? dpg_big_kernel<16> : dpg_big_kernel<32>;
-  k<<<grid, NT, (size_t)plan->bs_total * sizeof(double), stream>>>(*plan, L);
-  cudaError_t e = cudaGetLastError();
+  const size_t smem = (size_t)plan->bs_total * sizeof(double);
+  cudaError_t e;
+  if (team > 1) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    cluster_config(cfg, attr, grid * team, team, smem, stream);
+    e = cudaLaunchKernelEx(&cfg, kt, *plan, (const DpgLaunch)L);
+  } else {
+    KernelFn k = plan->big_zk == 16 ? dpg_big_kernel<16, false> : dpg_big_kernel<32, false>;
+    k<<<grid, NT, smem, stream>>>(*plan, L);
+    e = cudaGetLastError();
+  }
   if (ws) cudaFreeAsync(ws, stream);
   if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
   return DPG_OK;

@@ -32,6 +32,27 @@ constexpr int ZL = 68;  // shared row stride, == 4 (mod 16) doubles: conflict-fr
 // m16n8k16 steps per chunk); the plan's big_zk, chosen by dpg_plan_autotune
 constexpr int BIG_NOFAIL = 0x7fffffff;
 
+// A cell's CTAs: one, or the CTAs of a cluster (few cells: the idle SMs share each cell's tiles).
+// They share the cell's workspace; big_sync orders its writes before the other CTAs' reads.
+struct BigTeam {
+  int rank, size;
+};
+__device__ __forceinline__ BigTeam big_team() {
+  BigTeam t;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(t.rank));
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(t.size));
+  return t;
+}
+template <bool TEAM>
+__device__ __forceinline__ void big_sync() {
+  if (TEAM) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+}
+
 struct BigSm {
   double* D;   // [64][ZL] diagonal block, factored in place
   double* Xi;  // [64][ZL] inverse of its factor
@@ -135,11 +156,11 @@ __device__ __forceinline__ int big_var_mask(const DpgPlanDev& P, int r0) {
 // bh[q][r][a][k] = sum over IP entries of row r on var a of coef x slot x T_a[slot_e][k];
 // vt[row][k] = (w|J| or side measure) x coef x slot x (n_c) x (parity) x T_op[k] per term and point.
 __device__ void big_prep(const DpgPlanDev& P, const DpgLaunch& L, int cell, const BigSm& S, double* wq, double* bh,
-                         double* vt) {
-  const int tid = threadIdx.x;
+                         double* vt, const BigTeam team) {
+  const int tid = team.rank * NT + threadIdx.x, nth = team.size * NT;
   const int d = P.d, nv = P.nv;
   const double* co = L.coeff ? L.coeff + (size_t)cell * P.nslots * P.Ptot : nullptr;
-  for (int task = tid; task < P.QGpad * P.niprows; task += NT) {
+  for (int task = tid; task < P.QG * P.niprows; task += nth) {
     const int q = task / P.niprows, r = task - q * P.niprows;
     double gq[GEO];
     point_geometry(d, nv, S.nodes, P.dNG + (size_t)q * nv * d, P.wG[q], nullptr, gq);
@@ -161,7 +182,7 @@ __device__ void big_prep(const DpgPlanDev& P, const DpgLaunch& L, int cell, cons
   }
   const int nvt = P.nbe > 0 ? P.be[P.nbe - 1].z + P.be[P.nbe - 1].w : 0;
   const int8_t* par = L.parity + (size_t)cell * P.ns;
-  for (int task = tid; task < nvt; task += NT) {
+  for (int task = tid; task < nvt; task += nth) {
     int e = 0;
     while (task >= P.be[e].z + P.be[e].w) e++;
     const int4 be = P.be[e];
@@ -186,9 +207,8 @@ __device__ void big_prep(const DpgPlanDev& P, const DpgLaunch& L, int cell, cons
 // One formation tile.  kind 0: G rows r0.., columns c0.. (test rows); kind 1: E^T rows
 // (device trial columns) r0.., columns c0.. (test rows).
 template <int ZK>
-__device__ void big_form_tile(const DpgPlanDev& P, const DpgLaunch& L, int kind, int r0, int c0, bool diag, double* Z,
+__device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, int kind, int r0, int c0, bool diag, double* Z,
                               const BigSm& S, const double* wq, const double* bh, const double* vt) {
-  (void)L;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int wr = (warp >> 2) * 16, wc = (warp & 3) * 16;
@@ -331,9 +351,10 @@ __device__ void big_form_tile(const DpgPlanDev& P, const DpgLaunch& L, int kind,
             if (S.col[i] >= 0) {
               const double gii = acc[nb][e];
               if (gii > 0.0) s = 1.0 / sqrt(gii);
-              else atomicMin(&S.ints[0], i);
+              else atomicMin(fail, i);
             }
             S.sc[i] = s;
+            if (sc_out) sc_out[i] = s;
           }
         }
       __syncthreads();
@@ -531,6 +552,98 @@ __device__ void big_cholesky(const DpgPlanDev& P, double* Z, int kb, int ke, con
   __syncthreads();
 }
 
+// The same steps by the CTAs of a cluster: every CTA factors the diagonal block for itself, the row
+// blocks' panels and then the trailing tiles are dealt out (a contiguous run of the row-major tile list
+// per CTA, so a row's panel is loaded once), with a cluster barrier after each.  Same products
+// in the same order as big_cholesky.
+__device__ void big_cholesky_team(const DpgPlanDev& P, double* Z, int kb, int ke, const BigSm& S, int* fail,
+                                  const BigTeam team) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int wr = (warp >> 2) * 16, wc = (warp & 3) * 16;
+  const int ld = P.ldz, Zn = P.Zn;
+  auto load_block = [&](double* dst, int r0, int k0, int w) {
+    const int nr = min(ZT, Zn - r0);
+    double pre[ZT * ZT / NT];
+#pragma unroll
+    for (int u = 0; u < ZT * ZT / NT; u++) {
+      const int e = tid + u * NT, r = e >> 6, c = e & (ZT - 1);
+      pre[u] = (r < nr && c < w) ? Z[(size_t)(r0 + r) * ld + k0 + c] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < ZT * ZT / NT; u++) {
+      const int e = tid + u * NT;
+      dst[(e >> 6) * ZL + (e & (ZT - 1))] = pre[u];
+    }
+  };
+  for (int k0 = kb; k0 < ke; k0 += ZT) {
+    const int w = min(ZT, ke - k0);
+    const int wk = (w + 15) & ~15;
+    big_diag_block(Z, ld, k0, w, S, fail);
+    const int rbeg = k0 + w;
+    const int nrb = (Zn - rbeg + ZT - 1) / ZT;
+    for (int bi = team.rank; bi < nrb; bi += team.size) {
+      const int ri0 = rbeg + bi * ZT, nri = min(ZT, Zn - ri0);
+      __syncthreads();
+      load_block(S.LJ, ri0, k0, w);
+      __syncthreads();
+      double acc[2][4];
+#pragma unroll
+      for (int nb = 0; nb < 2; nb++) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.0;
+      big_mma_rows(S.LJ, S.Xi, wk, wr, wc, g, t, acc);
+#pragma unroll
+      for (int nb = 0; nb < 2; nb++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = wr + g + h * 8, c = wc + nb * 8 + 2 * t;
+          if (r < nri && c < w)
+            *reinterpret_cast<double2*>(Z + (size_t)(ri0 + r) * ld + k0 + c) =
+                make_double2(acc[nb][2 * h], acc[nb][2 * h + 1]);
+        }
+    }
+    big_sync<true>();
+    const int ntile = nrb * (nrb + 1) / 2;
+    const int t0 = (int)((long long)ntile * team.rank / team.size), t1 = (int)((long long)ntile * (team.rank + 1) / team.size);
+    int bi = 0;
+    while ((bi + 1) * (bi + 2) / 2 <= t0) bi++;
+    int bj = t0 - bi * (bi + 1) / 2, have = -1;
+    for (int tt = t0; tt < t1; tt++) {
+      const int ri0 = rbeg + bi * ZT, nri = min(ZT, Zn - ri0);
+      const int rj0 = rbeg + bj * ZT, nrj = min(ZT, Zn - rj0);
+      __syncthreads();  // the buffers are free
+      if (bi != have) load_block(S.LI, ri0, k0, w);
+      have = bi;
+      if (bj != bi) load_block(S.LJ, rj0, k0, w);
+      double2 zo[2][2];
+#pragma unroll
+      for (int nb = 0; nb < 2; nb++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = wr + g + h * 8, c = wc + nb * 8 + 2 * t;
+          zo[nb][h] = (r < nri && c < nrj) ? *reinterpret_cast<const double2*>(Z + (size_t)(ri0 + r) * ld + rj0 + c)
+                                           : make_double2(0.0, 0.0);
+        }
+      __syncthreads();
+      double acc[2][4];
+#pragma unroll
+      for (int nb = 0; nb < 2; nb++) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.0;
+      const bool upper = bj == bi && wc >= wr + 16;
+      if (!upper) big_mma_rows(S.LI, bj == bi ? S.LI : S.LJ, wk, wr, wc, g, t, acc);
+#pragma unroll
+      for (int nb = 0; nb < 2; nb++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = wr + g + h * 8, c = wc + nb * 8 + 2 * t;
+          if (!upper && r < nri && c < nrj)
+            *reinterpret_cast<double2*>(Z + (size_t)(ri0 + r) * ld + rj0 + c) =
+                make_double2(zo[nb][h].x - acc[nb][2 * h], zo[nb][h].y - acc[nb][2 * h + 1]);
+        }
+      if (++bj > bi) { bi++; bj = 0; }
+    }
+    big_sync<true>();
+  }
+}
+
 // Per-CTA table of a large plan: the test var and local dof of every device test row.
 __device__ __forceinline__ void big_cta_setup(const DpgPlanDev& P, const BigSm& S) {
   for (int i = threadIdx.x; i < P.Np; i += NT) {
@@ -543,56 +656,71 @@ __device__ __forceinline__ void big_cta_setup(const DpgPlanDev& P, const BigSm& 
   }
 }
 
-// One cell of a large plan; Z is this CTA's workspace (bz_per_cta doubles).
-template <int ZK>
-__device__ __forceinline__ void big_cell_body(const DpgPlanDev& P, const DpgLaunch& L, int cell, const BigSm& S, double* const Z) {
-  const int tid = threadIdx.x;
+// One cell of a large plan; Z is the workspace of its CTA or cluster (bz_per_cta doubles).
+template <int ZK, bool TEAM>
+__device__ __forceinline__ void big_cell_body(const DpgPlanDev& P, const DpgLaunch& L, int cell, const BigSm& S, double* const Z, const BigTeam team) {
+  const int tid = threadIdx.x, gtid = team.rank * NT + tid, nth = team.size * NT;
+  int* const fail = TEAM ? reinterpret_cast<int*>(Z + P.bz_sc + P.Np) : S.ints;  // first failing G column, field column
+  double* const sc_out = TEAM ? Z + P.bz_sc : nullptr;
   double* const wq = Z + P.bz_wq;
   double* const bh = Z + P.bz_bh;
   double* const vt = Z + P.bz_vt;
   const int Np = P.Np, Mp = P.Mp, M = P.M, ld = P.ldz;
   {
     __syncthreads();
-    if (tid == 0) { S.ints[0] = BIG_NOFAIL; S.ints[1] = BIG_NOFAIL; }
+    if (gtid == 0) { fail[0] = BIG_NOFAIL; fail[1] = BIG_NOFAIL; }
     if (tid < P.nv * P.d) S.nodes[tid] = L.nodes[(size_t)cell * P.nv * P.d + tid];
     __syncthreads();
-    big_prep(P, L, cell, S, wq, bh, vt);
-    for (size_t e = tid; e < (size_t)Mp * Mp; e += NT) {
+    big_prep(P, L, cell, S, wq, bh, vt, team);
+    for (size_t e = gtid; e < (size_t)Mp * Mp; e += nth) {
       const int r = (int)(e / Mp), c = (int)(e - (size_t)r * Mp);
       if (c <= r) Z[(size_t)(Np + r) * ld + Np + c] = 0.0;
     }
-    __syncthreads();
+    big_sync<TEAM>();
     const int nbg = (Np + ZT - 1) / ZT, nbm = (Mp + ZT - 1) / ZT;
-    for (int I = 0; I < nbg; I++) big_form_tile<ZK>(P, L, 0, I * ZT, I * ZT, true, Z, S, wq, bh, vt);
+    for (int I = team.rank; I < nbg; I += team.size)
+      big_form_tile<ZK>(P, fail, sc_out, 0, I * ZT, I * ZT, true, Z, S, wq, bh, vt);
+    if (TEAM) {
+      big_sync<TEAM>();
+      for (int i = tid; i < Np; i += NT) S.sc[i] = sc_out[i];
+      __syncthreads();
+    }
+    int deal = 0;  // the other tiles, dealt round robin
     for (int I = 1; I < nbg; I++)
-      for (int J = 0; J < I; J++) big_form_tile<ZK>(P, L, 0, I * ZT, J * ZT, false, Z, S, wq, bh, vt);
+      for (int J = 0; J < I; J++)
+        if (!TEAM || deal++ % team.size == team.rank)
+          big_form_tile<ZK>(P, fail, nullptr, 0, I * ZT, J * ZT, false, Z, S, wq, bh, vt);
     for (int J = 0; J < nbm; J++)
-      for (int I = 0; I < nbg; I++) big_form_tile<ZK>(P, L, 1, J * ZT, I * ZT, false, Z, S, wq, bh, vt);
+      for (int I = 0; I < nbg; I++)
+        if (!TEAM || deal++ % team.size == team.rank)
+          big_form_tile<ZK>(P, fail, nullptr, 1, J * ZT, I * ZT, false, Z, S, wq, bh, vt);
+    if (TEAM) big_sync<TEAM>();
     if (L.parts) {
       // G (N, N), B (M, N) and F (N) in user numbering: Z unscaled (dpg_assemble_parts)
       __syncthreads();
       const int N = P.N;
       if (L.G)
-        for (int e = tid; e < N * N; e += NT) {
+        for (int e = gtid; e < N * N; e += nth) {
           const int ur = e / N, uc = e - ur * N;
           const int dr = __ldg(P.u2d_test + ur), dc = __ldg(P.u2d_test + uc);
           L.G[(size_t)cell * N * N + e] = Z[(size_t)max(dr, dc) * ld + min(dr, dc)] / (S.sc[dr] * S.sc[dc]);
         }
       if (L.B)
-        for (int e = tid; e < M * N; e += NT) {
+        for (int e = gtid; e < M * N; e += nth) {
           const int ut = e / N, us = e - ut * N;
           const int ds = __ldg(P.u2d_test + us);
           L.B[(size_t)cell * M * N + e] = Z[(size_t)(Np + __ldg(P.u2d_trial + ut)) * ld + ds] / S.sc[ds];
         }
       if (L.F)
-        for (int us = tid; us < N; us += NT) {
+        for (int us = gtid; us < N; us += nth) {
           const int ds = __ldg(P.u2d_test + us);
           L.F[(size_t)cell * N + us] = Z[(size_t)(Np + P.fcol) * ld + ds] / S.sc[ds];
         }
-      __syncthreads();
+      big_sync<TEAM>();
       return;
     }
-    big_cholesky(P, Z, 0, Np, S, &S.ints[0]);
+    if (TEAM) big_cholesky_team(P, Z, 0, Np, S, &fail[0], team);
+    else big_cholesky(P, Z, 0, Np, S, &fail[0]);
     if (L.energy) {
       // energy error (dpg_energy_error): the rows below the test block now hold W = L^-1 E, so
       // e^2 = || L^-1 F - L^-1 B^T x ||^2 is a sum over the test rows, with no cancellation
@@ -607,75 +735,80 @@ __device__ __forceinline__ void big_cell_body(const DpgPlanDev& P, const DpgLaun
       double* red = S.LI;  // free after the factorisation
       if ((tid & 31) == 0) red[tid >> 5] = part;
       __syncthreads();
-      if (tid == 0) {
+      if (gtid == 0) {
         double e2 = 0.0;
         for (int w = 0; w < NT / 32; w++) e2 += red[w];
         // a failed factorisation of the test block leaves no energy to report
-        L.energy[cell] = S.ints[0] == BIG_NOFAIL ? sqrt(e2) : __longlong_as_double(0x7ff8000000000000ll);
+        L.energy[cell] = fail[0] == BIG_NOFAIL ? sqrt(e2) : __longlong_as_double(0x7ff8000000000000ll);
       }
     } else if (L.B) {
       // DLS local matrices (dpg_assemble_dls): the rows below the test block hold
       // W^T = (L^-1 E)^T, so W = L^-1 B^T and y = L^-1 F are read out in user numbering
       const int N = P.N;
       double* Wc = L.B + (size_t)cell * M * N;
-      for (size_t e = tid; e < (size_t)M * N; e += NT) {
+      for (size_t e = gtid; e < (size_t)M * N; e += nth) {
         const int ut = (int)(e / N), us = (int)(e - (size_t)ut * N);
         Wc[e] = Z[(size_t)(Np + __ldg(P.u2d_trial + ut)) * ld + __ldg(P.u2d_test + us)];
       }
       if (L.F)
-        for (int us = tid; us < N; us += NT) L.F[(size_t)cell * N + us] = Z[(size_t)(Np + P.fcol) * ld + __ldg(P.u2d_test + us)];
+        for (int us = gtid; us < N; us += nth) L.F[(size_t)cell * N + us] = Z[(size_t)(Np + P.fcol) * ld + __ldg(P.u2d_test + us)];
     } else {
     // trailing block = -[K_ext]: K, l out, then negate (padded field columns get a unit pivot)
     const double* T = Z + (size_t)Np * ld + Np;
     if (L.K)
-      for (size_t e = tid; e < (size_t)M * M; e += NT) {
+      for (size_t e = gtid; e < (size_t)M * M; e += nth) {
         const int ur = (int)(e / M), uc = (int)(e - (size_t)ur * M);
         const int dr = __ldg(P.u2d_trial + ur), dc = __ldg(P.u2d_trial + uc);
         L.K[(size_t)cell * M * M + e] = -T[(size_t)max(dr, dc) * ld + min(dr, dc)];
       }
     if (L.l)
-      for (int u = tid; u < M; u += NT) L.l[(size_t)cell * M + u] = -T[(size_t)P.fcol * ld + __ldg(P.u2d_trial + u)];
+      for (int u = gtid; u < M; u += nth) L.l[(size_t)cell * M + u] = -T[(size_t)P.fcol * ld + __ldg(P.u2d_trial + u)];
     if (L.S || L.s) {
-      __syncthreads();
-      for (size_t e = tid; e < (size_t)Mp * Mp; e += NT) {
+      big_sync<TEAM>();
+      for (size_t e = gtid; e < (size_t)Mp * Mp; e += nth) {
         const int r = (int)(e / Mp), c = (int)(e - (size_t)r * Mp);
         if (c <= r) {
           double* p = Z + (size_t)(Np + r) * ld + Np + c;
           *p = (r == c && r < P.nfp && __ldg(P.dev2user_trial + r) < 0) ? 1.0 : -*p;
         }
       }
-      big_cholesky(P, Z, Np, Np + P.nfp, S, &S.ints[1]);
+      big_sync<TEAM>();
+      if (TEAM) big_cholesky_team(P, Z, Np, Np + P.nfp, S, &fail[1], team);
+      else big_cholesky(P, Z, Np, Np + P.nfp, S, &fail[1]);
       const int nt = P.nt, nf = P.nf;
       if (L.S)
-        for (size_t e = tid; e < (size_t)nt * nt; e += NT) {
+        for (size_t e = gtid; e < (size_t)nt * nt; e += nth) {
           const int ur = (int)(e / nt), uc = (int)(e - (size_t)ur * nt);
           const int dr = __ldg(P.u2d_trial + nf + ur), dc = __ldg(P.u2d_trial + nf + uc);
           L.S[(size_t)cell * nt * nt + e] = T[(size_t)max(dr, dc) * ld + min(dr, dc)];
         }
       if (L.s)
-        for (int u = tid; u < nt; u += NT) L.s[(size_t)cell * nt + u] = T[(size_t)P.fcol * ld + __ldg(P.u2d_trial + nf + u)];
+        for (int u = gtid; u < nt; u += nth) L.s[(size_t)cell * nt + u] = T[(size_t)P.fcol * ld + __ldg(P.u2d_trial + nf + u)];
     }
     }
-    __syncthreads();
-    if (tid == 0 && L.info) {
+    big_sync<TEAM>();  // the cell's workspace is free for the next one
+    if (gtid == 0 && L.info) {
       int v = 0;
-      if (S.ints[0] != BIG_NOFAIL) {
-        const int u = P.dev2user_test[S.ints[0]];
-        v = (u >= 0 ? u : S.ints[0]) + 1;
-      } else if (S.ints[1] != BIG_NOFAIL) {
-        const int u = P.dev2user_trial[S.ints[1] - Np];
-        v = -((u >= 0 ? u : S.ints[1] - Np) + 1);
+      if (fail[0] != BIG_NOFAIL) {
+        const int u = P.dev2user_test[fail[0]];
+        v = (u >= 0 ? u : fail[0]) + 1;
+      } else if (fail[1] != BIG_NOFAIL) {
+        const int u = P.dev2user_trial[fail[1] - Np];
+        v = -((u >= 0 ? u : fail[1] - Np) + 1);
       }
       L.info[cell] = v;
     }
   }
 }
 
-template <int ZK>
+template <int ZK, bool TEAM>
 __global__ void __launch_bounds__(NT, 1) dpg_big_kernel(const __grid_constant__ DpgPlanDev P,
-                                                                  const __grid_constant__ DpgLaunch L) {
+                                                        const __grid_constant__ DpgLaunch L) {
   const BigSm S = big_views(P);
   big_cta_setup(P, S);
-  for (int cell = blockIdx.x; cell < L.C; cell += gridDim.x)
-    big_cell_body<ZK>(P, L, cell, S, L.scratch + (size_t)blockIdx.x * P.bz_per_cta);
+  BigTeam team{0, 1};
+  if (TEAM) team = big_team();
+  const int first = TEAM ? blockIdx.x / team.size : blockIdx.x, step = TEAM ? gridDim.x / team.size : gridDim.x;
+  double* const Z = L.scratch + (size_t)first * P.bz_per_cta;
+  for (int cell = first; cell < L.C; cell += step) big_cell_body<ZK, TEAM>(P, L, cell, S, Z, team);
 }

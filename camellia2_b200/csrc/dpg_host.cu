@@ -581,6 +581,7 @@ static int big_layout(HostPlan* P) {
   g.bz_wq = (int)o; o += al(g.QGpad);
   g.bz_bh = (int)o; o += al((size_t)g.QGpad * g.niprows * g.ntest * 4);
   g.bz_vt = (int)o; o += al((size_t)vrow * 4);
+  g.bz_sc = (int)o; o += al(g.Np + 1);
   g.bz_per_cta = o;
   g.big_zk = 32;
   int s = 5 * 64 * 68;  // diagonal block, its inverse, three panel blocks (formation buffers alias them)
@@ -827,9 +828,9 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
   g.nbt16 = nbt16;
   if (g.NBT > DPG_MAX_NBT) g.big = 1;  // the large-bucket kernel
   // staged reference slots of all test vars at a list of volume-reference points
-  auto fref_table = [&](const double* pts, int npts) {
+  auto fref_table = [&](const double* pts, int npts, int nreal) {  // padding repeats point 0
     std::vector<double> out((size_t)npts * g.featstride, 0.0);
-    for (int q = 0; q < npts; q++)
+    for (int q = 0; q < nreal; q++)
       for (int a = 0; a < g.ntest; a++) {
         const DpgTestVar& tv = g.test[a];
         std::vector<double> tmp((size_t)tv.card * (d + 1));
@@ -839,9 +840,10 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
         for (int i = 0; i < tv.card; i++)
           for (int m = 0; m <= d; m++) dst[(size_t)m * tv.ldA + i] = tmp[(size_t)i * (d + 1) + m];
       }
+    for (int q = nreal; q < npts; q++) std::copy_n(out.begin(), g.featstride, out.begin() + (size_t)q * g.featstride);
     return out;
   };
-  g.frefG = upload(P, fref_table(xG.data(), g.QGpad));
+  g.frefG = upload(P, fref_table(xG.data(), g.QGpad, g.QG));
   g.wG = upload(P, wG);
   g.dNG = upload(P, dshape(xG, g.QGpad));
 
@@ -1264,7 +1266,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
         xs[(size_t)q * d + k] = (sg == 0) ? rB.x[(size_t)src * d + k]
                                           : sidepts[((size_t)(sg - 1) * g.QSpad + src) * d + k];
     }
-    std::vector<double> slots = fref_table(xs.data(), npad);
+    std::vector<double> slots = fref_table(xs.data(), npad, S.npts);
     std::vector<double> rec((size_t)npad * S.rec_len, 0.0);
     for (int q = 0; q < npad; q++) {
       std::copy_n(slots.begin() + (size_t)q * g.featstride, foff, rec.begin() + (size_t)q * S.rec_len);
@@ -1308,7 +1310,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
       ses.push_back(st);
       for (int q = 0; q < g.QS; q++)
         for (int k = 0; k < d; k++) sidex[(size_t)q * d + k] = sidepts[((size_t)sd * g.QSpad + q) * d + k];
-      std::vector<double> sl = fref_table(sidex.data(), g.QS);
+      std::vector<double> sl = fref_table(sidex.data(), g.QS, g.QS);
       // reference side values of the test operator: T[q][r]
       std::vector<double> T((size_t)g.QS * V.card, 0.0);
       double tmax = 0.0;
@@ -1980,7 +1982,7 @@ struct dpg_graph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   int device = 0;
-  void* big_ws = nullptr;  // workspace of the large-bucket launches (they run one after another)
+  void* big_ws = nullptr;  // workspaces of the large-bucket launches
 };
 
 int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags, dpg_graph** out) {
@@ -1991,8 +1993,16 @@ int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags,
   int rc = multi_args(n_buckets, buckets, flags, plans, ls);
   if (rc != DPG_OK) return rc;
   split_big(plans, ls, bp, bl);
-  size_t big_bytes = 0;
-  for (size_t i = 0; i < bp.size(); i++) big_bytes = std::max(big_bytes, dpg_big_workspace_bytes(&bp[i], bl[i].C));
+  // every large bucket's own workspace, so that their launches can overlap; one for all of them, one after
+  // another, where that does not fit
+  size_t big_bytes = 0, big_most = 0;
+  std::vector<size_t> big_off;
+  for (size_t i = 0; i < bp.size(); i++) {
+    const size_t b = (dpg_big_workspace_bytes(&bp[i], bl[i].C) + 255) & ~(size_t)255;
+    big_off.push_back(big_bytes);
+    big_bytes += b;
+    big_most = std::max(big_most, b);
+  }
   if (plans.empty() && bp.empty()) return fail(DPG_ERR_INVALID_ARGUMENT, "no cells to capture");
   dpg_graph* G = new dpg_graph();
   std::memset(&G->dev, 0, sizeof(G->dev));
@@ -2007,26 +2017,61 @@ int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags,
     }
     rc = dpg_launch_multi(plans.data(), ls.data(), (int)plans.size(), nullptr, &G->dev, claim_of(flags));
   }
+  bool branches = true;
   if (rc == DPG_OK && big_bytes > 0 && cudaMalloc(&G->big_ws, big_bytes) != cudaSuccess) {
     cudaGetLastError();
-    G->big_ws = nullptr;
-    rc = fail(DPG_ERR_OUT_OF_MEMORY, "graph workspace of the large buckets");
+    branches = false;
+    if (cudaMalloc(&G->big_ws, big_most) != cudaSuccess) {
+      cudaGetLastError();
+      G->big_ws = nullptr;
+      rc = fail(DPG_ERR_OUT_OF_MEMORY, "graph workspace of the large buckets");
+    }
   }
-  // one stream: the large buckets' launches in decreasing order of cost, then the work queue
-  // of the single-CTA buckets (run beside them on a second branch, the queue's CTAs took SMs
-  // before the long large cells had started and lengthened the whole: 1.19 s against 1.17 s
-  // on the uneven-cell workload)
+  // one branch per large bucket and one for the work queue of the single-CTA buckets, with stream priorities
+  // in decreasing order of cost: a bucket's CTAs take the SMs that the last wave of the one before
+  // leaves idle, and the short cells come last.  (One after another, every bucket paid its own
+  // partial wave; without priorities, the queue's CTAs took SMs before the long cells had started.)
+  // 6,000 cells of the hp Stokes mesh: 64.9 ms one after another, 58.7 ms so.
   cudaStream_t cs0 = nullptr;
+  std::vector<cudaStream_t> bs;
+  std::vector<cudaEvent_t> ev;
+  auto new_event = [&]() {
+    cudaEvent_t e = nullptr;
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) ev.push_back(e);
+    else rc = fail(DPG_ERR_CUDA, "event creation");
+    return e;
+  };
+  int lo = 0, hi = 0;
+  cudaDeviceGetStreamPriorityRange(&lo, &hi);  // numerically: lowest priority, highest priority
   if (rc == DPG_OK && cudaStreamCreateWithFlags(&cs0, cudaStreamNonBlocking) != cudaSuccess)
     rc = fail(DPG_ERR_CUDA, "stream creation");
+  const size_t nbr = branches ? bp.size() + (plans.empty() ? 0 : 1) : 0;
+  for (size_t i = 0; rc == DPG_OK && i < nbr; i++) {
+    cudaStream_t st = nullptr;
+    const int pr = i < bp.size() ? std::min(hi + (int)i, lo) : lo;
+    if (cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, pr) != cudaSuccess) rc = fail(DPG_ERR_CUDA, "stream creation");
+    else bs.push_back(st);
+  }
   if (rc == DPG_OK) {
     cudaError_t e = cudaStreamBeginCapture(cs0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      for (size_t i = 0; rc == DPG_OK && i < bp.size(); i++) {
-        bl[i].scratch = (double*)G->big_ws;
-        rc = dpg_launch_assemble(&bp[i], nullptr, &bl[i], cs0);
+      cudaEvent_t fork = nullptr;
+      if (branches && (fork = new_event()) && cudaEventRecord(fork, cs0) != cudaSuccess) rc = fail(DPG_ERR_CUDA, "capture fork");
+      for (size_t i = 0; rc == DPG_OK && i < bp.size() + (plans.empty() ? 0 : 1); i++) {
+        cudaStream_t st = branches ? bs[i] : cs0;
+        if (branches && cudaStreamWaitEvent(st, fork, 0) != cudaSuccess) rc = fail(DPG_ERR_CUDA, "capture fork");
+        if (rc == DPG_OK && i < bp.size()) {
+          bl[i].scratch = (double*)((char*)G->big_ws + (branches ? big_off[i] : 0));
+          rc = dpg_launch_assemble(&bp[i], nullptr, &bl[i], st);
+        } else if (rc == DPG_OK) {
+          rc = dpg_launch_multi_prepared(&G->dev, st);
+        }
+        if (rc == DPG_OK && branches) {
+          cudaEvent_t join = new_event();
+          if (!join || cudaEventRecord(join, st) != cudaSuccess || cudaStreamWaitEvent(cs0, join, 0) != cudaSuccess)
+            rc = fail(DPG_ERR_CUDA, "capture join");
+        }
       }
-      if (rc == DPG_OK && !plans.empty()) rc = dpg_launch_multi_prepared(&G->dev, cs0);
       cudaError_t e2 = cudaStreamEndCapture(cs0, &G->graph);
       if (rc == DPG_OK && e2 != cudaSuccess) rc = fail(DPG_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e2));
     } else {
@@ -2035,6 +2080,8 @@ int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags,
   }
   if (rc == DPG_OK && cudaGraphInstantiate(&G->exec, G->graph, 0) != cudaSuccess)
     rc = fail(DPG_ERR_CUDA, "graph instantiation");
+  for (cudaEvent_t e : ev) cudaEventDestroy(e);
+  for (cudaStream_t st : bs) cudaStreamDestroy(st);
   if (cs0) cudaStreamDestroy(cs0);
   if (rc != DPG_OK) {
     cudaGetLastError();
