@@ -53,6 +53,16 @@ __device__ __forceinline__ void big_sync() {
   }
 }
 
+// A relevant entry of an E tile (one segment and term), in shared memory.
+struct BigEntry {
+  const double* rec;     // the segment's point records
+  int rec_len, tv;       // doubles per record; trial value of device column j at tv + j
+  int col0, col1;        // device trial columns
+  int var, foff, ld;     // test var, its slots in a record
+  int vt;                // first row of per-point factors
+  int k0, k1;            // its k range
+};
+
 struct BigSm {
   double* D;   // [64][ZL] diagonal block, factored in place
   double* Xi;  // [64][ZL] inverse of its factor
@@ -214,6 +224,7 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
   const int wr = (warp >> 2) * 16, wc = (warp & 3) * 16;
   int* rel = S.ints + 64;    // relevant IP rows (kind 0) or E entries (kind 1)
   int* relk = S.ints + 192;  // kind 1: first k of each relevant entry, then the total
+  BigEntry* const ent = reinterpret_cast<BigEntry*>(S.ints + 512);  // kind 1: the relevant entries
   __syncthreads();           // lists and operand buffers free
   if (tid == 0) {
     int n = 0, k = 0;
@@ -240,6 +251,27 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
   }
   __syncthreads();
   const int nrel = relk[120], nk = relk[121];
+  if (kind == 1) {
+    if (tid < nrel) {
+      const int4 be = P.be[rel[tid]];
+      const DpgSeg& Sg = P.seg[be.x];
+      const DpgBTerm& Tm = P.bterm[Sg.term0 + be.y];
+      BigEntry E;
+      E.rec = Sg.rec;
+      E.rec_len = Sg.rec_len;
+      E.tv = Sg.tvoff[be.y] - Tm.col0;
+      E.col0 = Tm.col0;
+      E.col1 = Tm.col0 + Tm.ncol;
+      E.var = Tm.test_var;
+      E.foff = P.test[Tm.test_var].foff;
+      E.ld = P.test[Tm.test_var].ldA;
+      E.vt = be.z;
+      E.k0 = relk[tid];
+      E.k1 = relk[tid] + be.w;
+      ent[tid] = E;
+    }
+    __syncthreads();
+  }
   double acc[2][4], acc2[2][4];
 #pragma unroll
   for (int nb = 0; nb < 2; nb++)
@@ -258,68 +290,91 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
     const int i = (side ? c0 : r0) + cc;
     crec[side] = (kind == 1 && side == 0) ? -1 : (i < P.Np ? S.col[i] : -1);
   }
-  // kind 1: each thread's k index only grows (chunk by chunk, and with u inside a chunk), so the
-  // entry holding it is found by a forward cursor per side instead of a scan from the start
-  int ecur[2] = {0, 0};
+  int fo[2], fl[2];  // the column's slots inside a Gram point's
+#pragma unroll
+  for (int side = 0; side < 2; side++) {
+    const DpgTestVar& V = P.test[crec[side] >= 0 ? crec[side] >> 16 : 0];
+    fo[side] = V.foff + (crec[side] & 0xffff);
+    fl[side] = V.ldA;
+  }
   // A thread forms KPT consecutive k of each side.  G tiles number k point-major (k = q nrel +
   // row), so a thread's run mostly stays on one point and reads its column's four reference slot
-  // values once for all the IP rows.
+  // values once for all the IP rows.  k only grows, by ZK per chunk: point and row (kind 0) or entry
+  // (kind 1) of the run's first k come from cursors, without divisions.
   constexpr int KPT = ZK / (NT / ZT);
+  const int kl0 = (tid >> 6) * KPT;
+  int cq = 0, cr = 0, dq = 0, dr = 0, ecur = 0;
+  if (kind == 0 && nrel > 0) {
+    cq = kl0 / nrel;
+    cr = kl0 - cq * nrel;
+    dq = ZK / nrel;
+    dr = ZK - dq * nrel;
+  }
   auto operands = [&](int k0, int buf) {
     double* const fa = S.fa + buf * 2 * ZK * ZL;
     double vals[NU];
-    int lastq = -1;
-    double fv[4] = {0.0, 0.0, 0.0, 0.0};
+    const int kk0 = k0 + kl0;
+    if (kind == 0) {
 #pragma unroll
-    for (int u = 0; u < NU; u++) {
-      const int side = u / KPT, kl = (tid >> 6) * KPT + (u % KPT);
-      if (u % KPT == 0) lastq = -1;
-      const int kk = k0 + kl;
-      double val = 0.0;
-      if (kk < nk) {
-        if (kind == 0) {
-          const int rec = crec[side];
-          if (rec >= 0) {
-            const int q = kk / nrel, r = rel[kk - q * nrel];
-            const int a = rec >> 16;
+      for (int side = 1; side >= 0; side--) {
+        if (side == 0 && diag) {  // the same columns: times the weight
+          int q = cq, r = cr;
+#pragma unroll
+          for (int u = 0; u < KPT; u++) {
+            vals[u] = kk0 + u < nk ? vals[KPT + u] * wq[q] : 0.0;
+            if (++r >= nrel) { r = 0; q++; }
+          }
+          break;
+        }
+        int q = cq, r = cr, lastq = -1;
+        double fv[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int u = 0; u < KPT; u++) {
+          double val = 0.0;
+          if (kk0 + u < nk && crec[side] >= 0) {
             if (q != lastq) {
-              const int ld = P.test[a].ldA;
-              const double* f = P.frefG + (size_t)q * P.featstride + P.test[a].foff + (rec & 0xffff);
-              fv[0] = __ldg(f); fv[1] = __ldg(f + ld); fv[2] = __ldg(f + 2 * ld); fv[3] = __ldg(f + 3 * ld);
+              const double* f = P.frefG + (size_t)q * P.featstride + fo[side];
+              fv[0] = __ldg(f); fv[1] = __ldg(f + fl[side]); fv[2] = __ldg(f + 2 * fl[side]); fv[3] = __ldg(f + 3 * fl[side]);
               lastq = q;
             }
-            const double* b = bh + ((size_t)(q * P.niprows + r) * P.ntest + a) * 4;
-            val = b[0] * fv[0] + b[1] * fv[1] + b[2] * fv[2] + b[3] * fv[3];
+            const double* b = bh + ((size_t)(q * P.niprows + rel[r]) * P.ntest + (crec[side] >> 16)) * 4;
+            const double2 b01 = *reinterpret_cast<const double2*>(b), b23 = *reinterpret_cast<const double2*>(b + 2);
+            val = b01.x * fv[0] + b01.y * fv[1] + b23.x * fv[2] + b23.y * fv[3];
             if (side == 0) val *= wq[q];
           }
-        } else {
-          int ei = ecur[side];
-          while (ei + 1 < nrel && kk >= relk[ei + 1]) ei++;
-          ecur[side] = ei;
-          const int4 be = P.be[rel[ei]];
-          const int q = kk - relk[ei];
-          const DpgSeg& Sg = P.seg[be.x];
-          const DpgBTerm& Tm = P.bterm[Sg.term0 + be.y];
-          const double* rq = Sg.rec + (size_t)q * Sg.rec_len;
-          if (side == 0) {
-            const int j = r0 + cc;
-            if (j >= Tm.col0 && j < Tm.col0 + Tm.ncol) val = __ldg(rq + Sg.tvoff[be.y] + (j - Tm.col0));
-          } else {
-            const int rec = crec[1];
-            if (rec >= 0 && (rec >> 16) == Tm.test_var) {
-              const int ld = P.test[Tm.test_var].ldA;
-              const double* f = rq + P.test[Tm.test_var].foff + (rec & 0xffff);
-              const double* v4 = vt + (size_t)(be.z + q) * 4;
-              val = v4[0] * __ldg(f) + v4[1] * __ldg(f + ld) + v4[2] * __ldg(f + 2 * ld) + v4[3] * __ldg(f + 3 * ld);
-            }
-          }
+          vals[side * KPT + u] = val;
+          if (++r >= nrel) { r = 0; q++; }
         }
       }
-      vals[u] = val;
+      cq += dq;
+      cr += dr;
+      if (cr >= nrel) { cr -= nrel; cq++; }
+    } else {
+      const int j = r0 + cc, rec = crec[1];
+#pragma unroll
+      for (int u = 0; u < KPT; u++) {
+        double v0 = 0.0, v1 = 0.0;
+        if (kk0 + u < nk) {
+          while (kk0 + u >= ent[ecur].k1) ecur++;
+          const BigEntry& E = ent[ecur];
+          const int q = kk0 + u - E.k0;
+          const double* rq = E.rec + (size_t)q * E.rec_len;
+          if (j >= E.col0 && j < E.col1) v0 = __ldg(rq + E.tv + j);
+          if (rec >= 0 && (rec >> 16) == E.var) {
+            const int ld = E.ld;
+            const double* f = rq + E.foff + (rec & 0xffff);
+            const double* v4 = vt + (size_t)(E.vt + q) * 4;
+            const double2 v01 = *reinterpret_cast<const double2*>(v4), v23 = *reinterpret_cast<const double2*>(v4 + 2);
+            v1 = v01.x * __ldg(f) + v01.y * __ldg(f + ld) + v23.x * __ldg(f + 2 * ld) + v23.y * __ldg(f + 3 * ld);
+          }
+        }
+        vals[u] = v0;
+        vals[KPT + u] = v1;
+      }
     }
 #pragma unroll
     for (int u = 0; u < NU; u++) {
-      const int side = u / KPT, kl = (tid >> 6) * KPT + (u % KPT);
+      const int side = u / KPT, kl = kl0 + (u % KPT);
       fa[side * ZK * ZL + kl * ZL + cc] = vals[u];
     }
   };
@@ -459,6 +514,19 @@ __device__ __forceinline__ void big_diag_block(const double* Z, int ld, int k0, 
   __syncthreads();
 }
 
+// Rows r0 .. r0 + 63 of panel columns k0 .. k0 + w - 1 of Z into a [64][ZL] block by asynchronous copies, zeros
+// beyond the matrix and the panel (k0, w and the row stride are even: 16-byte pieces; ld is a multiple of 8).
+__device__ __forceinline__ void big_copy_block(double* dst, const double* Z, int ld, int Zn, int r0, int k0, int w) {
+#pragma unroll
+  for (int u = 0; u < ZT * ZT / 2 / NT; u++) {
+    const int e = threadIdx.x + u * NT, r = e >> 5, c = 2 * (e & 31);
+    const bool in = r0 + r < Zn && c < w;
+    const double* src = in ? Z + (size_t)(r0 + r) * ld + k0 + c : Z;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + r * ZL + c)), "l"(src), "r"(in ? 16 : 0)
+                 : "memory");
+  }
+}
+
 // Steps kb .. ke-1 of a right-looking Cholesky of the lower triangle of Z (order Zn).  The
 // first column whose pivot is not positive goes to *fail (atomicMin); the cell's outputs are
 // then undefined (info reports the column).
@@ -471,20 +539,20 @@ __device__ void big_cholesky(const DpgPlanDev& P, double* Z, int kb, int ke, con
     const int w = min(ZT, ke - k0);
     const int wk = (w + 15) & ~15;
     big_diag_block(Z, ld, k0, w, S, fail);
-    // rows below the block: panel L_I = Z_I,k L_kk^-T (stored back), then Z_IJ -= L_I L_J^T
+    // rows below the block: panel L_I = Z_I,k L_kk^-T (stored back), then Z_IJ -= L_I L_J^T.  The
+    // next raw panel (in D, free after the diagonal block) and the next column block's panel are
+    // copied asynchronously while the products of a tile run; one barrier per tile.
     const int rbeg = k0 + w;
     const int nrb = (Zn - rbeg + ZT - 1) / ZT;
+    if (nrb > 0) big_copy_block(S.D, Z, ld, Zn, rbeg, k0, w);
     for (int bi = 0; bi < nrb; bi++) {
       const int ri0 = rbeg + bi * ZT, nri = min(ZT, Zn - ri0);
-      for (int e = tid; e < ZT * ZT; e += NT) {
-        const int r = e >> 6, c = e & (ZT - 1);
-        S.LJ[r * ZL + c] = (r < nri && c < w) ? Z[(size_t)(ri0 + r) * ld + k0 + c] : 0.0;
-      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
       double acc[2][4];
 #pragma unroll
       for (int nb = 0; nb < 2; nb++) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.0;
-      big_mma_rows(S.LJ, S.Xi, wk, wr, wc, g, t, acc);
+      big_mma_rows(S.D, S.Xi, wk, wr, wc, g, t, acc);
 #pragma unroll
       for (int nb = 0; nb < 2; nb++)
 #pragma unroll
@@ -494,33 +562,14 @@ __device__ void big_cholesky(const DpgPlanDev& P, double* Z, int kb, int ke, con
           *reinterpret_cast<double2*>(S.LI + r * ZL + c) = v;
           if (r < nri && c < w) *reinterpret_cast<double2*>(Z + (size_t)(ri0 + r) * ld + k0 + c) = v;
         }
-      // column blocks bj < bi come from the stored panel, double buffered through registers:
-      // tile bj + 1 is loaded while the MMAs of tile bj run; one barrier per tile
-      double pre[ZT * ZT / NT];
-      auto load_panel = [&](int bj) {
-        const int rj0 = rbeg + bj * ZT, nrj = min(ZT, Zn - rj0);
-#pragma unroll
-        for (int u = 0; u < ZT * ZT / NT; u++) {
-          const int e = tid + u * NT, r = e >> 6, c = e & (ZT - 1);
-          pre[u] = (r < nrj && c < w) ? Z[(size_t)(rj0 + r) * ld + k0 + c] : 0.0;
-        }
-      };
-      auto store_panel = [&](double* dst) {
-#pragma unroll
-        for (int u = 0; u < ZT * ZT / NT; u++) {
-          const int e = tid + u * NT;
-          dst[(e >> 6) * ZL + (e & (ZT - 1))] = pre[u];
-        }
-      };
-      if (bi > 0) {
-        load_panel(0);
-        store_panel(S.LJ1);
-      }
       __syncthreads();
+      if (bi + 1 < nrb) big_copy_block(S.D, Z, ld, Zn, ri0 + ZT, k0, w);
       for (int bj = 0; bj <= bi; bj++) {
         const int rj0 = rbeg + bj * ZT, nrj = min(ZT, Zn - rj0);
         const double* Lj = bj == bi ? S.LI : ((bj & 1) ? S.LJ : S.LJ1);
-        if (bj + 1 < bi) load_panel(bj + 1);
+        // column blocks bj < bi come from the stored panels; the first one of the next row block last
+        if (bj + 1 < bi) big_copy_block(((bj + 1) & 1) ? S.LJ : S.LJ1, Z, ld, Zn, rj0 + ZT, k0, w);
+        else if (bj == bi && bi + 1 < nrb) big_copy_block(S.LJ1, Z, ld, Zn, rbeg, k0, w);
         double2 zo[2][2];
 #pragma unroll
         for (int nb = 0; nb < 2; nb++)
@@ -544,8 +593,10 @@ __device__ void big_cholesky(const DpgPlanDev& P, double* Z, int kb, int ke, con
               *reinterpret_cast<double2*>(Z + (size_t)(ri0 + r) * ld + rj0 + c) =
                   make_double2(zo[nb][h].x - acc[nb][2 * h], zo[nb][h].y - acc[nb][2 * h + 1]);
           }
-        if (bj + 1 < bi) store_panel(((bj + 1) & 1) ? S.LJ : S.LJ1);
-        __syncthreads();
+        if (bj < bi) {
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          __syncthreads();
+        }
       }
     }
   }

@@ -587,7 +587,7 @@ static int big_layout(HostPlan* P) {
   int s = 5 * 64 * 68;  // diagonal block, its inverse, three panel blocks (formation buffers alias them)
   g.bs_sc = s; s += (g.Np + 15) & ~15;
   g.bs_col = s; s += ((g.Np + 1) / 2 + 15) & ~15;
-  g.bs_int = s; s += 256;  // 512 ints: flags, chunk point maps, relevance lists
+  g.bs_int = s; s += 256 + DPG_MAX_BF * 6;  // 512 ints: flags, relevance lists; then the E tile's entries (48 bytes)
   g.bs_nodes = s; s += 32;
   g.bs_total = s;
   if (s * 8 > DPG_SMEM) return fail(DPG_ERR_UNSUPPORTED, "large-bucket kernel: shared memory exceeded");
