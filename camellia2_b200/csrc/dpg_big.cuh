@@ -118,38 +118,48 @@ __device__ __forceinline__ void big_mma_kmajor(const double* fa, const double* f
   }
 }
 
-// acc += A B^T over k in [0, kn) (kn a multiple of 16), both stored row-major [row][k].  Odd
-// k-steps go to a second set of accumulators, so four independent DMMA chains are in flight.
+// acc += A B^T over k in [0, kn) (kn a multiple of 16, at most 64), both stored row-major [row][k].  Odd
+// k-steps go to a second set of accumulators, so four independent DMMA chains are in flight (the caller joins
+// them: big_join).  f0 and f1 run after the first and the second k-step: copies and loads of a tile issued
+// there cost nothing, between two tiles the tensor pipe waits for them.
+template <class F0, class F1>
 __device__ __forceinline__ void big_mma_rows(const double* A, const double* B, int kn, int wr, int wc, int g, int t,
-                                             double (&acc)[2][4]) {
-  double acc2[2][4];
+                                             double (&acc)[2][4], double (&acc2)[2][4], F0 f0, F1 f1) {
 #pragma unroll
-  for (int nb = 0; nb < 2; nb++) acc2[nb][0] = acc2[nb][1] = acc2[nb][2] = acc2[nb][3] = 0.0;
-  for (int k0 = 0; k0 < kn; k0 += 32) {
+  for (int s16 = 0; s16 < ZT / 16; s16++) {
+    const int kk = 16 * s16;
+    if (kk < kn) {
+      double a[8];
 #pragma unroll
-    for (int half = 0; half < 2; half++) {
-      const int kk = k0 + 16 * half;
-      if (kk < kn) {
-        double a[8];
+      for (int i = 0; i < 4; i++) {
+        a[2 * i] = A[(wr + g) * ZL + kk + t + 4 * i];
+        a[2 * i + 1] = A[(wr + g + 8) * ZL + kk + t + 4 * i];
+      }
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          a[2 * i] = A[(wr + g) * ZL + kk + t + 4 * i];
-          a[2 * i + 1] = A[(wr + g + 8) * ZL + kk + t + 4 * i];
-        }
+      for (int nb = 0; nb < 2; nb++) {
+        double b[4];
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++) {
-          double b[4];
-#pragma unroll
-          for (int i = 0; i < 4; i++) b[i] = B[(wc + nb * 8 + g) * ZL + kk + t + 4 * i];
-          dmma16(half ? acc2[nb] : acc[nb], a, b);
-        }
+        for (int i = 0; i < 4; i++) b[i] = B[(wc + nb * 8 + g) * ZL + kk + t + 4 * i];
+        dmma16((s16 & 1) ? acc2[nb] : acc[nb], a, b);
       }
     }
+    if (s16 == 0) f0();
+    if (s16 == 1) f1();
   }
+}
+
+__device__ __forceinline__ void big_zero(double (&a)[2][4], double (&b)[2][4]) {
 #pragma unroll
   for (int nb = 0; nb < 2; nb++)
 #pragma unroll
-    for (int e = 0; e < 4; e++) acc[nb][e] += acc2[nb][e];
+    for (int e = 0; e < 4; e++) a[nb][e] = b[nb][e] = 0.0;
+}
+
+__device__ __forceinline__ void big_join(double (&a)[2][4], const double (&b)[2][4]) {
+#pragma unroll
+  for (int nb = 0; nb < 2; nb++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) a[nb][e] += b[nb][e];
 }
 
 // Test vars whose (padded) rows meet [r0, r0 + 64).
@@ -549,10 +559,10 @@ __device__ void big_cholesky(const DpgPlanDev& P, double* Z, int kb, int ke, con
       const int ri0 = rbeg + bi * ZT, nri = min(ZT, Zn - ri0);
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
-      double acc[2][4];
-#pragma unroll
-      for (int nb = 0; nb < 2; nb++) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.0;
-      big_mma_rows(S.D, S.Xi, wk, wr, wc, g, t, acc);
+      double acc[2][4], acc2[2][4];
+      big_zero(acc, acc2);
+      big_mma_rows(S.D, S.Xi, wk, wr, wc, g, t, acc, acc2, [] {}, [] {});
+      big_join(acc, acc2);
 #pragma unroll
       for (int nb = 0; nb < 2; nb++)
 #pragma unroll
@@ -567,23 +577,32 @@ __device__ void big_cholesky(const DpgPlanDev& P, double* Z, int kb, int ke, con
       for (int bj = 0; bj <= bi; bj++) {
         const int rj0 = rbeg + bj * ZT, nrj = min(ZT, Zn - rj0);
         const double* Lj = bj == bi ? S.LI : ((bj & 1) ? S.LJ : S.LJ1);
-        // column blocks bj < bi come from the stored panels; the first one of the next row block last
-        if (bj + 1 < bi) big_copy_block(((bj + 1) & 1) ? S.LJ : S.LJ1, Z, ld, Zn, rj0 + ZT, k0, w);
-        else if (bj == bi && bi + 1 < nrb) big_copy_block(S.LJ1, Z, ld, Zn, rbeg, k0, w);
         double2 zo[2][2];
+        big_zero(acc, acc2);
+        // column blocks bj < bi come from the stored panels; the first one of the next row block last
+        auto next_block = [&]() {
+          if (bj + 1 < bi) big_copy_block(((bj + 1) & 1) ? S.LJ : S.LJ1, Z, ld, Zn, rj0 + ZT, k0, w);
+          else if (bj == bi && bi + 1 < nrb) big_copy_block(S.LJ1, Z, ld, Zn, rbeg, k0, w);
+        };
+        auto old_values = [&]() {
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++)
+          for (int nb = 0; nb < 2; nb++)
 #pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const int r = wr + g + h * 8, c = wc + nb * 8 + 2 * t;
-            zo[nb][h] = (r < nri && c < nrj) ? *reinterpret_cast<const double2*>(Z + (size_t)(ri0 + r) * ld + rj0 + c)
-                                             : make_double2(0.0, 0.0);
-          }
-#pragma unroll
-        for (int nb = 0; nb < 2; nb++) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.0;
+            for (int h = 0; h < 2; h++) {
+              const int r = wr + g + h * 8, c = wc + nb * 8 + 2 * t;
+              zo[nb][h] = (r < nri && c < nrj) ? *reinterpret_cast<const double2*>(Z + (size_t)(ri0 + r) * ld + rj0 + c)
+                                               : make_double2(0.0, 0.0);
+            }
+        };
         // on the diagonal tile, warp tiles wholly above the diagonal are not needed
         const bool upper = bj == bi && wc >= wr + 16;
-        if (!upper) big_mma_rows(S.LI, Lj, wk, wr, wc, g, t, acc);
+        big_mma_rows(S.LI, Lj, upper ? 0 : wk, wr, wc, g, t, acc, acc2, next_block, old_values);
+        // the barrier before the sums are touched: their products drain while the warps meet
+        if (bj < bi) {
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          __syncthreads();
+        }
+        big_join(acc, acc2);
 #pragma unroll
         for (int nb = 0; nb < 2; nb++)
 #pragma unroll
@@ -593,10 +612,6 @@ __device__ void big_cholesky(const DpgPlanDev& P, double* Z, int kb, int ke, con
               *reinterpret_cast<double2*>(Z + (size_t)(ri0 + r) * ld + rj0 + c) =
                   make_double2(zo[nb][h].x - acc[nb][2 * h], zo[nb][h].y - acc[nb][2 * h + 1]);
           }
-        if (bj < bi) {
-          asm volatile("cp.async.wait_all;" ::: "memory");
-          __syncthreads();
-        }
       }
     }
   }
@@ -638,10 +653,10 @@ __device__ void big_cholesky_team(const DpgPlanDev& P, double* Z, int kb, int ke
       __syncthreads();
       load_block(S.LJ, ri0, k0, w);
       __syncthreads();
-      double acc[2][4];
-#pragma unroll
-      for (int nb = 0; nb < 2; nb++) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.0;
-      big_mma_rows(S.LJ, S.Xi, wk, wr, wc, g, t, acc);
+      double acc[2][4], acc2[2][4];
+      big_zero(acc, acc2);
+      big_mma_rows(S.LJ, S.Xi, wk, wr, wc, g, t, acc, acc2, [] {}, [] {});
+      big_join(acc, acc2);
 #pragma unroll
       for (int nb = 0; nb < 2; nb++)
 #pragma unroll
@@ -675,11 +690,11 @@ __device__ void big_cholesky_team(const DpgPlanDev& P, double* Z, int kb, int ke
                                            : make_double2(0.0, 0.0);
         }
       __syncthreads();
-      double acc[2][4];
-#pragma unroll
-      for (int nb = 0; nb < 2; nb++) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.0;
+      double acc[2][4], acc2[2][4];
+      big_zero(acc, acc2);
       const bool upper = bj == bi && wc >= wr + 16;
-      if (!upper) big_mma_rows(S.LI, bj == bi ? S.LI : S.LJ, wk, wr, wc, g, t, acc);
+      if (!upper) big_mma_rows(S.LI, bj == bi ? S.LI : S.LJ, wk, wr, wc, g, t, acc, acc2, [] {}, [] {});
+      big_join(acc, acc2);
 #pragma unroll
       for (int nb = 0; nb < 2; nb++)
 #pragma unroll
