@@ -31,6 +31,7 @@ constexpr int ZL = 68;  // shared row stride, == 4 (mod 16) doubles: conflict-fr
 // ZK (template parameter below): k-chunk of a formation tile, 16 or 32 points (one or two
 // m16n8k16 steps per chunk); the plan's big_zk, chosen by dpg_plan_autotune
 constexpr int BIG_NOFAIL = 0x7fffffff;
+static_assert(DPG_MAX_IPROWS <= 32 && DPG_MAX_BF <= 120, "relevance lists of a formation tile");
 
 // A cell's CTAs: one, or the CTAs of a cluster (few cells: the idle SMs share each cell's tiles).
 // They share the cell's workspace; big_sync orders its writes before the other CTAs' reads.
@@ -236,28 +237,48 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
   int* relk = S.ints + 192;  // kind 1: first k of each relevant entry, then the total
   BigEntry* const ent = reinterpret_cast<BigEntry*>(S.ints + 512);  // kind 1: the relevant entries
   __syncthreads();           // lists and operand buffers free
-  if (tid == 0) {
+  if (warp == 0) {  // ordered lists by ballots (one thread walking a hundred entries took 10 K cycles)
+    const unsigned below = (1u << lane) - 1u;
     int n = 0, k = 0;
+    const int mc = big_var_mask(P, c0);
     if (kind == 0) {
-      const int mr = big_var_mask(P, r0), mc = big_var_mask(P, c0);
-      for (int r = 0; r < P.niprows; r++)
-        if ((P.ipmask[r] & mr) && (P.ipmask[r] & mc)) rel[n++] = r;
+      const int mr = big_var_mask(P, r0);
+      const bool in = lane < P.niprows && (P.ipmask[lane] & mr) && (P.ipmask[lane] & mc);
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (in) rel[__popc(m & below)] = lane;
+      n = __popc(m);
       k = n * P.QG;
     } else {
-      const int mc = big_var_mask(P, c0);
-      for (int e = 0; e < P.nbe; e++) {
-        const int4 be = P.be[e];
-        const DpgBTerm& Tm = P.bterm[P.seg[be.x].term0 + be.y];
-        if (!((mc >> Tm.test_var) & 1)) continue;
-        if (Tm.col0 >= r0 + ZT || Tm.col0 + Tm.ncol <= r0) continue;
-        rel[n] = e;
-        relk[n] = k;
-        k += be.w;
-        n++;
+      for (int e0 = 0; e0 < P.nbe; e0 += 32) {
+        const int e = e0 + lane;
+        bool in = e < P.nbe;
+        int w = 0;
+        if (in) {
+          const int4 be = P.be[e];
+          const DpgBTerm& Tm = P.bterm[P.seg[be.x].term0 + be.y];
+          in = ((mc >> Tm.test_var) & 1) && Tm.col0 < r0 + ZT && Tm.col0 + Tm.ncol > r0;
+          if (in) w = be.w;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        int sum = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int x = __shfl_up_sync(0xffffffffu, sum, o);
+          if (lane >= o) sum += x;
+        }
+        if (in) {
+          const int at = n + __popc(m & below);
+          rel[at] = e;
+          relk[at] = k + sum - w;
+        }
+        n += __popc(m);
+        k += __shfl_sync(0xffffffffu, sum, 31);
       }
     }
-    relk[120] = n;
-    relk[121] = k;
+    if (lane == 0) {
+      relk[120] = n;
+      relk[121] = k;
+    }
   }
   __syncthreads();
   const int nrel = relk[120], nk = relk[121];
@@ -320,22 +341,22 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
     dq = ZK / nrel;
     dr = ZK - dq * nrel;
   }
-  auto operands = [&](int k0, int buf) {
+  // part 0: the column side of a G tile, or the first half of an E tile's k; part 1: the rest
+  double vals[NU];
+  auto operands = [&](int k0, int buf, auto part_c) {
+    constexpr int part = decltype(part_c)::value;
     double* const fa = S.fa + buf * 2 * ZK * ZL;
-    double vals[NU];
     const int kk0 = k0 + kl0;
     if (kind == 0) {
+      constexpr int side = 1 - part;
+      if (side == 0 && diag) {  // the same columns: times the weight
+        int q = cq, r = cr;
 #pragma unroll
-      for (int side = 1; side >= 0; side--) {
-        if (side == 0 && diag) {  // the same columns: times the weight
-          int q = cq, r = cr;
-#pragma unroll
-          for (int u = 0; u < KPT; u++) {
-            vals[u] = kk0 + u < nk ? vals[KPT + u] * wq[q] : 0.0;
-            if (++r >= nrel) { r = 0; q++; }
-          }
-          break;
+        for (int u = 0; u < KPT; u++) {
+          vals[u] = kk0 + u < nk ? vals[KPT + u] * wq[q] : 0.0;
+          if (++r >= nrel) { r = 0; q++; }
         }
+      } else {
         int q = cq, r = cr, lastq = -1;
         double fv[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
@@ -356,13 +377,17 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
           if (++r >= nrel) { r = 0; q++; }
         }
       }
-      cq += dq;
-      cr += dr;
-      if (cr >= nrel) { cr -= nrel; cq++; }
+      if (part == 1) {
+        cq += dq;
+        cr += dr;
+        if (cr >= nrel) { cr -= nrel; cq++; }
+      }
+#pragma unroll
+      for (int u = 0; u < KPT; u++) fa[side * ZK * ZL + (kl0 + u) * ZL + cc] = vals[side * KPT + u];
     } else {
       const int j = r0 + cc, rec = crec[1];
 #pragma unroll
-      for (int u = 0; u < KPT; u++) {
+      for (int u = part * KPT / 2; u < (part + 1) * KPT / 2; u++) {
         double v0 = 0.0, v1 = 0.0;
         if (kk0 + u < nk) {
           while (kk0 + u >= ent[ecur].k1) ecur++;
@@ -381,20 +406,28 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
         vals[u] = v0;
         vals[KPT + u] = v1;
       }
-    }
 #pragma unroll
-    for (int u = 0; u < NU; u++) {
-      const int side = u / KPT, kl = kl0 + (u % KPT);
-      fa[side * ZK * ZL + kl * ZL + cc] = vals[u];
+      for (int u = part * KPT / 2; u < (part + 1) * KPT / 2; u++) {
+        fa[(kl0 + u) * ZL + cc] = vals[u];
+        fa[(ZK + kl0 + u) * ZL + cc] = vals[KPT + u];
+      }
     }
   };
-  if (nk > 0) operands(0, 0);
+  constexpr std::integral_constant<int, 0> part0{};
+  constexpr std::integral_constant<int, 1> part1{};
+  if (nk > 0) {
+    operands(0, 0, part0);
+    operands(0, 0, part1);
+  }
   __syncthreads();
   for (int k0 = 0, c = 0; k0 < nk; k0 += ZK, c++) {
-    // the products of chunk c are issued first, so they run while chunk c + 1's loads are in flight
+    // chunk c + 1's operands are formed between and after the products of chunk c, which run meanwhile
     const double* fa = S.fa + (c & 1) * 2 * ZK * ZL;
-    big_mma_kmajor<ZK>(fa, fa + ZK * ZL, wr, wc, g, t, acc, acc2);
-    if (k0 + ZK < nk) operands(k0 + ZK, (c + 1) & 1);
+    const bool more = k0 + ZK < nk;
+    big_mma_kmajor<16>(fa, fa + ZK * ZL, wr, wc, g, t, acc, acc2);
+    if (more) operands(k0 + ZK, (c + 1) & 1, part0);
+    if (ZK == 32) big_mma_kmajor<16>(fa + 16 * ZL, fa + (ZK + 16) * ZL, wr, wc, g, t, acc2, acc);
+    if (more) operands(k0 + ZK, (c + 1) & 1, part1);
     __syncthreads();
   }
 #pragma unroll
