@@ -629,6 +629,7 @@ static int smem_layout_stages(DpgPlanDev& g, int chg, int stages, bool adj_terms
   g.b_u = o; o += al(g.max_chunk * g.max_ustride);
   g.b_geo = o; o += al(g.nbpts * 24);
   g.b_fac = o; o += al(g.nse * g.QS);
+  g.b_row = o; o += al(2 * g.max_chunk * g.max_nterm * 4);
   int bphase = o;
   g.sm_w = 0;
   int wsz = g.MBT * g.NBT * 64;
@@ -1213,7 +1214,7 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
     // B points, per-point term rows R, coefficients
     auto fits = [&](int ch, int smem) {
       const int budget = smem / 8 - DPG_SM_PERSIST - 2 * ((g.ngb * (int)sizeof(DpgGTile) + 7) / 8) - 64 - g.Np - g.Mp - 64;
-      int need = 2 * ch * g.max_rec + ch * g.max_ustride + g.nbpts * 24 + g.nslots * g.Ptot + 64 +
+      int need = 2 * ch * g.max_rec + ch * g.max_ustride + 2 * ch * g.max_nterm * 4 + g.nbpts * 24 + g.nslots * g.Ptot + 64 +
                  (int)sterms.size() * g.QS + 16;
       return need <= budget;
     };
@@ -1286,6 +1287,21 @@ static int build(HostPlan* P, const dpg_bucket_desc* D) {
       }
     }
     S.rec = upload(P, rec);
+    if (!g.big) {
+      std::vector<int> ustart(1, 0), ucon;
+      for (int kb = 0; kb < S.nblk; kb++)
+        for (int cl = 0; cl < 8; cl++) {
+          for (int i = 0; i < S.blk[kb].nt; i++) {
+            const int lt = S.blk[kb].terms[i];
+            const DpgBTerm& t = g.bterm[S.term0 + lt];
+            const int mm = S.blk[kb].J * 8 + cl - t.col0;
+            if (mm >= 0 && mm < t.ncol) ucon.push_back((S.tvoff[lt] + mm) | (lt << 16));
+          }
+          ustart.push_back((int)ucon.size());
+        }
+      S.ustart = upload_i(P, ustart);
+      S.ucon = upload_i(P, ucon);
+    }
   }
 
   // separable side terms -> entries (row, col) with per-point weights

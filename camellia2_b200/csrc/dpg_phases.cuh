@@ -449,6 +449,36 @@ __device__ __noinline__ void tile_cholesky(int T_off, int nb, int nsteps, int fl
 // ---------------------------------------------------------------------------
 // Phase 1: B and F -> per-CTA scratch (or the B/F outputs in parts mode)
 // ---------------------------------------------------------------------------
+// Term rows of chunk c of segment sgi (or of the next segment's first chunk): row[lq][term][m] = w|J| (or the
+// side measure) x coef x slot x (n) x (parity) x T_op[m], one thread per point and term, counted from the
+// last thread; buf: which of the two row buffers.
+__device__ __forceinline__ void b_term_rows(const DpgPlanDev& P, const DpgLaunch& L, const int8_t* par_c,
+                                            const double* geo, int sgi, int c, int buf) {
+  DPG_SMEM_VIEWS(P);
+  if (c >= P.seg[sgi].nchunk) {
+    c = 0;
+    sgi++;
+    while (sgi < P.nseg && P.seg[sgi].nterm == 0) sgi++;
+    if (sgi >= P.nseg) return;
+  }
+  const DpgSeg& S = P.seg[sgi];
+  const int q0 = c * S.chunk, n = min(S.chunk, S.npts - q0) * S.nterm;
+  double* const rows = sm + P.b_row + buf * P.max_chunk * P.max_nterm * 4;
+  for (int task = NT - 1 - (int)threadIdx.x; task < n; task += NT) {
+    const int lq = task / S.nterm, lt = task - lq * S.nterm, q = q0 + lq;
+    const double* gq = geo + (S.geo0 + q) * GEO;
+    const DpgBTerm& Tm = P.bterm[S.term0 + lt];
+    double v = gq[19] * Tm.coef;
+    if (Tm.slot >= 0) v *= coef_s[Tm.slot * P.Ptot + S.pbase + q];
+    if (Tm.normal_comp >= 0) v *= gq[20 + Tm.normal_comp];
+    if (Tm.kind == DPG_VAR_FLUX) v *= (double)par_c[S.side];
+    double tr[4];
+    trow_op(P.test[Tm.test_var].space, P.d, Tm.test_op, gq, tr);
+    double* dst = rows + task * 4;
+    dst[0] = tr[0] * v; dst[1] = tr[1] * v; dst[2] = tr[2] * v; dst[3] = tr[3] * v;
+  }
+}
+
 template <int BTW>
 __device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, int cell) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -478,9 +508,10 @@ __device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, in
   // then one thread per entry (scratch element); entries are unique, and an element
   // that a bilinear block also writes is read-modified-written (the blocks add to it
   // after the chunk loop's barriers)
+  __syncthreads();  // geometry complete, scratch zeroed
+  if (first_seg < P.nseg) b_term_rows(P, L, par_c, geo, first_seg, 0, 0);
   if (P.nse > 0) {
     double* fac = sm + P.b_fac;  // [nse][QS]
-    __syncthreads();             // geometry complete, scratch zeroed
     for (int task = tid; task < P.nse * P.QS; task += NT) {
       const int se = task / P.QS, q = task - se * P.QS;
       const DpgSideTerm& E = P.se[se];
@@ -559,39 +590,32 @@ __device__ __noinline__ void phase_b(const DpgPlanDev& P, const DpgLaunch& L, in
         if (!mbar_wait(&mbar_s[DPG_BAR_B + buf], (par >> buf) & 1)) flag_s[2] = 1;
         flag_s[3] = par ^ (1 << buf);
       }
-      const int q0 = c * S.chunk;
-      const int nq = min(S.chunk, S.npts - q0);
+      const int nq = min(S.chunk, S.npts - c * S.chunk);
       __syncthreads();
-      // U blocks: U[lq][blk][m][col] = sum over the block's terms of
-      //   (w*|J| * coef * slot * (n) * (parity) * T_op[m]) * trial value
-      for (int task = tid; task < S.chunk * S.nblk * 8; task += NT) {
-        const int lq = task / (S.nblk * 8);
-        const int rem = task - lq * S.nblk * 8;
-        const int kb = rem >> 3, cl = rem & 7;
-        const DpgBBlock& Bk = S.blk[kb];
-        const int col = Bk.J * 8 + cl;
-        double u0 = 0.0, u1 = 0.0, u2 = 0.0, u3 = 0.0;
-        if (lq < nq) {
-          const int q = q0 + lq;
-          const double* rq = rec + lq * S.rec_len;
-          const double* gq = geo + (S.geo0 + q) * GEO;
-          const int space = P.test[Bk.var].space;
-          for (int i = 0; i < Bk.nt; i++) {
-            const int lt = Bk.terms[i];
-            const DpgBTerm& Tm = P.bterm[S.term0 + lt];
-            const int mm = col - Tm.col0;
-            if (mm < 0 || mm >= Tm.ncol) continue;
-            double v = gq[19] * Tm.coef * rq[S.tvoff[lt] + mm];
-            if (Tm.slot >= 0) v *= coef_s[Tm.slot * P.Ptot + S.pbase + q];
-            if (Tm.normal_comp >= 0) v *= gq[20 + Tm.normal_comp];
-            if (Tm.kind == DPG_VAR_FLUX) v *= (double)par_c[S.side];
-            double tr[4];
-            trow_op(space, d, Tm.test_op, gq, tr);
-            u0 += tr[0] * v; u1 += tr[1] * v; u2 += tr[2] * v; u3 += tr[3] * v;
+      // U blocks: U[lq][blk][m][col] = sum over the (block, column)'s terms of row[lq][term][m] x trial value;
+      // beside them the last threads form the next chunk's term rows
+      b_term_rows(P, L, par_c, geo, sgi, c + 1, (gc + 1) & 1);
+      {
+        const double* const rows = sm + P.b_row + (gc & 1) * P.max_chunk * P.max_nterm * 4;
+        const int per = S.nblk * 8, nterm = S.nterm, rl = S.rec_len, us = S.ustride;
+        const int *const ustart = S.ustart, *const ucon = S.ucon;
+        for (int task = tid; task < S.chunk * per; task += NT) {
+          const int lq = task / per, rem = task - lq * per;
+          double u0 = 0.0, u1 = 0.0, u2 = 0.0, u3 = 0.0;
+          if (lq < nq) {
+            const double* rq = rec + lq * rl;
+            const int i1 = __ldg(ustart + rem + 1);
+            for (int i = __ldg(ustart + rem); i < i1; i++) {
+              const int v = __ldg(ucon + i);
+              const double psi = rq[v & 0xffff];
+              const double2* R = reinterpret_cast<const double2*>(rows + (lq * nterm + (v >> 16)) * 4);
+              const double2 r01 = R[0], r23 = R[1];
+              u0 += r01.x * psi; u1 += r01.y * psi; u2 += r23.x * psi; u3 += r23.y * psi;
+            }
           }
+          double* uq = U + lq * us + (rem >> 3) * 4 * DPG_ULD + (rem & 7);
+          uq[0] = u0; uq[DPG_ULD] = u1; uq[2 * DPG_ULD] = u2; uq[3 * DPG_ULD] = u3;
         }
-        double* uq = U + lq * S.ustride + Bk.off + cl;
-        uq[0] = u0; uq[DPG_ULD] = u1; uq[2 * DPG_ULD] = u2; uq[3 * DPG_ULD] = u3;
       }
       __syncthreads();
       // DMMA over this warp's active blocks of the segment: m16n8k16, one k-step = 4 points x 4 slots
@@ -862,12 +886,6 @@ __device__ __forceinline__ void gram_body(const DpgPlanDev& P, const DpgLaunch& 
   }
 }
 
-// A function of its own in 3D, where inlining beside the other phases spills accumulators.
-template <int GTM>
-__device__ __noinline__ void gram_chunks3d(const DpgPlanDev& P, const DpgLaunch& L, int sm_nodes) {
-  gram_body<GTM, 3>(P, L, sm_nodes);
-}
-
 // ---------------------------------------------------------------------------
 // Phase 2: Gram matrix -> lower tiles in shared memory
 // ---------------------------------------------------------------------------
@@ -930,7 +948,7 @@ __device__ __forceinline__ void phase_gram(const DpgPlanDev& P, const DpgLaunch&
       bulk_g2s(sm + P.g_fref + c * P.gstage, P.frefG + (size_t)c * P.chg * P.featstride, chunk_bytes, &mbar_s[c]);
     }
   }
-  if (d == 3) gram_chunks3d<GTM>(P, L, P.sm_nodes);
+  if (d == 3) gram_body<GTM, 3>(P, L, P.sm_nodes);
   else gram_body<GTM, 2>(P, L, P.sm_nodes);
   // tiles of uncoupled var pairs are zero
   for (int e = tid; e < P.ngz * 64; e += NT) GT[P.gzero[e >> 6] * 64 + (e & 63)] = 0.0;

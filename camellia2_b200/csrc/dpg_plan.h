@@ -98,6 +98,8 @@ struct DpgSeg {
   int nblk;
   DpgBBlock blk[DPG_MAX_BLK];
   int ustride;              // doubles per point of staged U blocks
+  const int* ustart;        // [nblk * 8 + 1] first contribution of each (block, column)
+  const int* ucon;          // contributions: trial value's offset in a record | segment-local term << 16
   int term0, nterm;         // range in the segment-sorted term list
   int tvoff[DPG_MAX_BF / 4];// offset of each (segment-local) term's trial values inside a record
   int tile0, ntile;         // active (I, J) tiles of the segment: btiles[tile0 .. tile0 + ntile)
@@ -200,7 +202,7 @@ struct DpgPlanDev {
   int sm_coef;    // per cell: coefficients [nslots][Ptot]
   int g_fref, g_geo, g_D, g_beta;   // Gram phase (g_beta overlaps the stages after the first)
   int sm_gt, sm_linv, sm_scale;                    // factor
-  int b_rec0, b_rec1, b_u, b_geo, b_fac;      // B phase
+  int b_rec0, b_rec1, b_u, b_geo, b_fac, b_row;  // B phase (b_row: term rows of two chunks)
   int sm_w, sm_k;                                  // solve / Gram of W
   int a_sa, a_ldS;                                 // adjoint: S_A [MBT*8][a_ldS]
   int a_fs, a_xpf, a_ldx, a_geo, a_beta, a_cbar;   // adjoint pull-back
