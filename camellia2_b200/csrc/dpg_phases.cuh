@@ -348,6 +348,8 @@ __device__ __forceinline__ void chol_chain(double* T, int nb, int nsteps, int* f
   for (int k = 0; k < nsteps; k++) {
     const int i = k + 1;
     double* Lik = T + (i * (i + 1) / 2 + k) * 64;
+    double2 c2 = make_double2(0.0, 0.0);
+    if (i < nsteps) c2 = *reinterpret_cast<const double2*>(Lik + 64 + ak_cfrag(g, t));
     if (i < nb) {
       const double* Li = linv + k * 64;
       const double a0 = Lik[lane], a1 = Lik[32 + lane];
@@ -361,10 +363,9 @@ __device__ __forceinline__ void chol_chain(double* T, int nb, int nsteps, int* f
     __syncwarp();
     if (i < nsteps) {
       double* Tii = Lik + 64;
-      double2 c = *reinterpret_cast<const double2*>(Tii + ak_cfrag(g, t));
-      dmma(c, -Lik[lane], Lik[lane]);
-      dmma(c, -Lik[32 + lane], Lik[32 + lane]);
-      *reinterpret_cast<double2*>(Tii + ak_cfrag(g, t)) = c;
+      dmma(c2, -Lik[lane], Lik[lane]);
+      dmma(c2, -Lik[32 + lane], Lik[32 + lane]);
+      *reinterpret_cast<double2*>(Tii + ak_cfrag(g, t)) = c2;
       __syncwarp();
       factor_diag(T, i, flag, sgn, linv);
     }
@@ -393,14 +394,17 @@ __device__ __forceinline__ void chol_tile(double* T, int i, int j, int n, int la
   const double* pa = T + (i * (i + 1) / 2) * 64 + lane;
   const double* pb = T + (j * (j + 1) / 2) * 64 + lane;
   double* C = T + (i * (i + 1) / 2 + j) * 64 + ak_cfrag(g, t);
-  double2 c = *reinterpret_cast<const double2*>(C);
+  // two chains of products (m8n8k4: 26 cycles to its result, 16 on the pipe)
+  double2 c = *reinterpret_cast<const double2*>(C), c1 = make_double2(0.0, 0.0);
 #pragma unroll 2
   for (int m = 0; m < n; m++) {
     const double a0 = -pa[m * 64], a1 = -pa[m * 64 + 32];
     const double b0 = pb[m * 64], b1 = pb[m * 64 + 32];
     dmma(c, a0, b0);
-    dmma(c, a1, b1);
+    dmma(c1, a1, b1);
   }
+  c.x += c1.x;
+  c.y += c1.y;
   *reinterpret_cast<double2*>(C) = c;
 }
 
