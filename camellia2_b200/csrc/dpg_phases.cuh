@@ -30,7 +30,7 @@ constexpr int NW = DPG_CTA_WARPS;
 constexpr int NT = NW * 32;
 constexpr int CTAS_PER_SM = DPG_NWARPS / NW;
 constexpr int MAX_MBT = NW == DPG_NWARPS ? DPG_MAX_MBT : NW;  // trial tiles: one column tile per warp
-constexpr int MAX_KT = (MAX_MBT * (MAX_MBT + 1) / 2 + NW - 1) / NW;  // lower K_ext tiles per warp
+constexpr int MAX_KB = (MAX_MBT * MAX_MBT / 4 + NW - 1) / NW;  // 16x8 blocks of K_ext per warp (even MAX_MBT)
 constexpr int MBAR_SPIN_LIMIT = 1 << 22;
 constexpr int ERR_TIMEOUT_FLAG = 0x7fff0000;
 constexpr int GEO = 24;  // doubles per point geometry record: J(9) Ji(9) det w*|J| n(3) 1/det
@@ -1122,47 +1122,89 @@ __device__ __forceinline__ void phase_trsm(const DpgPlanDev& P, const DpgLaunch&
 // ---------------------------------------------------------------------------
 // Phase 5/6: K_ext = W^T W, outputs, condensation
 // ---------------------------------------------------------------------------
+// K_ext's lower tiles as 16x8 blocks of the row pairs (r, r + 1), r = 2p + o (o = MBT & 1), by the
+// columns J <= r, and what is left of the diagonal, the 8x8 tiles of every second row: no product is
+// done twice or for padding.  A warp's blocks k0 .. k0 + N - 1 (row by row) and, with SINGLE, the diagonal
+// tile of row I1, then their stores over W^T behind the block barrier.  Bound by the tensor pipe (18.5 K
+// cycles for 14 trial and 22 test tiles).  N and SINGLE are template arguments: with up to nine guarded
+// 8x8 tiles per warp every load waited behind a branch (31 K cycles).  48^3 hexes 144.9 -> 142.1 ms,
+// quads of k = 4 14.27 -> 14.15 ms; two steps of R per pass: 14.45 ms for the latter.
+template <int N, bool SINGLE>
+__device__ __forceinline__ void syrk_blocks(const double* __restrict__ WT, double* KT, int NBT, int o, int k0, int I1,
+                                            int lane) {
+  double acc[N + 1][4];
+  double2 acc1 = make_double2(0.0, 0.0);
+  int ai[N + 1], bj[N + 1];
+  uint32_t newrow = 1;  // bit u: block u is the first of its row pair
+  int p = 0;
+#pragma unroll
+  for (int u = 0; u < N; u++) {
+    while ((p + 1) * (p + 1 + o) <= k0 + u) p++;
+    ai[u] = (2 * p + o) * NBT * 64 + lane;
+    if (k0 + u == p * (p + o)) newrow |= 1u << u;
+    bj[u] = (k0 + u - p * (p + o)) * NBT * 64 + lane;
+#pragma unroll
+    for (int e = 0; e < 4; e++) acc[u][e] = 0.0;
+  }
+  const int row = NBT * 64;
+#pragma unroll 1
+  for (int R = 0; R < NBT; R++, WT += 64) {
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+      if (newrow >> u & 1) {
+        a0 = WT[ai[u]];
+        a1 = WT[ai[u] + row];
+        a2 = WT[ai[u] + 32];
+        a3 = WT[ai[u] + row + 32];
+      }
+      dmma16k8(acc[u], a0, a1, a2, a3, WT[bj[u]], WT[bj[u] + 32]);
+    }
+    if (SINGLE) {
+      const double w0 = WT[I1 * row + lane], w1 = WT[I1 * row + lane + 32];
+      dmma(acc1, w0, w0);
+      dmma(acc1, w1, w1);
+    }
+  }
+  asm volatile("bar.sync 0, %0;" ::"n"(NT) : "memory");
+  const int c = ak_cfrag(lane >> 2, lane & 3);
+  p = 0;
+#pragma unroll
+  for (int u = 0; u < N; u++) {
+    while ((p + 1) * (p + 1 + o) <= k0 + u) p++;
+    const int I = 2 * p + o, J = k0 + u - p * (p + o);
+    *reinterpret_cast<double2*>(KT + (I * (I + 1) / 2 + J) * 64 + c) = make_double2(acc[u][0], acc[u][1]);
+    *reinterpret_cast<double2*>(KT + ((I + 1) * (I + 2) / 2 + J) * 64 + c) = make_double2(acc[u][2], acc[u][3]);
+  }
+  if (SINGLE) *reinterpret_cast<double2*>(KT + (I1 * (I1 + 3) / 2) * 64 + c) = acc1;
+}
+
+// The instance for n blocks (at most N).
+template <int N, bool SINGLE>
+__device__ __forceinline__ void syrk_pick(int n, const double* WT, double* KT, int NBT, int o, int k0, int I1, int lane) {
+  if (n == N) syrk_blocks<N, SINGLE>(WT, KT, NBT, o, k0, I1, lane);
+  else if constexpr (N > 0) syrk_pick<N - 1, SINGLE>(n, WT, KT, NBT, o, k0, I1, lane);
+}
+
+__device__ __forceinline__ void syrk(int w_off, int k_off, int NBT, int MBT) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double* const WT = dpg_smem + w_off;
+  double* const KT = dpg_smem + k_off;
+  // the first warps take the blocks that do not divide evenly, the last ones the diagonal tiles
+  const int o = MBT & 1, np = MBT >> 1, nk = np * (np + o);
+  const int kbase = nk / NW, kextra = nk % NW;
+  const int k0 = warp * kbase + min(warp, kextra), I1 = 2 * (NW - 1 - warp) + 1 - o;
+  const int n = kbase + (warp < kextra ? 1 : 0);
+  if (I1 < MBT) syrk_pick<MAX_KB, true>(n, WT, KT, NBT, o, k0, I1, lane);
+  else syrk_pick<MAX_KB, false>(n, WT, KT, NBT, o, k0, I1, lane);
+}
+
 __device__ __forceinline__ void phase_syrk_out(const DpgPlanDev& P, const DpgLaunch& L, int cell) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
   DPG_SMEM_VIEWS(P);
-  const double* WT = sm + P.sm_w;
   double* KT = sm + P.sm_k;
-  {
-    const int nk = P.MBT * (P.MBT + 1) / 2;
-    const int kbase = nk / NW, kextra = nk % NW;
-    const int k0 = warp * kbase + min(warp, kextra);
-    const int nkw = kbase + (warp < kextra ? 1 : 0);
-    double2 kacc[MAX_KT];
-    int kI[MAX_KT], kJ[MAX_KT];
-#pragma unroll
-    for (int u = 0; u < MAX_KT; u++) {
-      kacc[u] = make_double2(0.0, 0.0);
-      int ij = (u < nkw) ? tri_s[k0 + u] : 0;
-      kI[u] = ij & 255;
-      kJ[u] = ij >> 8;
-    }
-    for (int R = 0; R < P.NBT; R++) {
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        int lastI = -1;
-        double afr = 0.0;
-#pragma unroll
-        for (int u = 0; u < MAX_KT; u++) {
-          if (u < nkw) {
-            if (kI[u] != lastI) { afr = WT[(kI[u] * P.NBT + R) * 64 + h * 32 + lane]; lastI = kI[u]; }
-            double bfr = WT[(kJ[u] * P.NBT + R) * 64 + h * 32 + lane];
-            dmma(kacc[u], afr, bfr);
-          }
-        }
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < MAX_KT; u++)
-      if (u < nkw) *reinterpret_cast<double2*>(KT + (k0 + u) * 64 + ak_cfrag(g, t)) = kacc[u];
-    __syncthreads();
-  }
+  syrk(P.sm_w, P.sm_k, P.NBT, P.MBT);
+  __syncthreads();
   // K and l out (user numbering; fields first: dev = i for i < nf, nfp + (i - nf) otherwise);
   // streaming stores, so the outputs do not evict the CTA's scratch slot from L2
   if (L.K) {

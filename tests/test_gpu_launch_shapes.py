@@ -9,7 +9,10 @@
     (condition below 100, so 1e-12 is a hundred times the rounding of either solve).
   * The scatter plan's staged apply: one dof, an odd S (unaligned cells), dofs shared within a cell, and
     a cell too large to stage, against a dense accumulation (sums of at most a few dozen O(1)
-    products in another order: 1e-13)."""
+    products in another order: 1e-13).
+  * K = B G^-1 B^T for every number of trial tiles (how its blocks are dealt out depends on it) against
+    dense solves: condition below 10, 125 test rows, so 1e-12 is ten times 125 roundings at that
+    condition."""
 import numpy as np
 import pytest
 
@@ -150,3 +153,18 @@ def test_scatter_plan_sizes(C, t, share):
     assert int(plan.missing) == 0
     assert np.abs(values.cpu().numpy() - A[rows, cols]).max() <= 1e-13 * max(1.0, np.abs(A).max())
     assert np.abs(rhs.cpu().numpy() - b).max() <= 1e-13 * max(1.0, np.abs(b).max())
+
+
+@pytest.mark.parametrize("M", [1, 9, 17, 25, 33, 41, 49, 57, 65, 73, 81, 89, 97, 105, 112])
+def test_gram_of_the_solution_for_every_number_of_trial_tiles(M):
+    rng = np.random.default_rng(M)
+    C, N = 5, 125
+    A = rng.standard_normal((C, N, N))
+    G = A @ A.transpose(0, 2, 1) / N + np.eye(N)
+    B, F = rng.standard_normal((C, M, N)), rng.standard_normal((C, N))
+    K, l, info = dlib.factoredCholeskySolve(_dev(G), _dev(B), _dev(F))
+    X = np.linalg.solve(G, np.concatenate([B, F[:, None]], 1).transpose(0, 2, 1))
+    Kx, lx = B @ X[:, :, :M], (B @ X[:, :, M:])[:, :, 0]
+    assert (info.cpu().numpy() == 0).all()
+    assert np.abs(K.cpu().numpy() - Kx).max() <= 1e-12 * np.abs(Kx).max()
+    assert np.abs(l.cpu().numpy() - lx).max() <= 1e-12 * np.abs(Kx).max()
