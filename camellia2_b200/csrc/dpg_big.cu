@@ -38,7 +38,8 @@ static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, i
 // CTAs per cell of a call of C cells, and the clusters that run at once.  With at most half as many
 // cells as SMs the others would idle, so a cluster shares each cell: the size with the least waves x
 // (serial tenth + rest / size), at most half the cell's 64-row blocks (a step's panels and trailing tiles
-// are what is dealt out).  37 Stokes quads of p = 6: 4.98 ms with a CTA per cell, 1.96 ms so.  With more cells than that one CTA per cell is faster: a cluster
+// are what is dealt out).  37 Stokes quads of p = 6: 4.98 ms with a CTA per cell, 1.96 ms so (1.77 ms with
+// today's formation and panels).  With more cells than that one CTA per cell is faster: a cluster
 // reloads a step's panels in every CTA and waits at two cluster barriers per step.
 static int team_size(const DpgPlanDev* plan, int C, KernelFn k, int* clusters) {
   const int sms = dpg::num_sms();

@@ -1,21 +1,24 @@
 // dpg_kernel.cu — fused FP64 per-cell DPG assembly for sm_100a.
 //
-// Persistent CTAs (16 warps, one per SM) walk the cells.  Per cell:
+// Persistent CTAs (16 warps, one per SM; small buckets: 8 warps, two per SM) walk the
+// cells.  Per cell:
 //   1. B and F (TBF::stiffnessMatrix, BF.cpp:575-656; RHS.cpp:68-82).  Volume: the
 //      per-point records (reference slots of the test bases plus each term's trial
-//      values) arrive by bulk (TMA) copy, double buffered; U = (weight x coefficient
-//      x Piola row) x trial value per active (test var, column tile) block, and each
-//      warp accumulates its 16x8 blocks with mma.m16n8k16.f64 over k-steps of 4
+//      values) arrive by bulk (TMA) copy, double buffered; each point's and term's row
+//      (weight x coefficient x Piola row) is formed a chunk ahead, U = row x trial
+//      value per active (test var, column tile) block and column, and each warp accumulates its 16x8 blocks with mma.m16n8k16.f64 over k-steps of 4
 //      points x 4 slots.  Boundary terms with a cell-independent side transform
 //      (HGRAD value; HDIV normal trace by the Piola identity) are separable: compact
 //      per-entry sums over the test rows nonzero on the side.  The tiles wait in a
 //      per-CTA scratch slot (L2-resident).
 //   2. Gram matrix G (IP::computeInnerProductMatrix, IP.cpp:215-292): the same slot
 //      form; per point and coupled test-var pair a 4x4 coupling D = T_a^T C T_b (C:
-//      graph-norm coefficients, T: Piola maps), h = D x slots by DMMA per chunk, and
-//      each warp accumulates its 16x8 blocks of the lower triangle (m16n8k16).
+//      graph-norm coefficients, T: Piola maps), folded into the row operand, and
+//      each warp accumulates its 16x8 blocks of the lower triangle from the staged
+//      slots (m16n8k8, 2D: m16n8k4).
 //   3. Equilibrated Cholesky of G (BF.cpp:944-982: DPOEQU scaling, DPOTRF('L'),
-//      unscaling), blocked right-looking with look-ahead on 8x8 tiles in shared memory.
+//      the solves take the scaled factor), blocked left-looking on 8x8 tiles in shared
+//      memory, the chain of diagonal tiles on a warp of its own.
 //   4. W = L^-1 [B | F] in registers (BF.cpp:987-988, 1013-1014): each warp runs a
 //      blocked forward substitution on its own column tile; diagonal blocks use
 //      precomputed inverses, row pairs update with mma.m16n8k8.f64.

@@ -2,7 +2,7 @@
 //
 // Layout conventions used by the kernels (all FP64):
 //  * Test dofs are stored var by var, each var padded to a multiple of 8
-//    ("test tiles"); trial dofs as [fields | traces | F column], each group padded
+//    ("test tiles"); trial dofs as [fields | traces, F column], each group padded
 //    to a multiple of 8 ("trial tiles").  The F column (the load vector) rides
 //    along as one extra trial column so y = L^-1 F and l = W^T y fall out of the
 //    same triangular solve and Gram product as W and K.

@@ -207,9 +207,9 @@ int dpg_plan_query(const dpg_plan* plan, dpg_plan_info* info);
  * launch shapes to choose).  Times dpg_assemble on the C given cells (DEVICE
  * pointers as for dpg_assemble) with each candidate shape, keeps the faster for
  * all later calls on this plan (dpg_assemble, the multi-bucket launch and its
- * graph) and returns it in *chosen: for single-CTA plans the Gram staging chunk
- * that fits the bucket's shared memory (8 or 4 quadrature points per chunk: it
- * sets the shared-memory layout and the kernel instance), for large-bucket plans
+ * graph) and returns it in *chosen: for single-CTA plans the Gram staging ring
+ * that fits the bucket's shared memory (8: chunks of 16 or 8 quadrature points,
+ * 4: chunks of 4; it sets the shared-memory layout), for large-bucket plans
  * the formation k-chunk (32 or 16 points).  Results of the configurations agree
  * to rounding (sums are ordered differently).  Allocates its timing outputs from
  * the library's pool. */
@@ -376,9 +376,13 @@ int dpg_multi_autotune(int n_buckets, const dpg_bucket_batch* buckets, void* str
  * same buffers).  Capture uploads the bucket tables and allocates the
  * workspace (outside any stream capture of the caller); every launch then
  * reads the buffers named at capture time.  The graph holds the large buckets'
- * launches in decreasing order of cost, then the work queue of the single-CTA
- * buckets (whose counters reset themselves at the end of each launch).  Launches
- * of one graph must not overlap on the GPU (they share the workspace). */
+ * launches and the work queue of the single-CTA buckets (whose counters reset
+ * themselves at the end of each launch) as branches, with priorities in
+ * decreasing order of cost and a workspace for each large bucket, so that one
+ * bucket's CTAs take the SMs that another's last wave leaves idle; where the
+ * workspaces do not fit together, the launches share one and run one after
+ * another.  Launches of one graph must not overlap on the GPU (they share the
+ * workspaces). */
 typedef struct dpg_graph dpg_graph;
 int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags, dpg_graph** out);
 int dpg_graph_launch(dpg_graph* graph, void* stream);
@@ -402,8 +406,8 @@ int dpg_graph_destroy(dpg_graph* graph);
  *   - large-bucket plans (more than 192 test rows or 120 trial columns after
  *     padding) are rejected with DPG_ERR_UNSUPPORTED, and so are buckets whose
  *     per-CTA scratch exceeds 32 MiB; otherwise the launch uses as many CTAs as
- *     fit (floor(32 MiB / per-CTA scratch), at most one per SM): the 3D hex k=2
- *     bucket (298 KiB per CTA) runs on 110 CTAs;
+ *     fit (floor(32 MiB / per-CTA scratch), at most one per SM, two for the
+ *     small buckets): the 3D hex k=2 bucket (286 KiB per CTA) runs on 114 CTAs;
  *   - every call shares the one array: calls that overlap on the GPU (other
  *     streams, other threads, other plans) race and must be serialised by the
  *     caller.  The array keeps the last call's contents; every call writes the
