@@ -66,12 +66,21 @@ static int team_size(const DpgPlanDev* plan, int C, KernelFn k, int* clusters) {
   return best;
 }
 
+static KernelFn team_kernel(const DpgPlanDev* plan) {
+  return plan->big_zk == 16 ? dpg_big_kernel<16, true> : dpg_big_kernel<32, true>;
+}
+
+int dpg_big_team(const DpgPlanDev* plan, int C) {
+  int clusters = 0;
+  return team_size(plan, C, team_kernel(plan), &clusters);
+}
+
 // Large buckets: one CTA per SM, or a cluster per cell, each with its own workspace (Z and the per-point
 // factors).
 int dpg_launch_big(const DpgPlanDev* plan, const DpgLaunch* Lin, cudaStream_t stream) {
   if (Lin->solve_only)
     return dpg::fail(DPG_ERR_UNSUPPORTED, "large-bucket plans support the assembly entry points only");
-  KernelFn kt = plan->big_zk == 16 ? dpg_big_kernel<16, true> : dpg_big_kernel<32, true>;
+  KernelFn kt = team_kernel(plan);
   int grid = 0;  // workspaces: CTAs or clusters
   const int team = team_size(plan, Lin->C, kt, &grid);
   DpgLaunch L = *Lin;

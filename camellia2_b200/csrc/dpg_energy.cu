@@ -8,7 +8,7 @@ namespace {
 int dpg_launch_energy(const DpgPlanDev* plan, const DpgLaunch* Lin, cudaStream_t stream) {
   if (Lin->C <= 0) return DPG_OK;
   if (plan->big) return dpg_launch_big(plan, Lin, stream);  // energy error or DLS output
-  DpgKernelChoice kc = dpg_small_kernel(plan, Lin->xsol ? DPG_KIND_ENERGY : DPG_KIND_DLS);
+  DpgKernelChoice kc = dpg_small_kernel(plan, Lin->xsol ? DPG_KIND_ENERGY : DPG_KIND_DLS, Lin->C);
   if (!kc.k) kc = DpgKernelChoice{Lin->xsol ? pick_energy_kernel(plan) : pick_dls_kernel(plan), NT, 1};
   KernelFn k = kc.k;
   if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no kernel instance for this bucket size");

@@ -1747,6 +1747,17 @@ int dpg_plan_autotune(dpg_plan* p, int C, const double* nodes, const int8_t* par
   return DPG_OK;
 }
 
+// Launch shape of a call of C cells (kind: DPG_KIND_*), for tests: warps per CTA, CTAs per SM, CTAs per cell.
+int dpg_debug_launch_shape(const dpg_plan* p, int kind, int C, int* warps, int* per_sm, int* per_cell) {
+  if (!p || C <= 0 || !warps || !per_sm || !per_cell) return fail(DPG_ERR_INVALID_ARGUMENT, "bad shape query");
+  const DpgPlanDev& g = p->hp.dev;
+  const bool small = !g.big && dpg_small_kernel(&g, kind, C).k;
+  *warps = small ? DPG_SMALL_WARPS : DPG_NWARPS;
+  *per_sm = small ? 2 : 1;
+  *per_cell = g.big ? dpg_big_team(&g, C) : 1;
+  return DPG_OK;
+}
+
 int dpg_assemble_noalloc(dpg_plan* p, int C, const double* nodes, const int8_t* parity, const double* coeff,
                          double* K, double* l, double* S, double* s, int32_t* info, void* stream, int flags) {
   if (!p) return fail(DPG_ERR_BAD_PLAN, "null plan");

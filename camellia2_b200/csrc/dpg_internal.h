@@ -59,12 +59,13 @@ struct DpgKernelChoice {
   int threads, per_sm;
 };
 enum { DPG_KIND_ASSEMBLE, DPG_KIND_ADJOINT, DPG_KIND_ENERGY, DPG_KIND_DLS };
-DpgKernelChoice dpg_small_kernel(const DpgPlanDev* plan, int kind);  // k null: not a small bucket
+DpgKernelChoice dpg_small_kernel(const DpgPlanDev* plan, int kind, int C);  // k null: the 16-warp kernels run these C cells
 
 int dpg_configure_kernels(const DpgPlanDev* plan);
 int dpg_configure_adjoint(const DpgPlanDev* plan, int bytes);
 int dpg_configure_big(const DpgPlanDev* plan);
 int dpg_launch_big(const DpgPlanDev* plan, const DpgLaunch* L, cudaStream_t stream);
+int dpg_big_team(const DpgPlanDev* plan, int C);  // CTAs per cell of a call of C cells
 int dpg_launch_assemble(const DpgPlanDev* plan, const DpgPlanDev* d_plan, const DpgLaunch* L, cudaStream_t stream);
 int dpg_host_pipeline(const DpgPlanDev* plan, const DpgPlanDev* d_plan, void** d_ws, size_t* ws_bytes,
                       cudaStream_t* streams, int C, const double* nodes, const int8_t* parity, const double* coeff,

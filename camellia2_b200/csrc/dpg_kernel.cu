@@ -30,6 +30,8 @@
 // reverse mode, the energy error and the multi-bucket launch reuse these phases.
 #include "dpg_phases.cuh"
 
+#include <climits>
+
 namespace {
 
 #include "dpg_cell.cuh"
@@ -92,18 +94,15 @@ cudaError_t ws_alloc(void** p, size_t bytes, cudaStream_t s) {
 }
 }  // namespace dpg
 
-// The small buckets run two CTAs per SM.
-static DpgKernelChoice choose_kernel(const DpgPlanDev* plan) {
-  DpgKernelChoice c = dpg_small_kernel(plan, DPG_KIND_ASSEMBLE);
+// The small buckets run two CTAs per SM when there are cells for them.
+static DpgKernelChoice choose_kernel(const DpgPlanDev* plan, int C) {
+  DpgKernelChoice c = dpg_small_kernel(plan, DPG_KIND_ASSEMBLE, C);
   if (!c.k) c = DpgKernelChoice{pick_kernel(plan), NT, 1};
   return c;
 }
 
 int dpg_configure_kernels(const DpgPlanDev* plan) {
   if (plan->big) return dpg_configure_big(plan);
-  const DpgKernelChoice kc = choose_kernel(plan);
-  KernelFn k = kc.k;
-  if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no kernel instance for this bucket size");
   // Several plans may share a kernel instance: the opt-in limit is the device's
   // maximum, so configuring one plan never lowers another's.
   int dev = 0, optin = 0;
@@ -112,10 +111,15 @@ int dpg_configure_kernels(const DpgPlanDev* plan) {
   size_t bytes = (size_t)plan->sm_total * sizeof(double);
   if (optin > 0 && bytes > (size_t)optin) return dpg::fail(DPG_ERR_UNSUPPORTED, "bucket needs more shared memory than one CTA has");
   if (optin > 0) bytes = (size_t)optin;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess && kc.per_sm > 1)
-    e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+  for (int C : {1, INT_MAX}) {  // few cells, many cells
+    const DpgKernelChoice kc = choose_kernel(plan, C);
+    KernelFn k = kc.k;
+    if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no kernel instance for this bucket size");
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && kc.per_sm > 1)
+      e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return dpg::fail(DPG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+  }
   return plan->adj_ok ? dpg_configure_adjoint(plan, (int)bytes) : DPG_OK;
 }
 
@@ -123,7 +127,7 @@ int dpg_launch_assemble(const DpgPlanDev* plan, const DpgPlanDev* d_plan, const 
   (void)d_plan;
   if (Lin->C <= 0) return DPG_OK;
   if (plan->big) return dpg_launch_big(plan, Lin, stream);
-  const DpgKernelChoice kc = choose_kernel(plan);
+  const DpgKernelChoice kc = choose_kernel(plan, Lin->C);
   KernelFn k = kc.k;
   if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no kernel instance for this bucket size");
   const int grid = std::min(Lin->C, dpg::num_sms() * kc.per_sm);
@@ -488,7 +492,7 @@ unsigned long long current_context_id() {
 int dpg_launch_assemble_noalloc(const DpgPlanDev* plan, const DpgLaunch* Lin, cudaStream_t stream) {
   if (Lin->C <= 0) return DPG_OK;
   if (plan->big) return dpg::fail(DPG_ERR_UNSUPPORTED, "dpg_assemble_noalloc: large-bucket plans need dpg_assemble");
-  const DpgKernelChoice kc = choose_kernel(plan);
+  const DpgKernelChoice kc = choose_kernel(plan, Lin->C);
   KernelFn k = kc.k;
   if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no kernel instance for this bucket size");
   if (plan->scratch_per_cta > DPG_NOALLOC_SCRATCH_DOUBLES)

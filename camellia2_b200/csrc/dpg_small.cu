@@ -17,9 +17,14 @@ namespace {
 #include "dpg_energy.cuh"
 }  // namespace
 
-DpgKernelChoice dpg_small_kernel(const DpgPlanDev* plan, int kind) {
+DpgKernelChoice dpg_small_kernel(const DpgPlanDev* plan, int kind, int C) {
   DpgKernelChoice c{nullptr, NT, CTAS_PER_SM};
   if (!plan->small) return c;
+  // Up to as many cells as SMs: a cell has its SM to itself, so 16 warps finish it sooner.  1..148 CDR quads of
+  // k = 3 (13 test tiles), 8 -> 16 warps: assembly 102 -> 83 us, parts 98 -> 70, DLS 100 -> 79, reverse mode
+  // 317 -> 245; Poisson quads of k = 1 (4 tiles): assembly 36 -> 34 us, reverse mode 44.4 -> 44.4..46.  With one
+  // cell more, 16 warps take a second wave: 122 against 160 us for 149 Poisson quads of k = 3 (13 tiles).
+  if (C <= dpg::num_sms()) return c;
   switch (kind) {
     case DPG_KIND_ASSEMBLE: c.k = pick_kernel(plan); break;
     case DPG_KIND_ADJOINT: c.k = pick_adjoint_kernel(plan); break;
