@@ -650,8 +650,16 @@ static int smem_layout_stages(DpgPlanDev& g, int chg, int stages, bool adj_terms
     g.a_geo = q; q += al(std::max(DPG_CHA_HOST, g.ns * g.QS) * 24);
     g.a_beta = q; q += al(DPG_CHA_HOST * g.niprows * 4 * g.ntest);
     g.a_cbar = q; q += al(std::max(1, g.nslots * g.Ptot));
-    const int ngt16 = g.nbt16 * (g.nbt16 + 1) / 2;
-    const int body16 = std::max(std::max(body, g.MBT * g.nbt16 * 64), (ngt16 + g.nbt16) * 64 + g.nbt16 * 8);
+    // The reverse mode is offered where its staging fits the space that the phases take with every var padded to
+    // 16 rows, F in a tile of its own and the Gram phase's tables side by side.  The space that the phases do
+    // take is no measure: for a few test dofs (Stokes quads k = 1, dk = 0: 20) it is less than the staging.
+    const int ngt16 = g.nbt16 * (g.nbt16 + 1) / 2, mbt8 = (g.nfp + g.ntp + 8) / 8, qg8 = (g.QG + 7) & ~7;
+    const int ch8 = std::min(chg, DPG_CHG);
+    int hs = 0;  // slots of the coupled pairs' column vars
+    for (int p = 0; p < g.npairs; p++) hs += 4 * g.test[g.pair_b[p]].ldA;
+    const int gram16 = 2 * al(ch8 * (g.featstride - 4)) + al(std::max(ch8 * hs, qg8 * g.niprows * 4 * g.ntest)) +
+                       al(qg8 * 24) + al(qg8 * g.npairs * 16);
+    const int body16 = std::max(std::max(std::max(body, gram16), mbt8 * g.nbt16 * 64), (ngt16 + g.nbt16) * 64 + g.nbt16 * 8);
     // a small layout makes room for the reverse mode wherever the full one has it
     g.adj_ok = g.small ? g.adj_ok : adj_terms_ok && std::max(sa_end, q) <= body16 && g.QB > 0;
     if (g.adj_ok) body = std::max(body, std::max(sa_end, q));
