@@ -1071,7 +1071,7 @@ __device__ __forceinline__ void solve_update(const double* __restrict__ GT, int 
     if (r <= k) continue;
     const double* Lik = GT + (r * (r + 1) / 2 + k) * 64;
     const double* Ln = GT + ((r + 1) * (r + 2) / 2 + k) * 64;
-    if (r + 1 < NBT) {
+    if (r + 1 < NBTM && r + 1 < NBT) {  // (an odd NBTM has no pair at its end)
       dmma16x8(y[r], y[r + 1], Lik[lane], Ln[lane], Lik[32 + lane], Ln[32 + lane], x0, x1);
     } else if (r < NBT) {
       dmma(y[r], Lik[lane], x0);
