@@ -683,14 +683,11 @@ static int smem_layout_stages(DpgPlanDev& g, int chg, int stages, bool adj_terms
   return DPG_OK;
 }
 
-// The largest ring that fits: 16-point chunks in two stages or 8-point ones in four or two (chg 8), 4-point
-// ones (chg 4).  A chunk costs its warps ~1 K cycles of barrier and parameter reads whatever its size.
+// The largest ring that fits: two 16- or 8-point chunks (chg 8), four or two 4-point chunks (chg 4).  A chunk costs
+// its warps ~1 K cycles of barrier and parameter reads whatever its size.  (Four 8-point chunks take as much
+// room as two 16-point ones, unless beta is larger than two of them: no bucket of the formulations.)
 static int smem_layout(DpgPlanDev& g, int chg, bool adj_terms_ok) {
-  if (chg == DPG_CHG) {
-    const int rc = smem_layout_stages(g, 2 * DPG_CHG, 2, adj_terms_ok);
-    if (rc != -1) return rc;
-  }
-  const int rc = smem_layout_stages(g, chg, 4, adj_terms_ok);
+  const int rc = chg == DPG_CHG ? smem_layout_stages(g, 2 * chg, 2, adj_terms_ok) : smem_layout_stages(g, chg, 4, adj_terms_ok);
   return rc != -1 ? rc : smem_layout_stages(g, chg, 2, adj_terms_ok);
 }
 
@@ -1697,6 +1694,14 @@ int dpg_assemble(dpg_plan* p, int C, const double* nodes, const int8_t* parity, 
   return dpg_launch_assemble(&p->hp.dev, p->hp.d_dev, &L, (cudaStream_t)stream);
 }
 
+// A plan of another launch shape takes the place of p's own.
+static int adopt(dpg_plan* p, const DpgPlanDev& g) {
+  p->hp.dev = g;
+  if (cudaMemcpy(p->hp.d_dev, &p->hp.dev, sizeof(DpgPlanDev), cudaMemcpyHostToDevice) != cudaSuccess)
+    return fail(DPG_ERR_CUDA, "plan upload");
+  return dpg_configure_kernels(&p->hp.dev);
+}
+
 int dpg_plan_autotune(dpg_plan* p, int C, const double* nodes, const int8_t* parity, const double* coeff, void* stream,
                       int* chosen) {
   if (!p) return fail(DPG_ERR_BAD_PLAN, "null plan");
@@ -1746,24 +1751,32 @@ int dpg_plan_autotune(dpg_plan* p, int C, const double* nodes, const int8_t* par
   cudaFreeAsync(out, st);
   if (rc != DPG_OK) return rc;
   if (best < 0.0f) return fail(DPG_ERR_UNSUPPORTED, "no Gram chunk size fits this bucket");
-  p->hp.dev = best_plan;
-  if (cudaMemcpy(p->hp.d_dev, &p->hp.dev, sizeof(DpgPlanDev), cudaMemcpyHostToDevice) != cudaSuccess)
-    return fail(DPG_ERR_CUDA, "plan upload");
-  rc = dpg_configure_kernels(&p->hp.dev);
-  if (rc != DPG_OK) return rc;
+  if ((rc = adopt(p, best_plan)) != DPG_OK) return rc;
   *chosen = p->hp.dev.big ? p->hp.dev.big_zk : std::min(p->hp.dev.chg, DPG_CHG);
   return DPG_OK;
 }
 
-// Launch shape of a call of C cells (kind: DPG_KIND_*), for tests: warps per CTA, CTAs per SM, CTAs per cell.
-int dpg_debug_launch_shape(const dpg_plan* p, int kind, int C, int* warps, int* per_sm, int* per_cell) {
-  if (!p || C <= 0 || !warps || !per_sm || !per_cell) return fail(DPG_ERR_INVALID_ARGUMENT, "bad shape query");
+// For tests: the launch shape of a call of C cells (kind: DPG_KIND_*): warps per CTA, CTAs per SM, CTAs per cell, and the
+// Gram ring's points per chunk and stages (0 for large plans).
+int dpg_debug_launch_shape(const dpg_plan* p, int kind, int C, int* out) {
+  if (!p || C <= 0 || !out) return fail(DPG_ERR_INVALID_ARGUMENT, "bad shape query");
   const DpgPlanDev& g = p->hp.dev;
   const bool small = !g.big && dpg_small_kernel(&g, kind, C).k;
-  *warps = small ? DPG_SMALL_WARPS : DPG_NWARPS;
-  *per_sm = small ? 2 : 1;
-  *per_cell = g.big ? dpg_big_team(&g, C) : 1;
+  out[0] = small ? DPG_SMALL_WARPS : DPG_NWARPS;
+  out[1] = small ? 2 : 1;
+  out[2] = g.big ? dpg_big_team(&g, C) : 1;
+  out[3] = g.chg;
+  out[4] = g.gstages;
   return DPG_OK;
+}
+
+// For tests: the choice of dpg_plan_autotune for a single-CTA plan (8 or 4) without its timing.
+int dpg_debug_set_gram_chunk(dpg_plan* p, int chunk) {
+  if (!p || p->hp.dev.big || (chunk != DPG_CHG && chunk != DPG_CHG / 2)) return fail(DPG_ERR_INVALID_ARGUMENT, "bad chunk");
+  DpgPlanDev cand = p->hp.dev;
+  const int rc = smem_layout(cand, chunk, p->hp.adj_terms_ok);
+  if (rc != DPG_OK) return rc == -1 ? fail(DPG_ERR_UNSUPPORTED, "the chunk does not fit") : rc;
+  return adopt(p, cand);
 }
 
 int dpg_assemble_noalloc(dpg_plan* p, int C, const double* nodes, const int8_t* parity, const double* coeff,

@@ -18,10 +18,9 @@ ASSEMBLE, ADJOINT, ENERGY, DLS = range(4)
 
 def shape(plan, kind, C):
     """(warps per CTA, CTAs per SM, CTAs per cell) of a call."""
-    w, s, c = ct.c_int(), ct.c_int(), ct.c_int()
-    rc = dlib.load().dpg_debug_launch_shape(plan.h, kind, C, ct.byref(w), ct.byref(s), ct.byref(c))
-    assert rc == 0
-    return w.value, s.value, c.value
+    out = (ct.c_int * 5)()
+    assert dlib.load().dpg_debug_launch_shape(plan.h, kind, C, out) == 0
+    return tuple(out[:3])
 
 
 def _dev(x):
