@@ -2033,7 +2033,8 @@ struct dpg_graph {
   void* big_ws = nullptr;  // workspaces of the large-bucket launches
 };
 
-int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags, dpg_graph** out) {
+// ws_limit: the most bytes that the large buckets' workspaces may take together.
+static int capture(int n_buckets, const dpg_bucket_batch* buckets, int flags, size_t ws_limit, dpg_graph** out) {
   if (!out) return fail(DPG_ERR_INVALID_ARGUMENT, "null output handle");
   *out = nullptr;
   std::vector<DpgPlanDev> plans, bp;
@@ -2066,7 +2067,7 @@ int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags,
     rc = dpg_launch_multi(plans.data(), ls.data(), (int)plans.size(), nullptr, &G->dev, claim_of(flags));
   }
   bool branches = true;
-  if (rc == DPG_OK && big_bytes > 0 && cudaMalloc(&G->big_ws, big_bytes) != cudaSuccess) {
+  if (rc == DPG_OK && big_bytes > 0 && (big_bytes > ws_limit || cudaMalloc(&G->big_ws, big_bytes) != cudaSuccess)) {
     cudaGetLastError();
     branches = false;
     if (cudaMalloc(&G->big_ws, big_most) != cudaSuccess) {
@@ -2138,6 +2139,15 @@ int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags,
   }
   *out = G;
   return DPG_OK;
+}
+
+int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags, dpg_graph** out) {
+  return capture(n_buckets, buckets, flags, SIZE_MAX, out);
+}
+
+// For tests: dpg_graph_capture on a device whose memory holds one shared workspace of the large buckets only.
+int dpg_debug_graph_capture_shared(int n_buckets, const dpg_bucket_batch* buckets, int flags, dpg_graph** out) {
+  return capture(n_buckets, buckets, flags, 0, out);
 }
 
 int dpg_graph_launch(dpg_graph* G, void* stream) {
