@@ -226,7 +226,7 @@ __device__ void big_prep(const DpgPlanDev& P, const DpgLaunch& L, int cell, cons
 }
 
 // One formation tile.  kind 0: G rows r0.., columns c0.. (test rows); kind 1: E^T rows
-// (device trial columns) r0.., columns c0.. (test rows).
+// (device trial columns) r0.., columns c0.. (test rows), without the F row (big_load_row).
 template <int ZK>
 __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, int kind, int r0, int c0, bool diag, double* Z,
                               const BigSm& S, const double* wq, const double* bh, const double* vt) {
@@ -256,7 +256,7 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
         if (in) {
           const int4 be = P.be[e];
           const DpgBTerm& Tm = P.bterm[P.seg[be.x].term0 + be.y];
-          in = ((mc >> Tm.test_var) & 1) && Tm.col0 < r0 + ZT && Tm.col0 + Tm.ncol > r0;
+          in = Tm.kind >= 0 && ((mc >> Tm.test_var) & 1) && Tm.col0 < r0 + ZT && Tm.col0 + Tm.ncol > r0;
           if (in) w = be.w;
         }
         const unsigned m = __ballot_sync(0xffffffffu, in);
@@ -478,10 +478,52 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int j = r0 + wr + g + h * 8, i = c0 + wc + nb * 8 + 2 * t;
-        if (j < P.Mp && i < P.Np)
+        if (j < P.Mp && i < P.Np && j != P.fcol)
           *reinterpret_cast<double2*>(Z + (size_t)(P.Np + j) * ld + i) =
               make_double2(acc[nb][2 * h] * S.sc[i], acc[nb][2 * h + 1] * S.sc[i + 1]);
       }
+  }
+}
+
+// The F row of E^T in blocks of 64 test rows; eight threads per row take every eighth point, their sums are joined in
+// order.  The products of a tile meet every entry with every row, zeros included: a load that is not finite must
+// not share them with B, nor a side of zero length with F.  (Not inlined: the 32 values in flight would
+// spill in the cell's body.)
+__device__ __noinline__ void big_load_row(const DpgPlanDev& P, double* row, const int* col, const double* sc, const double* vt,
+                                          double* red, int first, int step) {
+  const double* const rec = P.seg[0].rec;
+  const int rl = P.seg[0].rec_len, part = threadIdx.x >> 6, lr = threadIdx.x & 63;
+  for (int b = first, k = 0; b * ZT < P.Np; b += step, k ^= NT) {
+    const int i = b * ZT + lr, c = i < P.Np ? col[i] : -1;
+    double f = 0.0;
+    for (int e = 0; e < P.nle; e++) {
+      const int4 E = P.le[e];
+      if (c < 0 || E.w >> 24 != c >> 16) continue;
+      const double* const r = rec + E.x + (c & 0xffff);
+      const double* const v = vt + (size_t)(E.w & 0xffffff) * 4;
+#pragma unroll 1
+      for (int q0 = part; q0 < E.z; q0 += 64) {  // all loads of eight points in flight: no branch between them
+        double x[8][4];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+#pragma unroll
+          for (int m = 0; m < 4; m++) x[u][m] = __ldg(r + (size_t)min(q0 + 8 * u, E.z - 1) * rl + m * E.y);
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const int q = min(q0 + 8 * u, E.z - 1);
+          const double2 a = *reinterpret_cast<const double2*>(v + q * 4), d = *reinterpret_cast<const double2*>(v + q * 4 + 2);
+          const double g = a.x * x[u][0] + a.y * x[u][1] + d.x * x[u][2] + d.y * x[u][3];
+          f += q0 + 8 * u < E.z ? g : 0.0;
+        }
+      }
+    }
+    red[k + threadIdx.x] = f;  // two buffers, one barrier per block
+    __syncthreads();
+    if (part == 0 && i < P.Np) {
+#pragma unroll
+      for (int p = 1; p < NT / ZT; p++) f += red[k + p * ZT + lr];
+      row[i] = f * sc[i];
+    }
   }
 }
 
@@ -793,6 +835,7 @@ __device__ __forceinline__ void big_cell_body(const DpgPlanDev& P, const DpgLaun
       for (int I = 0; I < nbg; I++)
         if (!TEAM || deal++ % team.size == team.rank)
           big_form_tile<ZK>(P, fail, nullptr, 1, J * ZT, I * ZT, false, Z, S, wq, bh, vt);
+    big_load_row(P, Z + (size_t)(Np + P.fcol) * ld, S.col, S.sc, vt, S.fa, team.rank, team.size);
     if (TEAM) big_sync<TEAM>();
     if (L.parts) {
       // G (N, N), B (M, N) and F (N) in user numbering: Z unscaled (dpg_assemble_parts)

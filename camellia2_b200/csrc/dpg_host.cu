@@ -559,10 +559,13 @@ static int big_layout(HostPlan* P) {
     for (int e = g.rowstart[r]; e < g.rowstart[r + 1]; e++) g.ipmask[r] |= 1 << (g.ipent[e].gslot >> 2);
   }
   int vrow = 0;
-  g.nbe = 0;
+  g.nbe = g.nle = 0;
   for (int sg = 0; sg < g.nseg; sg++)
     for (int lt = 0; lt < g.seg[sg].nterm; lt++) {
       g.be[g.nbe++] = make_int4(sg, lt, vrow, g.seg[sg].npts);
+      const DpgBTerm& t = g.bterm[g.seg[sg].term0 + lt];
+      if (t.kind < 0)  // the load: volume terms, so segment 0
+        g.le[g.nle++] = make_int4(g.test[t.test_var].foff, g.test[t.test_var].ldA, g.seg[sg].npts, vrow | t.test_var << 24);
       vrow += g.seg[sg].npts;
     }
   std::vector<int> u2d(g.M, 0);

@@ -221,6 +221,8 @@ struct DpgPlanDev {
   int Zn, ldz;              // Z order (Np + Mp) and row stride (doubles)
   int nbe;                  // E-formation entries, one per (segment, term)
   int4 be[DPG_MAX_BF];      // (segment, segment-local term, first vt row, points)
+  int nle;                  // load entries: test var's slots in a record, their stride, points, first vt row | test var << 24
+  int4 le[DPG_MAX_RHS];
   int ipmask[DPG_MAX_IPROWS];  // test vars each IP row touches (bit a)
   const int* u2d_trial;     // [M] user trial index -> device column
   const int* u2d_test;      // [N] user test index -> device row
