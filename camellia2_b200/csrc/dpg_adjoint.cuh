@@ -1,5 +1,5 @@
-// dpg_adjoint.cuh — reverse mode of the per-cell assembly (included by dpg_kernel.cu
-// inside its anonymous namespace; it reuses the forward phases defined there).
+// dpg_adjoint.cuh — reverse mode of the per-cell assembly (included by dpg_adjoint.cu and, for 8 warps, by
+// dpg_small.cu inside their anonymous namespaces; it reuses the forward phases of dpg_phases.cuh).
 //
 // For a loss J(K, l) with Kbar = dJ/dK and lbar = dJ/dl (no counterpart in the
 // reference; the forward is TBF::localStiffnessMatrixAndRHS, BF.cpp:1385-1449):

@@ -35,12 +35,17 @@ static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, i
   cfg.numAttrs = 1;
 }
 
-// CTAs per cell of a call of C cells, and the clusters that run at once.  With at most half as many
-// cells as SMs the others would idle, so a cluster shares each cell: the size with the least waves x
-// (serial tenth + rest / size), at most half the cell's 64-row blocks (a step's panels and trailing tiles
-// are what is dealt out).  37 Stokes quads of p = 6: 4.98 ms with a CTA per cell, 1.96 ms so (1.77 ms with
-// today's formation and panels).  With more cells than that one CTA per cell is faster: a cluster
-// reloads a step's panels in every CTA and waits at two cluster barriers per step.
+// CTAs per cell of a call of C cells, and the clusters that run at once.  With at most half as many cells as SMs the
+// others would idle, so a cluster shares each cell: the size with the least waves x (serial tenth + rest / size),
+// at most half the cell's 64-row blocks (a step's panels and trailing tiles are what is dealt out).  ms of a
+// call, one CTA per cell -> the size chosen; in brackets the fastest of all sizes where it is another:
+//   Stokes quads p = 6      10 cells 3.95 -> 0.85 (8)  37: 4.02 -> 1.79 (3)  60: 4.05 -> 2.46 (2)  74: 4.08 -> 2.49 (2)
+//   Stokes quads p = 4      37: 1.36 -> 0.67 (3)  60: 1.37 -> 0.85 (2)  74: 1.37 -> 0.85 (2)
+//   Stokes triangles p = 4  10: 0.50 -> 0.28 (3) [0.23 (8)]  37: 0.51 -> 0.28 (3)  74: 0.51 -> 0.38 (2)
+//   3D Poisson hexes k = 3  10: 2.43 -> 0.75 (5) [0.56 (8)]  37: 2.49 -> 1.08 (3)  74: 2.50 -> 1.48 (2)
+// Beyond half the SMs clusters lose where one wave of CTAs holds the cells (quads p = 6, best cluster: 100 cells 4.14
+// -> 4.72, 148: 4.27 -> 4.95: a cluster reloads a step's panels in every CTA and waits at two barriers per step), and
+// would win where the last wave is nearly empty (75: 4.08 -> 3.54, 200: 8.32 -> 7.36); those keep one CTA.
 static int team_size(const DpgPlanDev* plan, int C, KernelFn k, int* clusters) {
   const int sms = dpg::num_sms();
   *clusters = std::min(C, sms);

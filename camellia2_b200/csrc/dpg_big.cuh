@@ -1,8 +1,8 @@
-// dpg_big.cuh — large buckets (N > 192 or M > 120 after padding), included by dpg_kernel.cu.
+// dpg_big.cuh — large buckets (N > 192 or M > 120 after padding), included by dpg_big.cu.
 //
-// One persistent CTA (16 warps) per SM walks the cells.  A cell's matrices do not fit in
-// shared memory, so each CTA owns a workspace in global memory (L2-resident for the
-// smaller buckets) holding the lower triangle of
+// One persistent CTA (16 warps) per SM walks the cells, or, with few cells, a cluster of CTAs takes each.
+// A cell's matrices do not fit in shared memory, so each CTA or cluster owns a workspace in global memory
+// (L2-resident for the smaller buckets) holding the lower triangle of
 //
 //     Z = [[ S G S , S E ],        E = [B^T | F]  (N x (M + 1), device trial order),
 //          [ E^T S ,  0  ]]        S = diag(G_ii^-1/2)  (DPOEQU scaling, BF.cpp:944-960)
@@ -15,7 +15,7 @@
 //      w|J| L_r(v_i) L_r(v_j) over the points and the IP rows r touching both tiles'
 //      test vars (IP::computeInnerProductMatrix, IP.cpp:215-292); an E tile sums trial value x
 //      test-operator value over the points of every segment and term touching the tile
-//      (TBF::stiffnessMatrix, BF.cpp:575-656; RHS.cpp:68-82).  The diagonal G tiles come
+//      (TBF::stiffnessMatrix, BF.cpp:575-656), the load's row is summed apart (RHS.cpp:68-82).  The diagonal G tiles come
 //      first and give the scales S.
 //   3. Np steps of a blocked right-looking Cholesky: the 64 x 64 diagonal block is factored in
 //      shared memory as 8 x 8 tiles (the single-CTA kernel's tile Cholesky) and inverted by block
@@ -24,7 +24,8 @@
 //      (DSYRK, BF.cpp:993-1005).  The trailing block is then -E^T G^-1 E = -[[K, l], [l^T, .]].
 //   4. K, l are written out, the trailing block is negated, and nfp more steps over the field
 //      columns leave [S s] = the Schur complement (CondensedDofInterpreter.cpp:1138-1192).
-// No step waits on another CTA or on an asynchronous copy.
+// A CTA waits on the CTAs of its own cluster (cluster barriers: they are resident together) and on its own
+// asynchronous copies (cp.async groups), on nothing else.
 
 constexpr int ZT = 64;  // tile edge
 constexpr int ZL = 68;  // shared row stride, == 4 (mod 16) doubles: conflict-free DMMA fragments

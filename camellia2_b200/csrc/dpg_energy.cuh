@@ -1,6 +1,6 @@
 // dpg_energy.cuh — per-cell energy error of a trial solution and the DLS local
-// matrices (included by dpg_kernel.cu inside its anonymous namespace; both reuse
-// the forward phases).
+// matrices (included by dpg_energy.cu and, for 8 warps, by dpg_small.cu inside their
+// anonymous namespaces; both reuse the forward phases of dpg_phases.cuh).
 //
 // TSolution::rankLocalEnergyError (Solution.cpp:2653-2684) with the error
 // representation of computeErrorRepresentation (Solution.cpp:2688-2722): for the

@@ -449,8 +449,8 @@ extern "C" int dpg_debug_wait_probe(int limit, int* status_dev, void* stream) {
 // ---------------------------------------------------------------------------
 // Allocation-free launch: the per-CTA scratch comes from a fixed device array
 // instead of a stream-ordered allocation.  32 MiB (4 Mi doubles): the 3D hex k=2
-// bucket needs 298 KiB per CTA (B tiles 165 KiB, Gram running sums 133 KiB), so
-// 110 CTAs fit; smaller buckets run one CTA per SM.
+// bucket needs 286 KiB per CTA (B tiles 154 KiB, Gram running sums 132 KiB), so
+// 114 CTAs fit; smaller buckets run one CTA per SM, or two of 8 warps.
 // ---------------------------------------------------------------------------
 #define DPG_NOALLOC_SCRATCH_DOUBLES ((size_t)4 << 20)
 

@@ -330,9 +330,8 @@ __device__ __forceinline__ void factor_diag(const double* __restrict__ T, int k,
 // A_i,k+1 -= sum_{j <= k} L_ij L_k+1,j^T at once, each tile in one warp's registers.  A
 // right-looking update reads and writes every trailing tile in every step (7.4 K cycles for
 // the first step of 22 tiles, a dozen warps each waiting on load, two products and store per
-// tile); here a tile is loaded and stored once, its products follow one another in the
-// same order (the same sums), and the work of a step stays below the time of the diagonal tile
-// next door.  That chain of diagonal tiles is what bounds the factorisation: warp 0 does
+// tile); here a tile is loaded and stored once, its products run in two chains joined at the
+// end, and the work of a step stays below the time of the diagonal tile next door.  That chain of diagonal tiles is what bounds the factorisation: warp 0 does
 // nothing else, with its sub-partition to itself (warps 4, 8, 12 only keep the barriers), and it
 // needs from the others only the sum over j < k of tile (k+1, k+1), formed a step ahead.
 constexpr int CHOL_NW = NW - NW / 4;  // warps that update: those of the other sub-partitions
@@ -761,9 +760,7 @@ __device__ __forceinline__ void gram_step2d(const double* __restrict__ f, const 
 // is the parity of the next first use of ring stage i.
 enum { GP_CHG, GP_QG, GP_RING, GP_STAGE, GP_STAGES, GP_FLUSH, GP_D, GP_NGB, GP_TILES, GP_FS, GP_DS, GP_GT, GP_PAR, GP_N };
 
-// The Gram chunk loop.  (The earlier form wrote D x slots of every column tile to shared memory before
-// the products: two block barriers per chunk and 30 K of the phase's 165 K cycles on the 48^3
-// hex workload.)  The chunks travel through a ring of stages: warps arrive on a stage's empty
+// The Gram chunk loop.  The chunks travel through a ring of stages: warps arrive on a stage's empty
 // mbarrier and warp 0 refills it while the next chunk is worked on, so no block barrier is left in
 // the loop and the warps drift apart by up to a ring.  Every GP_FLUSH chunks (except after the last)
 // each thread adds the accumulators of its flushed blocks (P.gflushmask) into its own running sums

@@ -226,8 +226,9 @@ struct DpgPlanDev {
   int ipmask[DPG_MAX_IPROWS];  // test vars each IP row touches (bit a)
   const int* u2d_trial;     // [M] user trial index -> device column
   const int* u2d_test;      // [N] user test index -> device row
-  int bz_wq, bz_bh, bz_vt, bz_sc;  // per-CTA workspace after Z (bz_sc: a cluster's shared scales and flags): w|J| at Gram points, per-point IP row
-                            // factors [QG][rows][ntest][4], per-point term factors [vt rows][4]
+  int bz_wq, bz_bh, bz_vt, bz_sc;  // per-CTA (or per-cluster) workspace after Z: w|J| at Gram points, per-point IP row
+                            // factors [QG][rows][ntest][4], per-point term factors [vt rows][4], a cluster's
+                            // shared scales and flags
   size_t bz_per_cta;        // doubles of per-CTA workspace
   int big_zk;               // formation k-chunk (16 or 32 points; dpg_plan_autotune picks it)
   int bs_sc, bs_col, bs_int, bs_nodes, bs_total;  // shared memory (doubles): scales, column

@@ -25,7 +25,7 @@ __device__ __forceinline__ void queue_leave(int* counters) {
   }
 }
 
-// Multi-bucket work queue of the single-CTA plans: the buckets' cell ranges are
+// Multi-bucket work queue of the single-CTA plans, 16 warps per CTA whatever the bucket: the buckets' cell ranges are
 // concatenated in decreasing order of per-cell cost (the host orders them), and each CTA
 // claims `claim` consecutive cells at a time from a device counter, so the long cells start
 // first and the short ones fill the tail.  Switching buckets rebuilds the CTA's tables and

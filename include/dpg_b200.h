@@ -210,9 +210,9 @@ int dpg_plan_query(const dpg_plan* plan, dpg_plan_info* info);
  * graph) and returns it in *chosen: for single-CTA plans the Gram staging ring
  * that fits the bucket's shared memory (8: chunks of 16 or 8 quadrature points,
  * 4: chunks of 4; it sets the shared-memory layout), for large-bucket plans
- * the formation k-chunk (32 or 16 points).  Results of the configurations agree
- * to rounding (sums are ordered differently).  Allocates its timing outputs from
- * the library's pool. */
+ * the formation k-chunk (32 or 16 points).  The rings sum in the same order and
+ * give the same bits; the k-chunks agree to rounding.  Allocates its timing
+ * outputs from the library's pool. */
 int dpg_plan_autotune(dpg_plan* plan, int C, const double* nodes, const int8_t* parity, const double* coeff,
                       void* stream, int* chosen);
 
@@ -379,9 +379,11 @@ int dpg_multi_autotune(int n_buckets, const dpg_bucket_batch* buckets, void* str
  * launches and the work queue of the single-CTA buckets (whose counters reset
  * themselves at the end of each launch) as branches, with priorities in
  * decreasing order of cost and a workspace for each large bucket, so that one
- * bucket's CTAs take the SMs that another's last wave leaves idle; where the
- * workspaces do not fit together, the launches share one and run one after
- * another.  Launches of one graph must not overlap on the GPU (they share the
+ * bucket's CTAs take the SMs that another's last wave leaves idle.  The graph
+ * holds them until dpg_graph_destroy: 2.95 GB for the seven large buckets of a
+ * Stokes mesh of p = 1..6 with as many cells in each as SMs (1.04 GB of it the
+ * p = 6 quads').  Where they do not fit together, the launches share the largest
+ * and run one after another.  Launches of one graph must not overlap on the GPU (they share the
  * workspaces). */
 typedef struct dpg_graph dpg_graph;
 int dpg_graph_capture(int n_buckets, const dpg_bucket_batch* buckets, int flags, dpg_graph** out);
