@@ -14,7 +14,8 @@ static DpgKernelChoice choose_adjoint_kernel(const DpgPlanDev* plan, int C) {
 }
 
 int dpg_configure_adjoint(const DpgPlanDev* plan, int bytes) {
-  for (int C : {1, INT_MAX}) {  // few cells, many cells
+  for (int C : {1, INT_MAX}) {  // few cells, many cells (a small bucket's other kernel)
+    if (C > 1 && !plan->small) break;
     const DpgKernelChoice kc = choose_adjoint_kernel(plan, C);
     KernelFn k = kc.k;
     if (!k) return DPG_OK;

@@ -111,7 +111,8 @@ int dpg_configure_kernels(const DpgPlanDev* plan) {
   size_t bytes = (size_t)plan->sm_total * sizeof(double);
   if (optin > 0 && bytes > (size_t)optin) return dpg::fail(DPG_ERR_UNSUPPORTED, "bucket needs more shared memory than one CTA has");
   if (optin > 0) bytes = (size_t)optin;
-  for (int C : {1, INT_MAX}) {  // few cells, many cells
+  for (int C : {1, INT_MAX}) {  // few cells, many cells (a small bucket's other kernel)
+    if (C > 1 && !plan->small) break;
     const DpgKernelChoice kc = choose_kernel(plan, C);
     KernelFn k = kc.k;
     if (!k) return dpg::fail(DPG_ERR_UNSUPPORTED, "no kernel instance for this bucket size");
