@@ -491,8 +491,20 @@ __device__ __forceinline__ void cp_async(void* dst, const void* src, int bytes) 
 }
 
 // Shared memory of one staged cell: S, entry weights, CSR row starts, positions, entry rows, starts.
-__host__ __device__ inline size_t staged_bytes(int t, int ecap, int ucap) {
-  return ((size_t)((t * t + 1) & ~1) + ecap + ucap) * 8 + ((size_t)ucap * ucap + ecap + ucap + 1) * 4;
+inline size_t staged_bytes(int t, int ecap, int ucap) {
+  return ((((size_t)t * t + 1) & ~(size_t)1) + ecap + ucap) * 8 + ((size_t)ucap * ucap + ecap + ucap + 1) * 4;
+}
+
+// Staging copies all of S, gathering reads what the map names, so staging wants a map that names enough of the t rows,
+// and more of them the fewer CTAs an SM holds.  Time gathered / staged (12,000 or 20,000 cells):
+//   up to 40 KB:  t = 26 0.38 of the rows 1.29, 0.27 0.90;  t = 50 0.3 1.29, 0.2 1.24, 0.1 0.73
+//   up to 75 KB (three CTAs):  t = 78 0.5 1.25, 0.4 0.98, 0.2 0.77, 0.03 0.42;  t = 72 0.44 1.03;  t = 86 0.44 1.07
+//   up to 110 KB (two):  t = 90 0.8 1.05, 0.64 0.93;  t = 94 0.8 1.07, 0.65 0.90;  t = 110 0.5 0.85, 0.2 0.49
+inline bool scatter_staged(int C, int t, int ecap, int ucap, int64_t entries) {
+  const size_t b = staged_bytes(t, ecap, ucap);
+  const double rows = (double)entries / ((double)C * t);
+  if (ucap > 1600) return false;
+  return b <= 40 * 1024 ? rows >= 0.3 : b <= 75 * 1024 ? rows >= 0.44 : b <= 110 * 1024 && rows >= 0.75;
 }
 
 __global__ void __launch_bounds__(SG_T) plan_apply_staged_kernel(int C, int t, int ecap, int ucap, PlanArrays A,
@@ -626,6 +638,7 @@ int dpg_launch_scatter_global(int C, int t, const int64_t* ptr, const int64_t* g
 struct dpg_scatter_plan {
   int C, t, ecap;
   int ucap;  // most distinct ids of a cell
+  int64_t entries;  // map entries of all cells
   int64_t n_global;
   void* base;
   PlanArrays A;
@@ -656,6 +669,7 @@ extern "C" int dpg_scatter_plan_create(int C, int t, const int64_t* map_ptr, con
   P->base = nullptr;
   P->ecap = 0;
   P->ucap = 0;
+  P->entries = 0;
   if (P->C == 0) {
     *out = P;
     return DPG_OK;
@@ -703,6 +717,7 @@ extern "C" int dpg_scatter_plan_create(int C, int t, const int64_t* map_ptr, con
   cudaMemcpyAsync(&P->ucap, d_max + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
   e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return bail(DPG_ERR_CUDA, std::string("scatter plan: ") + cudaGetErrorString(e));
+  P->entries = tot[1];
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const size_t b_off = al(3 * ((size_t)C + 1) * 8), b_u = al((size_t)tot[0] * 8), b_uf = al(((size_t)tot[0] + C) * 4),
                b_er = al((size_t)tot[1] * 4), b_ew = al((size_t)tot[1] * 8), b_pos = al((size_t)tot[2] * 4);
@@ -738,13 +753,18 @@ extern "C" int dpg_scatter_plan_create(int C, int t, const int64_t* map_ptr, con
   return DPG_OK;
 }
 
+// For tests: 1 if the plan's apply stages the cells' S.
+extern "C" int dpg_debug_scatter_staged(const dpg_scatter_plan* P) {
+  return P && P->C > 0 && scatter_staged(P->C, P->t, P->ecap, P->ucap, P->entries);
+}
+
 extern "C" int dpg_scatter_plan_apply(const dpg_scatter_plan* P, const double* S, const double* s, double* values,
                                       double* rhs, void* stream) {
   if (!P) return dpg::fail(DPG_ERR_INVALID_ARGUMENT, "null plan");
   if (P->C == 0) return DPG_OK;
   if (!S || !values) return dpg::fail(DPG_ERR_INVALID_ARGUMENT, "S and values are required");
-  const size_t staged = staged_bytes(P->t, P->ecap, P->ucap);
-  if (staged <= 110 * 1024 && P->ucap <= 1600) {  // two CTAs per SM at least
+  if (scatter_staged(P->C, P->t, P->ecap, P->ucap, P->entries)) {
+    const size_t staged = staged_bytes(P->t, P->ecap, P->ucap);
     plan_apply_staged_kernel<<<std::min(P->C, cell_grid((const void*)plan_apply_staged_kernel, staged)), SG_T, staged,
                                (cudaStream_t)stream>>>(P->C, P->t, P->ecap, P->ucap, P->A, S, s, values, rhs);
     cudaError_t e = cudaGetLastError();
