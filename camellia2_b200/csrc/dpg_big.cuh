@@ -488,8 +488,9 @@ __device__ void big_form_tile(const DpgPlanDev& P, int* fail, double* sc_out, in
 
 // The F row of E^T in blocks of 64 test rows; eight threads per row take every eighth point, their sums are joined in
 // order.  The products of a tile meet every entry with every row, zeros included: a load that is not finite must
-// not share them with B, nor a side of zero length with F.  (Not inlined: the 32 values in flight would
-// spill in the cell's body.)
+// not share them with B, nor a side of zero length with F.  Bound by the latency of its loads (records in L2): 148
+// Poisson quads of k = 5 425 us with F in the tiles, 435 with one thread per row, 429 so; 37 Stokes quads of
+// p = 6 1.778 -> 1.761 ms.  (Not inlined: the 32 values in flight would spill in the cell's body.)
 __device__ __noinline__ void big_load_row(const DpgPlanDev& P, double* row, const int* col, const double* sc, const double* vt,
                                           double* red, int first, int step) {
   const double* const rec = P.seg[0].rec;

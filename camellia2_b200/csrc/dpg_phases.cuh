@@ -331,9 +331,10 @@ __device__ __forceinline__ void factor_diag(const double* __restrict__ T, int k,
 // right-looking update reads and writes every trailing tile in every step (7.4 K cycles for
 // the first step of 22 tiles, a dozen warps each waiting on load, two products and store per
 // tile); here a tile is loaded and stored once, its products run in two chains joined at the
-// end, and the work of a step stays below the time of the diagonal tile next door.  That chain of diagonal tiles is what bounds the factorisation: warp 0 does
-// nothing else, with its sub-partition to itself (warps 4, 8, 12 only keep the barriers), and it
-// needs from the others only the sum over j < k of tile (k+1, k+1), formed a step ahead.
+// end, and the work of a step stays below the time of the diagonal tile next door.  That chain of
+// diagonal tiles is what bounds the factorisation: warp 0 does nothing else, with its sub-partition
+// to itself (warps 4, 8, 12 only keep the barriers), and it needs from the others only the sum over
+// j < k of tile (k+1, k+1), formed a step ahead.
 constexpr int CHOL_NW = NW - NW / 4;  // warps that update: those of the other sub-partitions
 
 __device__ __forceinline__ int chol_rank(int warp) { return warp - (warp >> 2) - 1; }
